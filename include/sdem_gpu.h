@@ -278,7 +278,7 @@ int sdem_selftest_fp64(long long n, unsigned long long seed, long long* mismatch
 
 /* ---- launch shape (no counterpart in the reference) -------------------------
  * The step's search/force pipeline runs in pipeline_chunks chunks of target
- * sort positions (1..4; default 2), the first of them holding
+ * sort positions (1..4; default 1), the first of them holding
  * first_chunk_percent percent of the targets (10..90; -1: the default split,
  * where the first chunk holds as many whole waves of resident search blocks
  * as fit in an even share when that trims the share by a quarter at most,

@@ -4,9 +4,10 @@
 //
 // One step (the body of DEMS_iterate, Prtcl_DEMSystem.f90:214-247) is:
 //   k_step_begin                       UpdateNearPrtclsPW (Prtcl_ContactSearchPW.f90:159-235),
-//                                      device-predicated on iter >= Next_iter_update; the
-//                                      step's image and gather-order counters reset
-//   k_ghost_*                          PC_Comm_For_Cntct on one rank (periodic directions only):
+//                                      device-predicated on iter >= Next_iter_update; the list of the
+//                                      particles near a wall
+//   k_wall_detect                      FindContactsPW's detection (:298-319) over that list
+//   k_ghost                            PC_Comm_For_Cntct on one rank (periodic directions only):
 //                                      images of the particles near periodic faces, in the
 //                                      reference's pass order, as ordered stream compactions
 //   k_bin, scan, k_scatter, k_cellorder
@@ -18,31 +19,24 @@
 //   k_search                           LoopNBSMask + FineSearch2/3 (:302-473, :503-557): one thread per
 //                                      target particle, same 13-cell half shell + same-cell tail, same
 //                                      exact FP64 overlap test; contacts go to the target's row (in visit
-//                                      order) and an entry (target, slot) to the partner's in-list
-//   k_wall_detect                      FindContactsPW's detection (:298-319) over the near-wall mask,
-//                                      and the contact count of every particle for the gather order
-//   scan, k_row_fill                   row offsets (CSR) and each contact's row
+//                                      order), an entry (target, slot) to the partner's in-list, and the
+//                                      row's contacts to their place in the contact arrays
 //   k_force                            Find_insert history lookup + ContactForce_PP / _PPG
 //                                      (Prtcl_CL_and_CF.f90:142-198, 256-296, 732-798): one thread per
-//                                      contact, full warps of FP64 work
-//   k_wall_force                       ContactForce_PW (:832-856), one thread per wall contact
-//   k_degree_scatter                   particles grouped by contact count (the gather order), one
-//                                      record per gather position with what the gather reads first
+//                                      contact, full warps of FP64 work; after the pairs the wall
+//                                      contacts (ContactForce_PW, :832-856)
 //
-// Search, row offsets, row fill and forces run in chunks of target sort
-// positions on two streams, so that the search of one chunk (integer and
-// memory work) overlaps the force kernel of the one before (FP64 work); wall
-// detection, wall forces and the gather order follow the searches on the
-// second stream, beside the forces.
+// The walls run on a second stream beside the images, the binning and the
+// sort.  Search and forces can run in chunks of target sort positions
+// (sdem_set_launch), the search of one beside the forces of the one before.
 //   k_gather                           per particle, sums its contact records in the reference's scatter
 //                                      order (a deterministic gather; records signed for the row's
 //                                      target, moments scaled by the particle's own radius), then its
 //                                      wall contacts in near-list order
 //   k_integrate                        clc_Acceleration (Prtcl_DEMSystem.f90:166-181), Prtcl_Integrate
 //                                      (Prtcl_Integration.f90:15-88) and the periodic wrap, in index
-//                                      order
-//   k_finish                           one-rank out-of-domain delete (Prtcl_Comm.f90:1569-1840),
-//                                      iterNumber += 1, counters
+//                                      order; its last block ends the step: one-rank out-of-domain
+//                                      delete (Prtcl_Comm.f90:1569-1840), iterNumber += 1, counters
 // RemvReleased/PreIteration have no kernel: the history of step n+1 is exactly
 // the contact records written at step n (double-buffered, keyed by particle id).
 #include <cuda_runtime.h>
@@ -72,11 +66,11 @@ constexpr int kMaxK = 64;         // row / in-list capacity limit (6-bit slot in
 constexpr int kKw = 4;            // wall contacts per particle
 constexpr int kMaxWalls = 64;     // near-wall mask is 64 bits
 constexpr int kOutCap = 4096;     // out-of-domain deletions per step
-constexpr int kScanThreads = 256, kScanItems = 32;
+constexpr int kScanThreads = kThreads, kScanItems = 16;
 constexpr int kScanTile = kScanThreads * kScanItems;   // elements per scan block
-constexpr int kDegBuckets = 64;   // gather-order buckets by number of contact records
+constexpr int kDegBuckets = 64;   // gather: buckets by number of contact records
 #ifndef SDEM_PIPELINE_CHUNKS
-#define SDEM_PIPELINE_CHUNKS 2
+#define SDEM_PIPELINE_CHUNKS 1
 #endif
 constexpr int kChunks = SDEM_PIPELINE_CHUNKS;   // search/force pipeline chunks per step (default)
 constexpr int kMaxChunks = 4;                   // most chunks sdem_set_launch accepts
@@ -84,9 +78,6 @@ constexpr int kSearchBlocksPerSM = 6;           // k_search's register budget: r
 constexpr int kForceBlocksPerSM = 3;            // k_force blocks per SM in the pipeline (default)
 #ifndef SDEM_FORCE_MIN_BLOCKS
 #define SDEM_FORCE_MIN_BLOCKS 3    // k_force blocks of 256 threads per SM its register budget allows
-#endif
-#ifndef SDEM_SEARCH_PREFETCH
-#define SDEM_SEARCH_PREFETCH 0     // 1: k_search requests the next candidate's record before testing one
 #endif
 constexpr int kMaxLevels = 6;     // hierarchical search levels (Init_Munjiza_Hrchl caps at 6)
 
@@ -108,18 +99,6 @@ enum Phase { PH_WALL, PH_BIN, PH_SCAN_CELLS, PH_SCATTER, PH_CELLORDER, PH_SEARCH
 const char* const kPhaseNames[kPhases] = {"wall_refresh", "bin", "scan_cells", "scatter", "cellorder", "search",
                                           "scan_rows", "row_fill", "force", "wall_force", "gather_integrate",
                                           "delete", "step_end"};
-
-// What the gather reads first for the sphere at one gather position, written
-// by the degree scatter in index order (coalesced there) so that the gather
-// reads one record instead of several scattered values.
-struct __align__(32) GRec {
-  int p;        // the sphere
-  int s;        // its sort position
-  int own_a;    // its row start
-  int counts;   // row length << 16 | in-list length << 8 | wall contacts
-  double r;     // its radius
-  double pad;
-};
 
 // ---------------------------------------------------------------------------
 // The force kernel's record of one contact for the gather, 96 bytes in one
@@ -150,7 +129,8 @@ struct Dev {
   int per[3];
   double3 Lbox;
   double lencs;   // LenForCS = Prtcl_cs_ratio * maxD (Prtcl_Comm.f90:80-81)
-  int *gflag, *goff;
+  struct ScanCtl* gctl;          // ghost passes: tickets and tile words
+  unsigned long long* gwords;
   int max_gid, K, Kin, ccap;
   int tsize, rsize, pi, pri, quirk;
   sdem::LawCfg law;
@@ -196,7 +176,8 @@ struct Dev {
   // the lower id for particle-particle pairs, the local particle for a pair
   // with a periodic image; own_c lists this step's contacts of each owner id
   int Ko;
-  int* c_row;   // row (target sort position) of each contact
+  int* c_cnt;     // contacts found by each chunk of the search (kMaxChunks)
+  int2* c_pair;   // per contact: the row's target and its partner
   int* own_cnt;
   int2* own_c;   // (contact index, partner id): the lookup reads the partner ids of one owner in one sector
   const int* own_cnt_prev;
@@ -204,18 +185,19 @@ struct Dev {
   int *wh_cnt, *wh_wall;
   dbl4* wh_hist;
   // wall contacts of this step: per particle up to kKw slots (decreasing wall
-  // index), and a compact list (particle << 3 | slot) for the force kernel
+  // index), and a compact list (particle << 3 | slot) for the force kernel;
+  // the particles near a wall, as of the last rebuild of that list
   int* w_cnt;
   int* w_wall;
   dbl4* w_geo;       // (nv, ovrlp)
   dbl4 *w_S, *w_M, *w_Mr;
   int* wl;
   int* wl_cnt;
-  // gather order: particles bucketed by their number of contact records, so a
-  // warp's summation loops run the same trip count
-  int *deg_cnt, *deg_of, *deg_rank;
-  struct GRec* gorder;   // per gather position: what the gather reads first
-  const int *wh_cnt_prev, *wh_wall_prev;
+  int* near_list;
+  int* near_cnt;
+  int* near_stale;   // 1: the list is rebuilt at the start of the next step (near_cnt is 0 then)
+  int* wh_cnt_prev;
+  const int* wh_wall_prev;
   const dbl4* wh_hist_prev;
   // status and scalars
   int* status;                    // [0] error code, [1] detail
@@ -237,98 +219,107 @@ __device__ __forceinline__ void raise(const Dev& d, int code, int detail) {
 }
 
 // ---------------------------------------------------------------------------
-// Exclusive scan of int32 (n elements) into out[0..n], out[n] = total, in
-// three launches: tile sums, a scan of the tile sums, the tiles.  A tile is
-// 256 threads x 32 elements; full, 16-byte-aligned tiles move as int4
-// (each load instruction covers 512 contiguous bytes of a warp).
-__device__ __forceinline__ bool scan_vec_ok(const int* p, long long base, long long n) {
-  return base + kScanTile <= n && ((reinterpret_cast<uintptr_t>(p) & 15u) == 0);
+// Ordered prefix sums in one launch (decoupled look-back: Merrill and Garland,
+// "Single-pass Parallel Prefix Scan with Decoupled Look-back", 2016).  Blocks
+// take tiles in order from a ticket, so every earlier tile is running or done;
+// each publishes its tile's sum, then adds up its predecessors' words until it
+// meets a complete prefix.  A tile's word holds epoch (30 bits), state (1: the
+// tile's sum, 2: the prefix through the tile) and value (32 bits) together, so
+// a reader needs no fence; the epoch, one per launch, makes the words of
+// earlier launches stale without clearing them.
+struct ScanCtl {
+  int ticket, done;
+  unsigned epoch;
+  int total;   // ghost passes: images made by the pass
+};
+constexpr int kSpinLimit = 1 << 20;   // polls of one word before a wait gives up
+
+__device__ __forceinline__ unsigned long long scan_word(unsigned epoch, unsigned state, int v) {
+  return (unsigned long long)((epoch << 2) | state) << 32 | (unsigned)v;
 }
 
-__global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const int* __restrict__ in, long long n,
-                                                               int* __restrict__ bsum) {
-  __shared__ int warp_sums[kScanThreads / 32];
-  const long long base = (long long)blockIdx.x * kScanTile;
-  int s = 0;
-  if (scan_vec_ok(in, base, n)) {
-    const int4* v = reinterpret_cast<const int4*>(in + base);
-#pragma unroll
-    for (int j = 0; j < kScanItems / 4; j++) {
-      const int4 q = v[j * kScanThreads + threadIdx.x];
-      s += (q.x + q.y) + (q.z + q.w);
-    }
-  } else {
-    for (int e = threadIdx.x; e < kScanTile; e += kScanThreads)
-      if (base + e < n) s += in[base + e];
-  }
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) warp_sums[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
+// Exclusive prefix of `tile` whose sum is `sum` (thread 0's); the whole block
+// calls, so that one round looks back over kThreads tiles: with one warp's 32 a
+// scan of 2,200 tiles took 81 us, the chain of waits alone.  A wait that runs
+// out is reported and counts as zero: the prefixes then come out too small,
+// never too large, so what is indexed with them stays in range.
+__device__ int scan_lookback(volatile unsigned long long* words, unsigned epoch, int tile, int sum, int* status) {
+  __shared__ int part[kThreads / 32], first_full[kThreads / 32];
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const unsigned key = epoch & 0x3FFFFFFFu;
+  if (t == 0) words[tile] = scan_word(key, tile == 0 ? 2u : 1u, sum);
+  int excl = 0;
+  for (int j = tile - 1; j >= 0; j -= kThreads) {
+    const int i = j - t;
+    unsigned state = 2u;
     int v = 0;
-    for (int w = 0; w < kScanThreads / 32; w++) v += warp_sums[w];
-    bsum[blockIdx.x] = v;
-  }
-}
-
-__device__ __forceinline__ int block_exclusive_scan_1024(int v, int* sh, int* total) {
-  // inclusive warp scan
-  int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  int x = v;
-  for (int o = 1; o < 32; o <<= 1) {
-    int y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
-  }
-  if (lane == 31) sh[wid] = x;
-  __syncthreads();
-  if (wid == 0) {
-    int w = (lane < (int)(blockDim.x >> 5)) ? sh[lane] : 0;
-    int z = w;
-    for (int o = 1; o < 32; o <<= 1) {
-      int y = __shfl_up_sync(0xffffffffu, z, o);
-      if (lane >= o) z += y;
+    if (i >= 0) {
+      int polls = 0;
+      unsigned long long x;
+      do {
+        x = words[i];
+      } while (((unsigned)(x >> 34) != key || ((unsigned)(x >> 32) & 3u) == 0u) && ++polls < kSpinLimit);
+      if (polls < kSpinLimit) {
+        state = (unsigned)(x >> 32) & 3u;
+        v = (int)(unsigned)x;
+      } else if (atomicCAS(status, 0, SDEM_E_TIMEOUT) == 0) {
+        status[1] = i;
+      }
     }
-    sh[lane] = z - w;  // exclusive warp offsets
-    if (lane == 31) sh[32] = z;
+    // the nearest complete prefix ends the walk
+    const unsigned full = __ballot_sync(0xffffffffu, state == 2u);
+    const int stop = full ? __ffs(full) - 1 : 31;
+    int add = lane <= stop ? v : 0;
+    for (int o = 16; o > 0; o >>= 1) add += __shfl_xor_sync(0xffffffffu, add, o);
+    if (lane == 0) {
+      part[w] = add;
+      first_full[w] = full != 0u;
+    }
+    __syncthreads();
+    bool done = false;
+    for (int k = 0; k < kThreads / 32 && !done; k++) {
+      excl += part[k];
+      done = first_full[k] != 0;
+    }
+    __syncthreads();
+    if (done) break;
   }
-  __syncthreads();
-  int r = sh[wid] + x - v;
-  *total = sh[32];
-  __syncthreads();
-  return r;
+  if (t == 0 && tile > 0) words[tile] = scan_word(key, 2u, excl + sum);
+  return excl;
 }
 
-__global__ void k_scan_blocks(int* bsum, int nb) {
-  __shared__ int sh[33];
-  int carry = 0;
-  for (int base = 0; base < nb; base += 1024) {
-    int i = base + threadIdx.x;
-    int v = (i < nb) ? bsum[i] : 0;
-    int tot;
-    int e = block_exclusive_scan_1024(v, sh, &tot);
-    if (i < nb) bsum[i] = e + carry;
-    carry += tot;
+// out[i] = sum of in[0..i), out[n] = the total; in[] is left zero for the next
+// step's counting.  A tile is 256 threads x 16 elements through shared memory
+// (padded: element e at e + e/16, so that the striped int4 copies and the
+// per-thread runs of 16 are both free of bank conflicts).
+// One launch where the three of a reduce-then-scan took 14.5 us of dependent
+// latency: 6 us at 7,000 cells, 9 us at 60,000.
+template <bool kOnePass>
+__global__ void __launch_bounds__(kScanThreads) k_scan(int* __restrict__ in, long long n, int* __restrict__ out,
+                                                       ScanCtl* ctl, unsigned long long* words, int* status) {
+  __shared__ int sh[kScanTile + kScanTile / kScanItems];
+  __shared__ int wsum[kScanThreads / 32];
+  __shared__ int s_tile, s_total;
+  __shared__ unsigned s_epoch;
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  if (kOnePass) {
+    if (t == 0) {
+      s_epoch = ctl->epoch + 1u;
+      s_tile = atomicAdd(&ctl->ticket, 1);
+    }
+    __syncthreads();
+    if (s_tile >= (int)gridDim.x) return;   // (only a caller that shares ctl between overlapping launches gets here)
   }
-}
-
-// out[i] = *offset + sum of in[0..i), out[n] = the total (offset may be null).
-// The tile goes through shared memory (padded: element e at e + e/32, so that
-// both the striped int4 copies and the per-thread runs of 32 are free of bank
-// conflicts); each thread scans its 32 consecutive elements, the block scans
-// the 256 thread totals.
-__global__ void __launch_bounds__(kScanThreads) k_scan_apply(const int* __restrict__ in, long long n,
-                                                              const int* __restrict__ bsum, int* __restrict__ out,
-                                                              const int* __restrict__ offset) {
-  __shared__ int sh[kScanTile + kScanTile / 32];
-  __shared__ int wsum[kScanThreads / 32 + 1];
-  const int t = threadIdx.x;
-  const long long base = (long long)blockIdx.x * kScanTile;
-  auto pad = [](int e) { return e + (e >> 5); };
-  if (scan_vec_ok(in, base, n)) {
-    const int4* v = reinterpret_cast<const int4*>(in + base);
+  const int tile = kOnePass ? s_tile : (int)blockIdx.x;
+  const long long base = (long long)tile * kScanTile;
+  const bool whole = base + kScanTile <= n;
+  auto pad = [](int e) { return e + e / kScanItems; };
+  if (whole) {
+    int4* v = reinterpret_cast<int4*>(in + base);
 #pragma unroll
     for (int j = 0; j < kScanItems / 4; j++) {
       const int4 q = v[j * kScanThreads + t];
+      v[j * kScanThreads + t] = make_int4(0, 0, 0, 0);
       const int e = pad((j * kScanThreads + t) * 4);
       sh[e] = q.x;
       sh[e + 1] = q.y;
@@ -336,7 +327,10 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(const int* __restri
       sh[e + 3] = q.w;
     }
   } else {
-    for (int e = t; e < kScanTile; e += kScanThreads) sh[pad(e)] = base + e < n ? in[base + e] : 0;
+    for (int e = t; e < kScanTile; e += kScanThreads) {
+      sh[pad(e)] = base + e < n ? in[base + e] : 0;
+      if (base + e < n) in[base + e] = 0;
+    }
   }
   __syncthreads();
   int loc[kScanItems];
@@ -347,8 +341,6 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(const int* __restri
     loc[i] = sum;
     sum += v;
   }
-  // exclusive scan of the thread totals
-  const int lane = t & 31, w = t >> 5;
   int x = sum;
   for (int o = 1; o < 32; o <<= 1) {
     const int y = __shfl_up_sync(0xffffffffu, x, o);
@@ -356,22 +348,35 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(const int* __restri
   }
   if (lane == 31) wsum[w] = x;
   __syncthreads();
-  if (t == 0) {
-    int acc = 0;
-    for (int k = 0; k < kScanThreads / 32; k++) {
-      const int c = wsum[k];
-      wsum[k] = acc;
-      acc += c;
+  if (w == 0) {
+    const int v = lane < kScanThreads / 32 ? wsum[lane] : 0;
+    int z = v;
+    for (int o = 1; o < kScanThreads / 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, z, o);
+      if (lane >= o) z += y;
     }
-    wsum[kScanThreads / 32] = acc;
+    if (lane < kScanThreads / 32) wsum[lane] = z - v;
+    if (lane == kScanThreads / 32 - 1) s_total = z;
   }
   __syncthreads();
-  const int carry = bsum[blockIdx.x] + (offset ? *offset : 0);
-  const int first = carry + wsum[w] + x - sum;
+  int excl = 0;
+  if (kOnePass) {
+    excl = scan_lookback(words, s_epoch, tile, s_total, status);
+  } else {   // the sums of the tiles before this one (k_scan_sums)
+    __shared__ int part[kScanThreads / 32];
+    const int* __restrict__ sums = reinterpret_cast<const int*>(words);
+    for (int i = t; i < tile; i += kScanThreads) excl += sums[i];
+    for (int o = 16; o > 0; o >>= 1) excl += __shfl_xor_sync(0xffffffffu, excl, o);
+    if (lane == 0) part[w] = excl;
+    __syncthreads();
+    excl = 0;
+    for (int k = 0; k < kScanThreads / 32; k++) excl += part[k];
+  }
+  const int first = excl + wsum[w] + x - sum;
 #pragma unroll
   for (int i = 0; i < kScanItems; i++) sh[t * (kScanItems + 1) + i] = first + loc[i];
   __syncthreads();
-  if (scan_vec_ok(out, base, n)) {
+  if (whole) {
     int4* v = reinterpret_cast<int4*>(out + base);
 #pragma unroll
     for (int j = 0; j < kScanItems / 4; j++) {
@@ -382,31 +387,75 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(const int* __restri
     for (int e = t; e < kScanTile; e += kScanThreads)
       if (base + e < n) out[base + e] = sh[pad(e)];
   }
-  if (blockIdx.x == gridDim.x - 1 && t == 0) out[n] = carry + wsum[kScanThreads / 32];
+  if (t == 0) {
+    if (tile == (int)gridDim.x - 1) out[n] = excl + s_total;
+    if (kOnePass && atomicAdd(&ctl->done, 1) == (int)gridDim.x - 1) {   // every block has its ticket and epoch
+      ctl->ticket = 0;
+      ctl->done = 0;
+      ctl->epoch = s_epoch;
+    }
+  }
+}
+
+// The tiles' sums for the two-launch form.
+__global__ void __launch_bounds__(kScanThreads) k_scan_sums(const int* __restrict__ in, long long n, int* __restrict__ sums) {
+  __shared__ int part[kScanThreads / 32];
+  const long long base = (long long)blockIdx.x * kScanTile;
+  int v = 0;
+  if (base + kScanTile <= n) {
+    const int4* q = reinterpret_cast<const int4*>(in + base);
+#pragma unroll
+    for (int j = 0; j < kScanItems / 4; j++) {
+      const int4 a = q[j * kScanThreads + threadIdx.x];
+      v += (a.x + a.y) + (a.z + a.w);
+    }
+  } else {
+    for (int e = threadIdx.x; e < kScanTile; e += kScanThreads)
+      if (base + e < n) v += in[base + e];
+  }
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    v = 0;
+    for (int k = 0; k < kScanThreads / 32; k++) v += part[k];
+    sums[blockIdx.x] = v;
+  }
+}
+
+// Scans n cell counts into out[0..n] and leaves them zero; launches issued.
+// Up to 256 tiles (1M cells) in one launch; beyond, the look-back's chain of
+// waits costs more than a second launch: 317 tiles 14.7 against 11.8 us, 2,470
+// tiles 77 against 43 us; 128 tiles 10.5 against 11.3 us, 7 tiles 6 against 9.6.
+constexpr int kOnePassTiles = 256;
+int scan_tiles(long long n) { return (int)std::max<long long>(1, (n + kScanTile - 1) / kScanTile); }
+
+int scan_cells(int* cnt, long long n, int* out, ScanCtl* ctl, unsigned long long* words, int* status, cudaStream_t st) {
+  const int tiles = scan_tiles(n);
+  if (tiles <= kOnePassTiles) {
+    k_scan<true><<<tiles, kScanThreads, 0, st>>>(cnt, n, out, ctl, words, status);
+    return 1;
+  }
+  k_scan_sums<<<tiles, kScanThreads, 0, st>>>(cnt, n, reinterpret_cast<int*>(words));
+  k_scan<false><<<tiles, kScanThreads, 0, st>>>(cnt, n, out, ctl, words, status);
+  return 2;
 }
 
 // ---------------------------------------------------------------------------
-// The start of a step.  UpdateNearPrtclsPW (Prtcl_ContactSearchPW.f90:159-235)
-// when iter >= Next_iter_update: the near-wall bit mask of every particle
-// (walls whose AABB +- DeltaXmax2 holds it) and max |v|, max |a|, reduced per
-// block into partials; the last block to finish reduces the partials and
-// computes the next refresh iteration.  Every step: the image and
-// gather-order counters reset.  A fixed grid (grid-stride over particles), so
-// that a step without refresh costs a few hundred block launches.
+// UpdateNearPrtclsPW (Prtcl_ContactSearchPW.f90:159-235) when iter >=
+// Next_iter_update: the near-wall bit mask of every particle (walls whose AABB
+// +- DeltaXmax2 holds it) and max |v|, max |a|, reduced per block into
+// partials; the last block to finish reduces the partials and computes the
+// next refresh iteration.  With the masks the list of the particles near any
+// wall is made, which k_wall_detect walks; after a step that deleted particles (and
+// moved others to their indices) it is rebuilt from the masks as they are.
+// A fixed grid (grid-stride over particles), so that a step without a rebuild
+// costs a few hundred block launches.
 constexpr int kBeginBlocksPerSM = 4;
 
-__device__ __forceinline__ void reset_step_counters(const Dev& d) {
-  *d.ng = 0;
-  *d.nt = *d.n;
-  for (int b = 0; b < kDegBuckets; b++) d.deg_cnt[b] = 0;   // gather-order buckets of this step
-}
-
 __global__ void __launch_bounds__(kThreads) k_step_begin(Dev d) {
+  if (*d.near_stale == 0) return;
   const bool refresh = *d.iter >= *d.next_update;
-  if (!refresh) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) reset_step_counters(d);
-    return;
-  }
   // expanded wall boxes, pmin = min - DeltaXmax2 and pmax = max + DeltaXmax2
   // (FP64, as the reference), once per block; the tests run on the integer pipes
   __shared__ double box[64][6];
@@ -420,18 +469,36 @@ __global__ void __launch_bounds__(kThreads) k_step_begin(Dev d) {
   // non-negative doubles order like their bit patterns
   unsigned long long vb = 0ull, ab = 0ull;
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
-    const dbl4 P = d.posr[p];
     unsigned long long mask = 0ull;
-    for (int k = 0; k < d.nw; k++) {
-      if (fpi::ge(P.x, box[k][0]) && fpi::le(P.x, box[k][3]) && fpi::ge(P.y, box[k][1]) && fpi::le(P.y, box[k][4]) &&
-          fpi::ge(P.z, box[k][2]) && fpi::le(P.z, box[k][5]))
-        mask |= (1ull << k);
+    if (refresh) {
+      const dbl4 P = d.posr[p];
+      for (int k = 0; k < d.nw; k++) {
+        if (fpi::ge(P.x, box[k][0]) && fpi::le(P.x, box[k][3]) && fpi::ge(P.y, box[k][1]) && fpi::le(P.y, box[k][4]) &&
+            fpi::ge(P.z, box[k][2]) && fpi::le(P.z, box[k][5]))
+          mask |= (1ull << k);
+      }
+      d.near_mask[p] = mask;
+      const unsigned long long v = fpi::bits(sdem::norm3(sdem::xyz(d.vel0[p])));
+      const unsigned long long a = fpi::bits(sdem::norm3(sdem::xyz(d.acc0[p])));
+      vb = v > vb ? v : vb;
+      ab = a > ab ? a : ab;
+    } else {
+      mask = d.near_mask[p];
     }
-    d.near_mask[p] = mask;
-    const unsigned long long v = fpi::bits(sdem::norm3(sdem::xyz(d.vel0[p])));
-    const unsigned long long a = fpi::bits(sdem::norm3(sdem::xyz(d.acc0[p])));
-    vb = v > vb ? v : vb;
-    ab = a > ab ? a : ab;
+    const unsigned act = __activemask(), in = __ballot_sync(act, mask != 0ull);
+    if (mask) {
+      const int lane = threadIdx.x & 31, leader = __ffs(in) - 1;
+      int base = 0;
+      if (lane == leader) base = atomicAdd(d.near_cnt, __popc(in));
+      base = __shfl_sync(in, base, leader);
+      d.near_list[base + __popc(in & ((1u << lane) - 1u))] = p;
+    } else {
+      // off the list: no wall contacts and no wall history until it is back
+      const int g = d.gid[p];
+      d.w_cnt[p] = 0;
+      d.wh_cnt[g] = 0;
+      d.wh_cnt_prev[g] = 0;
+    }
   }
   __shared__ unsigned long long part[kThreads / 32][2];
   __shared__ int last;
@@ -459,6 +526,8 @@ __global__ void __launch_bounds__(kThreads) k_step_begin(Dev d) {
   if (!last || threadIdx.x != 0) return;
   __threadfence();
   *d.ticket = 0;
+  *d.near_stale = 0;   // every block has read it
+  if (!refresh) return;
   // the other blocks' partials, read at L2 (never cached in this SM's L1)
   vb = 0ull;
   ab = 0ull;
@@ -481,16 +550,14 @@ __global__ void __launch_bounds__(kThreads) k_step_begin(Dev d) {
   numIter = numIter > 1 ? numIter : 1;
   numIter = numIter < d.wall_max_update_iter ? numIter : d.wall_max_update_iter;
   *d.next_update = it + numIter;
-  reset_step_counters(d);
 }
 
 // ---------------------------------------------------------------------------
 // Periodic images: PC_Comm_For_Cntct (Prtcl_Comm.f90:554-877, y pencil, one
 // rank).  Passes in the reference's order -- y (from the locals, up to two
 // images each), then +x, -x, +z, -z, each over the images made so far and
-// then the locals -- as ordered stream compactions: a flag per candidate
-// (images first, then locals), an exclusive scan, a scatter.  Candidate j of
-// a pass: j < gcap is image j (if j < ng), j >= gcap is local j - gcap.
+// then the locals -- as ordered stream compactions of one launch each (the
+// look-back above orders the tiles).
 enum GhostPass { GP_Y = 0, GP_XP = 1, GP_XM = 2, GP_ZP = 3, GP_ZM = 4 };
 
 
@@ -506,28 +573,9 @@ __device__ __forceinline__ int ghost_count(const Dev& d, int pass, const dbl4& P
   }
 }
 
-__global__ void k_ghost_flag(Dev d, int pass) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  const int len = d.gcap + d.n_launch;
-  if (j >= len) return;
-  const int n = *d.n, ng = *d.ng;
-  int src = -1;
-  if (j < d.gcap) {
-    if (pass != GP_Y && j < ng) src = n + j;
-  } else if (j - d.gcap < n) {
-    src = j - d.gcap;
-  }
-  d.gflag[j] = src >= 0 ? ghost_count(d, pass, d.posr[src]) : 0;
-}
-
-__global__ void k_ghost_scatter(Dev d, int pass) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  const int len = d.gcap + d.n_launch;
-  if (j >= len || d.gflag[j] == 0) return;
-  const int n = *d.n, ng = *d.ng;
-  const int src = j < d.gcap ? n + j : j - d.gcap;
+// the images of particle src in this pass, at image positions out, out+1
+__device__ __forceinline__ void ghost_emit(const Dev& d, int pass, int n, int src, int out) {
   const dbl4 P = d.posr[src];
-  int out = ng + d.goff[j];
   auto emit = [&](int dir, double shift) {
     if (out >= d.gcap) {
       raise(d, SDEM_E_CAPACITY, out);
@@ -557,12 +605,74 @@ __global__ void k_ghost_scatter(Dev d, int pass) {
   }
 }
 
-__global__ void k_ghost_count(Dev d) {
-  const int add = d.goff[d.gcap + d.n_launch];
-  int ng = *d.ng + add;
-  if (ng > d.gcap) ng = d.gcap;
-  *d.ng = ng;
-  *d.nt = *d.n + ng;
+constexpr int kGhostItems = 4, kGhostTile = kThreads * kGhostItems;
+
+// Six launches a pass (flags, a three-launch scan, scatter, count) took 29 us at
+// 60k spheres, this takes 12.
+__global__ void __launch_bounds__(kThreads) k_ghost(Dev d, int pass) {
+  __shared__ int wsum[kGhostItems * kThreads / 32];
+  __shared__ int s_tile, s_total;
+  __shared__ unsigned s_epoch;
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const int n = *d.n, ng = *d.ng;
+  if (t == 0) {
+    s_epoch = d.gctl->epoch + 1u;
+    s_tile = atomicAdd(&d.gctl->ticket, 1);
+  }
+  __syncthreads();
+  const int tile = s_tile;
+  const int ni = pass == GP_Y ? 0 : ng, len = ni + n;   // candidates: the images so far, then the locals
+  const int tiles = (len + kGhostTile - 1) / kGhostTile;
+  if (tile < tiles) {
+    int cnt[kGhostItems], off[kGhostItems];
+#pragma unroll
+    for (int i = 0; i < kGhostItems; i++) {
+      const int j = tile * kGhostTile + i * kThreads + t;
+      cnt[i] = j < len ? ghost_count(d, pass, d.posr[j < ni ? n + j : j - ni]) : 0;
+      int x = cnt[i];
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
+      off[i] = x - cnt[i];
+      if (lane == 31) wsum[i * (kThreads / 32) + w] = x;
+    }
+    __syncthreads();
+    if (w == 0) {   // 32 partial sums in candidate order: item, then warp
+      static_assert(kGhostItems * kThreads / 32 == 32, "one partial sum per lane");
+      const int v = wsum[lane];
+      int z = v;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, z, o);
+        if (lane >= o) z += y;
+      }
+      wsum[lane] = z - v;
+      if (lane == 31) s_total = z;
+    }
+    __syncthreads();
+    const int excl = scan_lookback(d.gwords, s_epoch, tile, s_total, d.status);
+    if (t == 0 && tile == tiles - 1) d.gctl->total = excl + s_total;
+#pragma unroll
+    for (int i = 0; i < kGhostItems; i++) {
+      if (cnt[i] == 0) continue;
+      const int j = tile * kGhostTile + i * kThreads + t;
+      ghost_emit(d, pass, n, j < ni ? n + j : j - ni, ng + excl + wsum[i * (kThreads / 32) + w] + off[i]);
+    }
+  }
+  __syncthreads();
+  if (t == 0) {
+    __threadfence();
+    if (atomicAdd(&d.gctl->done, 1) == (int)gridDim.x - 1) {   // every block has read the counts
+      __threadfence();
+      const int made = tiles > 0 ? __ldcg(&d.gctl->total) : 0;
+      const int now = min(ng + made, d.gcap);
+      *d.ng = now;
+      *d.nt = n + now;
+      d.gctl->ticket = 0;
+      d.gctl->done = 0;
+      d.gctl->epoch = s_epoch;
+    }
+  }
 }
 
 // The fourth word of a velocity record carries the particle's id and type
@@ -602,6 +712,7 @@ __global__ void k_fixed_append(Dev d) {
 __global__ void k_bin(Dev d) {
   int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= *d.nt) return;
+  if (d.in_cnt) d.in_cnt[p] = 0;   // this step's in-lists start empty
   const dbl4 P = d.posr[p];
   // the grid of the particle's level (hierarchical search: by type,
   // NBSMH_clcBoxIndex_and_BuildYList, Prtcl_Hrchl_Munjiza.f90:247-336)
@@ -680,16 +791,15 @@ __global__ void k_cellorder(Dev d) {
 // Six blocks per SM (40 registers): the walk is latency bound, and the extra
 // resident warps measured faster than the unconstrained 60-register build.
 template <bool kHier>
-__global__ void __launch_bounds__(kThreads, kSearchBlocksPerSM) k_search(Dev d, int s_begin, int s_end) {
+__global__ void __launch_bounds__(kThreads, kSearchBlocksPerSM) k_search(Dev d, int s_begin, int s_end, int chunk) {
   int s = s_begin + blockIdx.x * blockDim.x + threadIdx.x;
   const int nt = *d.nt;
   const int nloc = *d.n;
   unsigned long long cand = 0, cand_x = 0;
+  int rows = 0, m = 0;   // contacts of this thread's row, and its target
   if (s < s_end) {
-    if (s >= nt) {
-      d.row_cnt[s] = 0;
-    } else {
-      const int m = d.sorted[s];
+    if (s < nt) {
+      m = d.sorted[s];
       // a periodic image as target pairs with local particles only
       // (LoopNBSMask, Prtcl_NBS_Munjiza.f90:358-405 -> FineSearch3(n, m))
       const bool m_img = m >= nloc;
@@ -747,8 +857,8 @@ __global__ void __launch_bounds__(kThreads, kSearchBlocksPerSM) k_search(Dev d, 
         if (cnt < K) {
           d.row_partner[(size_t)cnt * nall + s] = q;
           if (q < nloc) {   // an image receives no force: it has no in-list
-            int slot = atomicAdd(&d.in_cnt[q], 1);
-            if (slot < Kin) d.in_list[(size_t)q * Kin + slot] = ((unsigned)s << 6) | (unsigned)cnt;
+            int slot = atomicAdd(&d.in_cnt[t], 1);
+            if (slot < Kin) d.in_list[(size_t)t * Kin + slot] = ((unsigned)s << 6) | (unsigned)cnt;
             else raise(d, SDEM_E_CL_FULL, q);
           }
         } else {
@@ -756,23 +866,12 @@ __global__ void __launch_bounds__(kThreads, kSearchBlocksPerSM) k_search(Dev d, 
         }
         cnt++;
       };
-      // Candidates [a, b) of one range, in order; with SDEM_SEARCH_PREFETCH the
-      // next candidate's record is requested (read-only path) before the
-      // current one is tested.  In a column (cells iz-1, iz, iz+1 consecutive
-      // in the sort) the z offset changes at the inner boundaries z1, z2.
+      // Candidates [a, b) of one range, in order.  In a column (cells iz-1, iz,
+      // iz+1 consecutive in the sort) the z offset changes at the inner
+      // boundaries z1, z2.
       auto walk = [&](int a, int b, int z1, int z2, float ox, float oy, float oz0, float oz1, float oz2,
                       unsigned long long& ctr) {
-#if SDEM_SEARCH_PREFETCH
-        if (a >= b) return;
-        float4 Qn = __ldg(&d.spos[a]);
-        for (int t = a; t < b; t++) {
-          const float4 Qf = Qn;
-          if (t + 1 < b) Qn = __ldg(&d.spos[t + 1]);
-          test(t, Qf, ox, oy, t < z1 ? oz0 : (t < z2 ? oz1 : oz2), ctr);
-        }
-#else
         for (int t = a; t < b; t++) test(t, d.spos[t], ox, oy, t < z1 ? oz0 : (t < z2 ? oz1 : oz2), ctr);
-#endif
       };
       // Cell boundaries of the whole half shell are loaded up front (they do
       // not depend on one another), then the candidates are walked in the
@@ -841,9 +940,35 @@ __global__ void __launch_bounds__(kThreads, kSearchBlocksPerSM) k_search(Dev d, 
           }
         }
       }
-      d.row_cnt[s] = cnt < K ? cnt : K;
-
+      rows = cnt < K ? cnt : K;
     }
+    d.row_cnt[s] = rows;
+  }
+  // The row's place in the contact arrays: a warp scan and one atomic per warp
+  // on the chunk's counter; the chunk starts where the earlier chunks' (their
+  // searches are complete) end.  Which place a row gets differs from run to
+  // run, what is computed from it does not: contacts are found through
+  // row_off and summed by (sort position, slot).  It replaces a row-count scan
+  // (three launches) and a row-fill kernel between each search and its forces
+  // (27 us of the 1M step, 4 of ~27 dependent launches per chunk in a small
+  // one), and gives k_force its pair in one coalesced read instead of a chain
+  // of three dependent ones.
+  const int lane = threadIdx.x & 31;
+  int incl = rows;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  int base = 0;
+  if (lane == 31 && incl > 0) {
+    base = atomicAdd(&d.c_cnt[chunk], incl);
+    for (int k = 0; k < chunk; k++) base += d.c_cnt[k];
+  }
+  base = __shfl_sync(0xffffffffu, base, 31) + incl - rows;
+  if (s < s_end) {
+    d.row_off[s] = base;
+    for (int j = 0; j < rows; j++)   // contacts past the capacity: k_force reports them
+      if (base + j < d.ccap) d.c_pair[base + j] = make_int2(m, d.row_partner[(size_t)j * d.nall + s]);
   }
   for (int o = 16; o > 0; o >>= 1) {
     cand += __shfl_down_sync(0xffffffffu, cand, o);
@@ -853,481 +978,166 @@ __global__ void __launch_bounds__(kThreads, kSearchBlocksPerSM) k_search(Dev d, 
   if ((threadIdx.x & 31) == 0 && cand_x) atomicAdd(&d.counters[9], cand_x);
 }
 
-// ---------------------------------------------------------------------------
-// The same search on the one-level grid, warp-cooperative and staged through
-// shared memory.  A warp takes 32 consecutive target sort positions; the
-// targets of one cell form a group and share one candidate list -- the cell
-// itself (each target uses the tail after its own position), then the
-// reference's half shell in its visit order.  Every lane first loads the
-// cell boundaries of its own target's list (the loads of all groups in
-// flight at once).  The warp then stages each group's list in shared memory
-// with asynchronous copies (cp.async: the candidates' single-precision
-// records and particle indices), one group ahead: group g+1's copies travel
-// while group g is tested.  One target at a time, the lanes test 32
-// consecutive candidates; a ballot over the hits gives every hit its row
-// slot in visit order, so rows, in-list keys and counters equal those of the
-// thread-per-target walk.  The tests are the same expressions as k_search's
-// (the prefilter, then the exact FP64 test inside its band).
-constexpr int kSearchWarps = 8;        // warps per block
-constexpr int kStage = 96;             // staged candidates per warp and buffer (longer lists go in pieces)
-#ifndef SDEM_SEARCH_MIN_BLOCKS
-#define SDEM_SEARCH_MIN_BLOCKS 2       // resident blocks per SM the register budget allows
-#endif
-#ifndef SDEM_SEARCH_WARP
-#define SDEM_SEARCH_WARP 0             // 1: the warp-cooperative search on the one-level grid
-#endif
-
-__device__ __forceinline__ float corner_offset(int code, float cellf) {
-  return code == 1 ? cellf : (code == 2 ? -cellf : 0.f);
-}
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
-  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(sa), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_1() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_0() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
-
-// The candidate list of a target cell in visit order: six ranges of sort
-// positions (own cell; cell (ix,iy,iz-1); columns (ix-1,iy), (ix-1..ix+1,iy-1),
-// each of cells iz-1..iz+1, consecutive in the sort).  Corner offsets
-// (target cell corner minus candidate cell corner) per axis are codes
-// 0 -> 0, 1 -> +cell, 2 -> -cell, packed x | y << 2 | z << 4; a column's z
-// code changes at its inner cell boundaries zb1, zb2.
-struct CandList {
-  int ra[6], rb[6], zb1[4], zb2[4];
-};
-
-__device__ __forceinline__ void cand_list(const int* __restrict__ cs, int key, int ix, int iy, int iz, int nx, int nz,
-                                          CandList& L) {
-  const int a0 = cs[key];
-  L.ra[0] = a0; L.rb[0] = cs[key + 1];
-  L.ra[1] = iz > 0 ? cs[key - 1] : 0; L.rb[1] = iz > 0 ? a0 : 0;
-#pragma unroll
-  for (int c = 0; c < 4; c++) {
-    const int cx = c == 0 ? ix - 1 : ix - 2 + c, cy = c == 0 ? iy : iy - 1;
-    int b0 = 0, b1 = 0, b2 = 0, b3 = 0;
-    if (!(cx < 0 || cx >= nx || cy < 0)) {
-      const int kb = (cy * nx + cx) * nz + iz;   // the grid holds fewer than 2^31 cells
-      b1 = cs[kb];
-      b2 = cs[kb + 1];
-      b0 = iz > 0 ? cs[kb - 1] : b1;
-      b3 = iz + 1 < nz ? cs[kb + 2] : b2;
-    }
-    L.ra[2 + c] = b0; L.rb[2 + c] = b3; L.zb1[c] = b1; L.zb2[c] = b2;
-  }
-}
-
-// the list of lane `src` (all lanes call)
-__device__ __forceinline__ void shfl_list(const CandList& mine, int src, CandList& L) {
-#pragma unroll
-  for (int r = 0; r < 6; r++) {
-    L.ra[r] = __shfl_sync(0xffffffffu, mine.ra[r], src);
-    L.rb[r] = __shfl_sync(0xffffffffu, mine.rb[r], src);
-  }
-#pragma unroll
-  for (int c = 0; c < 4; c++) {
-    L.zb1[c] = __shfl_sync(0xffffffffu, mine.zb1[c], src);
-    L.zb2[c] = __shfl_sync(0xffffffffu, mine.zb2[c], src);
-  }
-}
-
-__device__ __forceinline__ int list_len(const CandList& L) {
-  int m = 0;
-#pragma unroll
-  for (int r = 0; r < 6; r++) m += L.rb[r] - L.ra[r];
-  return m;
-}
-
-// sort position and corner-offset code of entry i of the list
-__device__ __forceinline__ void list_entry(const CandList& L, int i, int& t, int& cd) {
-  t = 0;
-  cd = 0;
-  int base = 0;
-#pragma unroll
-  for (int r = 0; r < 6; r++) {
-    const int len = L.rb[r] - L.ra[r];
-    if (i >= base && i < base + len) {
-      t = L.ra[r] + (i - base);
-      if (r == 1) {
-        cd = 1 << 4;
-      } else if (r >= 2) {
-        const int c = r - 2;
-        const int xy = (c <= 1 ? 1 : (c == 2 ? 0 : 2)) | (c == 0 ? 0 : 1) << 2;
-        cd = xy | (t < L.zb1[c] ? 1 : (t < L.zb2[c] ? 0 : 2)) << 4;
-      }
-    }
-    base += len;
-  }
-}
-
-__global__ void __launch_bounds__(kSearchWarps * 32, SDEM_SEARCH_MIN_BLOCKS) k_search_warp(Dev d, int s_begin, int s_end) {
-  __shared__ float4 st_q[kSearchWarps][2][kStage];
-  __shared__ int st_i[kSearchWarps][2][kStage];
-  __shared__ unsigned char st_c[kSearchWarps][2][kStage];
-  const unsigned FULL = 0xffffffffu;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int s0 = s_begin + (blockIdx.x * kSearchWarps + w) * 32;
-  if (s0 >= s_end) return;   // the whole warp
-  const int nt = *d.nt, nloc = *d.n;
-  const int K = d.K, Kin = d.Kin, nall = d.nall;
-  const float margin = d.pf_margin, cellf = d.cellf;
-  const int* __restrict__ cs = d.cell_start;
-  const int s_me = s0 + lane;
-  const bool live = s_me < s_end && s_me < nt;
-  if (s_me < s_end && s_me >= nt) d.row_cnt[s_me] = 0;
-  int m_me = 0, cnt_me = 0, key_me = -1;
-  float4 pf_me = make_float4(0.f, 0.f, 0.f, 0.f);
-  CandList mine;
-  if (live) {
-    m_me = d.sorted[s_me];
-    const int4 tc = d.pcell[m_me];
-    key_me = tc.w;
-    pf_me = d.spos[s_me];
-    cand_list(cs, tc.w, tc.x, tc.y, tc.z, d.nx, d.nz, mine);
-  } else {
-#pragma unroll
-    for (int r = 0; r < 6; r++) mine.ra[r] = mine.rb[r] = 0;
-#pragma unroll
-    for (int c = 0; c < 4; c++) mine.zb1[c] = mine.zb2[c] = 0;
-  }
-  // live targets are a prefix of the warp's lanes; a group starts where the
-  // cell changes (the sort order is the cell order)
-  const int nlive = __popc(__ballot_sync(FULL, live));
-  const int key_prev = __shfl_up_sync(FULL, key_me, 1);
-  unsigned leaders = __ballot_sync(FULL, live && (lane == 0 || key_me != key_prev));
-  unsigned long long cand = 0;
-
-  // stage the list of the group led by lane `lead` into buffer `buf` (copies
-  // only when it fits; one commit group either way)
-  auto stage = [&](int lead, int buf) -> int {
-    CandList L;
-    shfl_list(mine, lead, L);
-    const int M = list_len(L);
-    if (M <= kStage) {
-      for (int i = lane; i < M; i += 32) {
-        int t, cd;
-        list_entry(L, i, t, cd);
-        cp_async16(&st_q[w][buf][i], &d.spos[t]);
-        cp_async4(&st_i[w][buf][i], &d.sorted[t]);
-        st_c[w][buf][i] = (unsigned char)cd;
-      }
-    }
-    cp_async_commit();
-    return M;
-  };
-
-  // test candidates [lo, hi) of the buffer (entry i at i - base) for target lane jj
-  auto test_range = [&](int jj, int buf, int base, int lo, int hi) {
-    const int s_t = s0 + jj;
-    const int m_t = __shfl_sync(FULL, m_me, jj);
-    const bool img = m_t >= nloc;
-    float4 Pf;
-    Pf.x = __shfl_sync(FULL, pf_me.x, jj);
-    Pf.y = __shfl_sync(FULL, pf_me.y, jj);
-    Pf.z = __shfl_sync(FULL, pf_me.z, jj);
-    Pf.w = __shfl_sync(FULL, pf_me.w, jj);
-    int cnt_t = __shfl_sync(FULL, cnt_me, jj);
-    for (int i0 = lo; i0 < hi; i0 += 32) {
-      const int i = i0 + lane;
-      bool hit = false;
-      int q = 0;
-      if (i < hi) {
-        const float4 Qf = st_q[w][buf][i - base];
-        q = st_i[w][buf][i - base];
-        const int cd = st_c[w][buf][i - base];
-        if (!img || q < nloc) {   // an image or fixed target pairs with local particles only
-          cand++;
-          const float ox = corner_offset(cd & 3, cellf), oy = corner_offset((cd >> 2) & 3, cellf),
-                      oz = corner_offset((cd >> 4) & 3, cellf);
-          const float fx = (Pf.x - Qf.x) + ox, fy = (Pf.y - Qf.y) + oy, fz = (Pf.z - Qf.z) + oz;
-          const float d2f = fx * fx + fy * fy + fz * fz;
-          const float rs = Pf.w + Qf.w;
-          const float bhi = rs + margin;
-          if (!(d2f > bhi * bhi)) {
-            hit = true;
-            const float blo = rs - margin;
-            if (!(d2f < blo * blo)) {
-              const dbl4 Pm = d.posr[m_t], Pq = d.posr[q];
-              double dr = Pm.w + Pq.w;
-              double dr2 = dr * dr;
-              double dx = Pm.x - Pq.x;
-              double d2sum = dx * dx;
-              if (d2sum > dr2) hit = false;
-              double dy = Pm.y - Pq.y;
-              d2sum = dy * dy + d2sum;
-              if (d2sum > dr2) hit = false;
-              double dz = Pm.z - Pq.z;
-              d2sum = dz * dz + d2sum;
-              if (d2sum > dr2) hit = false;
-            }
-          }
-        }
-      }
-      const unsigned mask = __ballot_sync(FULL, hit);
-      if (hit) {
-        const int slot = cnt_t + __popc(mask & ((1u << lane) - 1u));
-        if (slot < K) {
-          d.row_partner[(size_t)slot * nall + s_t] = q;
-          if (q < nloc) {   // an image receives no force: it has no in-list
-            const int is = atomicAdd(&d.in_cnt[q], 1);
-            if (is < Kin) d.in_list[(size_t)q * Kin + is] = ((unsigned)s_t << 6) | (unsigned)slot;
-            else raise(d, SDEM_E_CL_FULL, q);
-          }
-        } else {
-          raise(d, SDEM_E_CL_FULL, m_t);
-        }
-      }
-      cnt_t += __popc(mask);
-    }
-    if (lane == jj) cnt_me = cnt_t;
-  };
-
-  if (nlive > 0) {
-    int lead = __ffs(leaders) - 1;
-    leaders &= leaders - 1;
-    int M = stage(lead, 0);
-    for (int g = 0; lead < nlive; g++) {
-      const int buf = g & 1;
-      const int next = leaders ? __ffs(leaders) - 1 : nlive;   // the next group's leader ends this group
-      int Mn = 0;
-      if (leaders) Mn = stage(next, buf ^ 1);
-      else cp_async_commit();
-      cp_async_wait_1();
-      __syncwarp();
-      const int a0 = __shfl_sync(FULL, mine.ra[0], lead);
-      if (M <= kStage) {
-        for (int jj = lead; jj < next; jj++) test_range(jj, buf, 0, s0 + jj - a0 + 1, M);
+// Wall contacts: FindContactsPW (Prtcl_ContactSearchPW.f90:308-317), one thread
+// per particle of the near-wall list.  The walk goes front-first, i.e. the
+// highest wall index first; slots j < kKw per particle keep that order, and
+// the compact list of contacts feeds k_force.
+// Latency bound: 13 us at 1M spheres (90k near a wall, 37k contacts), 8 us for
+// small beds, on the second stream beside the binning.  Over all particles with
+// their masks it took 73 us, one or two lanes of every warp in the wall tests;
+// with the forces in the same kernel 55 us, holding every SM's registers.
+constexpr int kWallThreads = 128;
+__global__ void __launch_bounds__(kWallThreads) k_wall_detect(Dev d) {
+  const int nn = *d.near_cnt;
+  const int ncap = d.ncap;
+  int total = 0;
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x) {
+    const int p = d.near_list[k];
+    unsigned long long mask = d.near_mask[p];
+    const dbl4 P = d.posr[p];
+    int nwc = 0;
+    while (mask) {
+      const int wi = 63 - __clzll((long long)mask);
+      mask &= ~(1ull << wi);
+      double ovrlp;
+      r3 nv;
+      if (!sdem::wall_contact(sdem::load_wall(d.walls, d.wflags, wi), P, ovrlp, nv)) continue;
+      if (nwc < kKw) {
+        d.w_wall[(size_t)nwc * ncap + p] = wi;
+        d.w_geo[(size_t)nwc * ncap + p] = make_dbl4(nv.x, nv.y, nv.z, ovrlp);
+        d.wl[atomicAdd(d.wl_cnt, 1)] = (p << 3) | nwc;
       } else {
-        // a list longer than the buffer: pieces staged with plain loads
-        CandList L;
-        shfl_list(mine, lead, L);
-        for (int pb = 0; pb < M; pb += kStage) {
-          const int pe = min(M, pb + kStage);
-          for (int i = pb + lane; i < pe; i += 32) {
-            int t, cd;
-            list_entry(L, i, t, cd);
-            st_q[w][buf][i - pb] = d.spos[t];
-            st_i[w][buf][i - pb] = d.sorted[t];
-            st_c[w][buf][i - pb] = (unsigned char)cd;
-          }
-          __syncwarp();
-          for (int jj = lead; jj < next; jj++) test_range(jj, buf, pb, max(s0 + jj - a0 + 1, pb), pe);
-          __syncwarp();
-        }
+        raise(d, SDEM_E_CL_FULL, p);
       }
-      __syncwarp();
-      lead = next;
-      if (leaders) leaders &= leaders - 1;
-      M = Mn;
+      nwc++;
     }
-    cp_async_wait_0();
+    const int kept = nwc < kKw ? nwc : kKw;
+    d.w_cnt[p] = kept;
+    d.wh_cnt[d.gid[p]] = kept;
+    total += nwc;
   }
-  if (live) d.row_cnt[s_me] = cnt_me < K ? cnt_me : K;
-  for (int o = 16; o > 0; o >>= 1) cand += __shfl_down_sync(FULL, cand, o);
-  if (lane == 0 && cand) atomicAdd(&d.counters[0], cand);
-}
-
-// Wall contacts of each particle: FindContactsPW (Prtcl_ContactSearchPW.f90:308-317)
-// walks the near-wall list front-first, i.e. the highest wall index first.
-// Slots j < kKw per particle keep that order; the compact list feeds k_wall_force.
-__global__ void __launch_bounds__(kThreads) k_wall_detect(Dev d) {
-  const int m = blockIdx.x * blockDim.x + threadIdx.x;
-  int nwc = 0;
-  if (m < *d.n) {
-    unsigned long long mask = d.near_mask[m];
-    if (mask) {
-      const dbl4 Pm = d.posr[m];
-      const int ncap = d.ncap;
-      while (mask) {
-        int wi = 63 - __clzll((long long)mask);
-        mask &= ~(1ull << wi);
-        sdem::Wall W = sdem::load_wall(d.walls, d.wflags, wi);
-        double ovrlp;
-        r3 nv;
-        if (!sdem::wall_contact(W, Pm, ovrlp, nv)) continue;
-        if (nwc < kKw) {
-          d.w_wall[(size_t)nwc * ncap + m] = wi;
-          d.w_geo[(size_t)nwc * ncap + m] = make_dbl4(nv.x, nv.y, nv.z, ovrlp);
-          int k = atomicAdd(d.wl_cnt, 1);
-          d.wl[k] = (m << 3) | nwc;
-        } else {
-          raise(d, SDEM_E_CL_FULL, m);
-        }
-        nwc++;
-      }
-    }
-    const int nw_c = nwc < kKw ? nwc : kKw;
-    d.w_cnt[m] = nw_c;
-    d.wh_cnt[d.gid[m]] = nw_c;
-    int deg = min(d.in_cnt[m], d.Kin) + d.row_cnt[d.sortpos[m]] + nw_c;
-    deg = deg < kDegBuckets - 1 ? deg : kDegBuckets - 1;
-    d.deg_of[m] = deg;
-    // warp-aggregated slot in the bucket: one atomic per distinct degree per warp
-    const unsigned act = __activemask();
-    const unsigned peers = __match_any_sync(act, deg);
-    const int lane = threadIdx.x & 31;
-    const int leader = __ffs(peers) - 1;
-    int base = 0;
-    if (lane == leader) base = atomicAdd(&d.deg_cnt[deg], __popc(peers));
-    base = __shfl_sync(peers, base, leader);
-    d.deg_rank[m] = base + __popc(peers & ((1u << lane) - 1u));
-  }
-  for (int o = 16; o > 0; o >>= 1) nwc += __shfl_down_sync(0xffffffffu, nwc, o);
-  if ((threadIdx.x & 31) == 0 && nwc) atomicAdd(&d.counters[1], (unsigned long long)nwc);
-}
-
-// Gather order: bucket starts (highest degree first; every block scans the
-// 64 bucket counts itself), then each particle to its bucket slot.
-__global__ void k_degree_scatter(Dev d) {
-  static_assert(kDegBuckets == 64, "two buckets per lane of one warp");
-  __shared__ int start[kDegBuckets];
-  if (threadIdx.x < 32) {
-    const int l = threadIdx.x;
-    const int b0 = kDegBuckets - 1 - 2 * l, b1 = b0 - 1;
-    const int c0 = d.deg_cnt[b0], c1 = d.deg_cnt[b1];
-    const int v = c0 + c1;
-    int incl = v;
-    for (int o = 1; o < 32; o <<= 1) {
-      const int t = __shfl_up_sync(0xffffffffu, incl, o);
-      if (l >= o) incl += t;
-    }
-    start[b0] = incl - v;
-    start[b1] = incl - v + c0;
-  }
-  __syncthreads();
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= *d.n) return;
-  // what the gather needs first, read here in index order (coalesced, apart
-  // from the row of p) and stored at the gather position in one record
-  const int s = d.sortpos[p];
-  const int nin = min(d.in_cnt[p], d.Kin);
-  GRec g;
-  g.p = p;
-  g.s = s;
-  g.own_a = d.row_off[s];
-  g.counts = (d.row_cnt[s] << 16) | (nin << 8) | d.w_cnt[p];
-  g.r = d.posr[p].w;
-  g.pad = 0.0;
-  d.gorder[start[d.deg_of[p]] + d.deg_rank[p]] = g;
-}
-
-// One thread per wall contact: Find_insert on the particle's bucket (key = wall)
-// + ContactForce_PW (Prtcl_CL_and_CF.f90:227-249, 832-856).
-__global__ void __launch_bounds__(kThreads) k_wall_force(Dev d) {
-  const int nwl = *d.wl_cnt;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nwl; k += gridDim.x * blockDim.x) {
-    const int e = d.wl[k];
-    const int p = e >> 3, j = e & 7;
-    const size_t at = (size_t)j * d.ncap + p;
-    const int wi = d.w_wall[at];
-    const dbl4 geo = d.w_geo[at];
-    const int g = d.gid[p];
-    dbl4 hist = make_dbl4(0.0, 0.0, 0.0, -2.0);
-    const int pc = d.wh_cnt_prev[g];
-    for (int i = 0; i < pc; i++)
-      if (d.wh_wall_prev[(size_t)g * kKw + i] == wi) { hist = d.wh_hist_prev[(size_t)g * kKw + i]; break; }
-    sdem::Wall W = sdem::load_wall(d.walls, d.wflags, wi);
-    const double* P = d.bpw + ((size_t)(W.wall_type - 1) * d.nT + (d.ptype[p] - 1)) * SDEM_BP_SIZE;
-    const double ri = d.posr[p].w;
-    r3 S, M, Mr;
-    // "the normal vector points from particle i to j": Norm_v = (-1)*nv (:849-851)
-    r3 Norm_v = sdem::scale3(sdem::mk3(geo.x, geo.y, geo.z), -1.0);
-    sdem::force_law(d.law, P, sdem::xyz(d.vel0[p]), W.vel, sdem::xyz(d.rv0[p]), sdem::mk3(0.0, 0.0, 0.0), ri,
-                    1.00E20 * ri, Norm_v, geo.w, hist, S, M, Mr);
-    d.w_S[at] = sdem::d4(S, 0.0);
-    d.w_M[at] = sdem::d4(M, 0.0);   // Moment (the gather scales it by ri)
-    d.w_Mr[at] = sdem::d4(Mr, 0.0);
-    d.wh_wall[(size_t)g * kKw + j] = wi;
-    d.wh_hist[(size_t)g * kKw + j] = hist;
-  }
-}
-
-// Each contact's row (its target's sort position) for the rows [s_begin, s_end),
-// so that the one-thread-per-contact force kernel reads its row instead of
-// searching the row offsets.
-__global__ void k_row_fill(Dev d, int s_begin, int s_end) {
-  const int s = s_begin + blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= s_end) return;
-  const int a = d.row_off[s], k = d.row_cnt[s];
-  for (int j = 0; j < k; j++)
-    if (a + j < d.ccap) d.c_row[a + j] = s;
+  for (int o = 16; o > 0; o >>= 1) total += __shfl_down_sync(0xffffffffu, total, o);
+  if ((threadIdx.x & 31) == 0 && total) atomicAdd(&d.counters[1], (unsigned long long)total);
 }
 
 // ---------------------------------------------------------------------------
 // One thread per contact: Find_insert's history lookup + ContactForce_PP.
-// Contacts of the rows [s_begin, s_end).  kOneSided: the search holds periodic
+// Contacts of one chunk of the search.  kOneSided: the search holds periodic
 // images or fixed spheres (pairs whose force goes to one sphere only).
 template <bool kOneSided>
-__global__ void __launch_bounds__(kThreads, SDEM_FORCE_MIN_BLOCKS) k_force(Dev d, int s_begin, int s_end) {
+__global__ void __launch_bounds__(kThreads, SDEM_FORCE_MIN_BLOCKS) k_force(Dev d, int chunk) {
   const int nloc = *d.n;
-  const int c0 = d.row_off[s_begin], C = d.row_off[s_end];
-  if (C > d.ccap) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) raise(d, SDEM_E_CL_FULL, C);
+  int c0 = 0;
+  for (int k = 0; k < chunk; k++) c0 += d.c_cnt[k];
+  const int npp = d.c_cnt[chunk];
+  if (c0 + npp > d.ccap) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) raise(d, SDEM_E_CL_FULL, c0 + npp);
     return;
   }
+  // the first chunk's launch also takes the wall contacts, after the pairs
+  const int items = npp + (chunk == 0 ? *d.wl_cnt : 0);
   unsigned long long nimg = 0, nfx = 0;
   const int first_fixed = nloc + *d.ng;   // search index of the first fixed sphere
-  for (int c = c0 + blockIdx.x * blockDim.x + threadIdx.x; c < C; c += gridDim.x * blockDim.x) {
-    const int s = d.c_row[c];
-    const int slot = c - d.row_off[s];
-    int m = d.sorted[s];
-    int q = d.row_partner[(size_t)slot * d.nall + s];
-    // both particles' state records; the velocity records carry id and type
-    const dbl4 Pm = d.posr[m], Pq = d.posr[q];
-    const dbl4 Vm = d.vel0[m], Vq = d.vel0[q], Wm = d.rv0[m], Wq = d.rv0[q];
-    const int gm = tag_gid(Vm.w), gq = tag_gid(Vq.w);
-    // particle-particle (AddContactPP) or local-image (AddContactPPG) pair; the
-    // lower id is particle i of the force law either way
-    // (Prtcl_NBS_Munjiza.f90:525-529, Prtcl_CL_and_CF.f90:773-797)
-    const bool img = kOneSided && ((m >= nloc) || (q >= nloc));
-    const bool m_loc = m < nloc;              // the local particle of an image pair is m
-    const int oth = m_loc ? q : m;
-    const bool m_lo = gm < gq;
-    // Find_insert's bucket: the lower id's for PP, the local particle's for PPG
-    const int owner = img ? (m_loc ? gm : gq) : (m_lo ? gm : gq);
-    const int partner = img ? (m_loc ? gq : gm) : (m_lo ? gq : gm);
-    const dbl4 Pi = m_lo ? Pm : Pq, Pj = m_lo ? Pq : Pm;
-    const dbl4 Vi = m_lo ? Vm : Vq, Vj = m_lo ? Vq : Vm;
-    const dbl4 Wi = m_lo ? Wm : Wq, Wj = m_lo ? Wq : Wm;
-    // Prtcl_BnryProp(pType(lower id), pType(higher id)) for PP (:743),
-    // (pType(local), pType(image)) for PPG (:772)
-    const int tm = tag_type(Vm.w), tq = tag_type(Vq.w);
-    const int ta = img ? (m_loc ? tm : tq) : (m_lo ? tm : tq);
-    const int tb = img ? (m_loc ? tq : tm) : (m_lo ? tq : tm);
+  for (int it = blockIdx.x * blockDim.x + threadIdx.x; it < items; it += gridDim.x * blockDim.x) {
+    const bool pp = it < npp;
+    r3 Veli, Velj, Rvei, Rvej, Norm_v;
+    double ri, rj, ovrlp;
+    const double* P;
     dbl4 hist = make_dbl4(0.0, 0.0, 0.0, -2.0);
-    {
-      const int2* oe = d.own_c_prev + (size_t)owner * d.Ko;
-      // the first entry is read beside the count (the table always holds Ko
-      // entries per owner; an entry past the count is not used)
-      const int2 e0 = oe[0];
-      const int k = d.own_cnt_prev[owner];
-      if (k > 0 && e0.y == partner) {
-        hist = d.c_hist_prev[e0.x];
-      } else {
-        for (int j = 1; j < k; j++) {
-          const int2 e = oe[j];
-          if (e.y == partner) { hist = d.c_hist_prev[e.x]; break; }
+    bool img = false, m_lo = true;
+    int owner, partner, oth = 0;   // a pair: its bucket; a wall contact: particle and slot
+    if (pp) {
+      const int2 mq = d.c_pair[c0 + it];
+      const int m = mq.x, q = mq.y;
+      // both particles' state records; the velocity records carry id and type
+      const dbl4 Pm = d.posr[m], Pq = d.posr[q];
+      const dbl4 Vm = d.vel0[m], Vq = d.vel0[q], Wm = d.rv0[m], Wq = d.rv0[q];
+      const int gm = tag_gid(Vm.w), gq = tag_gid(Vq.w);
+      // particle-particle (AddContactPP) or local-image (AddContactPPG) pair; the
+      // lower id is particle i of the force law either way
+      // (Prtcl_NBS_Munjiza.f90:525-529, Prtcl_CL_and_CF.f90:773-797)
+      img = kOneSided && ((m >= nloc) || (q >= nloc));
+      const bool m_loc = m < nloc;              // the local particle of an image pair is m
+      oth = m_loc ? q : m;
+      m_lo = gm < gq;
+      // Find_insert's bucket: the lower id's for PP, the local particle's for PPG
+      owner = img ? (m_loc ? gm : gq) : (m_lo ? gm : gq);
+      partner = img ? (m_loc ? gq : gm) : (m_lo ? gq : gm);
+      const dbl4 Pi = m_lo ? Pm : Pq, Pj = m_lo ? Pq : Pm;
+      Veli = sdem::xyz(m_lo ? Vm : Vq);
+      Velj = sdem::xyz(m_lo ? Vq : Vm);
+      Rvei = sdem::xyz(m_lo ? Wm : Wq);
+      Rvej = sdem::xyz(m_lo ? Wq : Wm);
+      // Prtcl_BnryProp(pType(lower id), pType(higher id)) for PP (:743),
+      // (pType(local), pType(image)) for PPG (:772)
+      const int tm = tag_type(Vm.w), tq = tag_type(Vq.w);
+      const int ta = img ? (m_loc ? tm : tq) : (m_lo ? tm : tq);
+      const int tb = img ? (m_loc ? tq : tm) : (m_lo ? tq : tm);
+      {
+        const int2* oe = d.own_c_prev + (size_t)owner * d.Ko;
+        // the first entry is read beside the count (the table always holds Ko
+        // entries per owner; an entry past the count is not used)
+        const int2 e0 = oe[0];
+        const int k = d.own_cnt_prev[owner];
+        if (k > 0 && e0.y == partner) {
+          hist = d.c_hist_prev[e0.x];
+        } else {
+          for (int j = 1; j < k; j++) {
+            const int2 e = oe[j];
+            if (e.y == partner) { hist = d.c_hist_prev[e.x]; break; }
+          }
         }
       }
+      P = d.bpp + ((size_t)(tb - 1) * d.nT + (ta - 1)) * SDEM_BP_SIZE;
+      // Norm_v = Posj .nv. Posi (real4_nv, Prtcl_TypeDef.f90:268-281) and
+      // ovrlp = dr - sqrt(d2sum) (NBSM_FineSearch2/3, Prtcl_NBS_Munjiza.f90:514-522)
+      // share one length: d2sum = dz*dz + (dy*dy + dx*dx) is bitwise
+      // (sx*sx + sy*sy) + sz*sz for s = Posj - Posi (squares ignore the sign and
+      // a two-term IEEE sum is commutative).
+      const r3 sv = sdem::sub3(sdem::xyz(Pj), sdem::xyz(Pi));
+      const double normv = sdem::norm3(sv);
+      ri = Pi.w;
+      rj = Pj.w;
+      ovrlp = (ri + rj) - normv;
+      Norm_v = fpi::gt(normv, 1.0000E-10) ? sdem::div3(sv, normv) : sdem::mk3(0.0, 0.0, 0.0);
+    } else {
+      // a wall contact: Find_insert on the particle's bucket (key = wall) +
+      // ContactForce_PW (Prtcl_CL_and_CF.f90:227-249, 832-856)
+      const int e = d.wl[it - npp];
+      owner = e >> 3;
+      partner = e & 7;
+      const size_t at = (size_t)partner * d.ncap + owner;
+      const int wi = d.w_wall[at];
+      const dbl4 geo = d.w_geo[at], V = d.vel0[owner];
+      const int g = tag_gid(V.w);
+      const int pc = d.wh_cnt_prev[g];
+      for (int i = 0; i < pc; i++)
+        if (d.wh_wall_prev[(size_t)g * kKw + i] == wi) { hist = d.wh_hist_prev[(size_t)g * kKw + i]; break; }
+      const double* wv = d.walls + (size_t)wi * SDEM_W_SIZE + SDEM_W_VEL;
+      P = d.bpw + ((size_t)(d.wflags[wi * SDEM_WF_SIZE + SDEM_WF_WALL_TYPE] - 1) * d.nT + (tag_type(V.w) - 1)) * SDEM_BP_SIZE;
+      Veli = sdem::xyz(V);
+      Velj = sdem::mk3(wv[0], wv[1], wv[2]);
+      Rvei = sdem::xyz(d.rv0[owner]);
+      Rvej = sdem::mk3(0.0, 0.0, 0.0);
+      ri = d.posr[owner].w;
+      rj = 1.00E20 * ri;
+      ovrlp = geo.w;
+      // "the normal vector points from particle i to j": Norm_v = (-1)*nv (:849-851)
+      Norm_v = sdem::scale3(sdem::mk3(geo.x, geo.y, geo.z), -1.0);
     }
-    const double* P = d.bpp + ((size_t)(tb - 1) * d.nT + (ta - 1)) * SDEM_BP_SIZE;
-    // Norm_v = Posj .nv. Posi (real4_nv, Prtcl_TypeDef.f90:268-281) and
-    // ovrlp = dr - sqrt(d2sum) (NBSM_FineSearch2/3, Prtcl_NBS_Munjiza.f90:514-522)
-    // share one length: d2sum = dz*dz + (dy*dy + dx*dx) is bitwise
-    // (sx*sx + sy*sy) + sz*sz for s = Posj - Posi (squares ignore the sign and
-    // a two-term IEEE sum is commutative).
-    const r3 sv = sdem::sub3(sdem::xyz(Pj), sdem::xyz(Pi));
-    const double normv = sdem::norm3(sv);
-    const double ovrlp = (Pi.w + Pj.w) - normv;
-    r3 Norm_v = fpi::gt(normv, 1.0000E-10) ? sdem::div3(sv, normv) : sdem::mk3(0.0, 0.0, 0.0);
     r3 S, M, Mr;
-    sdem::force_law(d.law, P, sdem::xyz(Vi), sdem::xyz(Vj), sdem::xyz(Wi), sdem::xyz(Wj), Pi.w, Pj.w, Norm_v, ovrlp,
-                    hist, S, M, Mr);
+    sdem::force_law(d.law, P, Veli, Velj, Rvei, Rvej, ri, rj, Norm_v, ovrlp, hist, S, M, Mr);
+    if (!pp) {
+      const size_t at = (size_t)partner * d.ncap + owner;
+      d.w_S[at] = sdem::d4(S, 0.0);
+      d.w_M[at] = sdem::d4(M, 0.0);   // Moment (the gather scales it by the radius)
+      d.w_Mr[at] = sdem::d4(Mr, 0.0);
+      const size_t gs = (size_t)d.gid[owner] * kKw + partner;
+      d.wh_wall[gs] = d.w_wall[at];
+      d.wh_hist[gs] = hist;
+      continue;
+    }
+    const int c = c0 + it;
     d.c_ogid[c] = owner | (img ? kImgFlag : 0);
     d.c_pgid[c] = partner;
     d.c_hist[c] = hist;
@@ -1386,100 +1196,6 @@ __device__ __forceinline__ void sort_net(unsigned (&v)[N]) {
           else { v[i] = hi; v[l] = lo; }
         }
       }
-}
-
-__global__ void __launch_bounds__(kThreads) k_gather(Dev d) {
-  const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-  if (tid >= *d.n) return;
-  const GRec gr = d.gorder[tid];
-  const int p = gr.p, s = gr.s;
-  const int ncap = d.ncap;
-  const double rp = gr.r;
-  r3 F = sdem::mk3(0.0, 0.0, 0.0), T = sdem::mk3(0.0, 0.0, 0.0);
-
-  // The contact records of p in the reference's scatter order: in-list
-  // entries of earlier targets, p's own row, in-list entries of later
-  // targets, then wall contacts.  Their indices go to a small per-thread list
-  // first (integer work), so the FP64 additions run in one loop whose trip
-  // count is the warp's maximum, not once per branch.
-  const int own_a = gr.own_a, own_n = gr.counts >> 16;
-  const int nin = (gr.counts >> 8) & 0xFF;
-  const int nwc = gr.counts & 0xFF;
-  // entry: (contact index << 1) | (p is the row's target), or -(wall slot + 1)
-  int list[2 * kMaxK + kKw];
-  int nl = 0;
-  auto push_in = [&](unsigned key) { list[nl++] = (d.row_off[key >> 6] + (int)(key & 63u)) << 1; };
-  auto push_own = [&]() {
-    for (int j = 0; j < own_n; j++) list[nl++] = ((own_a + j) << 1) | 1;
-  };
-  if (nin <= 8) {
-    unsigned u[8];
-#pragma unroll
-    for (int k = 0; k < 8; k++) u[k] = k < nin ? d.in_list[(size_t)p * d.Kin + k] : 0xffffffffu;
-    sort_net<8>(u);
-#pragma unroll
-    for (int k = 0; k < 8; k++)
-      if (k < nin && (int)(u[k] >> 6) < s) push_in(u[k]);
-    push_own();
-#pragma unroll
-    for (int k = 0; k < 8; k++)
-      if (k < nin && (int)(u[k] >> 6) > s) push_in(u[k]);
-  } else if (nin <= 16) {
-    unsigned u[16];
-#pragma unroll
-    for (int k = 0; k < 16; k++) u[k] = k < nin ? d.in_list[(size_t)p * d.Kin + k] : 0xffffffffu;
-    sort_net<16>(u);
-#pragma unroll
-    for (int k = 0; k < 16; k++)
-      if (k < nin && (int)(u[k] >> 6) < s) push_in(u[k]);
-    push_own();
-#pragma unroll
-    for (int k = 0; k < 16; k++)
-      if (k < nin && (int)(u[k] >> 6) > s) push_in(u[k]);
-  } else {
-    unsigned e[kMaxK];
-    for (int k = 0; k < nin; k++) {
-      unsigned v = d.in_list[(size_t)p * d.Kin + k];
-      int j = k - 1;
-      while (j >= 0 && e[j] > v) { e[j + 1] = e[j]; j--; }
-      e[j + 1] = v;
-    }
-    int k = 0;
-    for (; k < nin && (int)(e[k] >> 6) < s; k++) push_in(e[k]);
-    push_own();
-    for (; k < nin; k++) push_in(e[k]);
-  }
-  for (int j = 0; j < nwc; j++) list[nl++] = -(j + 1);
-
-  for (int k = 0; k < nl; k++) {
-    const int e = list[k];
-    const int c = e >= 0 ? (e >> 1) : e;
-    const bool tgt = e < 0 || (e & 1);   // a wall record or p's own row: as stored
-    dbl4 S, Ms, Mr;
-    if (c >= 0) {
-      const ContactRec& rec = d.c_rec[c];
-      S = rec.S;
-      Ms = rec.M;
-      Mr = rec.Mr;
-    } else {
-      const size_t at = (size_t)(-c - 1) * ncap + p;
-      S = d.w_S[at];
-      Ms = d.w_M[at];
-      Mr = d.w_Mr[at];
-    }
-    // F(pid) + (Fnij+Ftij) / F(pjd) - (Fnij+Ftij);
-    // T + r*Moment + Mrij / T + r*Moment - Mrij  (Prtcl_ContactForce_inc.f90:69-86).
-    // The records are signed for the row's target; the partner adds their
-    // negations (x - y is x + (-y) in IEEE arithmetic), so that every lane
-    // runs the same FP64 additions.
-    const uint64_t sg = tgt ? 0ull : fpi::kSign;
-    auto flip = [sg](double v) { return fpi::from_bits(fpi::bits(v) ^ sg); };
-    F = sdem::add3(F, sdem::mk3(flip(S.x), flip(S.y), flip(S.z)));
-    // r*Moment with p's own radius (ri*Moment or rj*Moment of the reference)
-    T = sdem::add3(sdem::add3(T, sdem::scale3(sdem::xyz(Ms), rp)), sdem::mk3(flip(Mr.x), flip(Mr.y), flip(Mr.z)));
-  }
-  d.F[p] = sdem::d4(F, 0.0);
-  d.T[p] = sdem::d4(T, 0.0);
 }
 
 // Per particle: clc_Acceleration, Prtcl_Integrate and the periodic wrap /
@@ -1620,13 +1336,6 @@ __device__ __forceinline__ void integrate_body(const Dev& d, const int p, const 
     if (k2 < kOutCap) d.out_list[k2] = p;
     else raise(d, SDEM_E_CAPACITY, p);
   }
-}
-
-// The update in index order, one thread per particle (coalesced records).
-__global__ void __launch_bounds__(kThreads) k_integrate(Dev d) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= *d.n) return;
-  integrate_body(d, p, [&](int f) { return int_src(d, f)[p]; });
 }
 
 // ---------------------------------------------------------------------------
@@ -1917,8 +1626,22 @@ __global__ void k_pack3(double* __restrict__ dst, const dbl4* __restrict__ src, 
 // Ends a step: the counters of the step (CL and search logs), running sums and
 // per-step resets.
 __device__ void step_end_serial(const Dev& d, int* counters_out) {
+  // the next step's start: no images yet; the near-wall list is made anew when
+  // the masks are due or particles were deleted (others have their indices)
+  *d.ng = 0;
+  *d.nt = *d.n;
+  if (*d.out_cnt > 0 || *d.iter + 1 >= *d.next_update) {
+    *d.near_cnt = 0;
+    *d.near_stale = 1;
+  }
+
   // every value first (the loads issue together), then the stores
-  const int C = d.row_off[d.nall_launch];
+  int C = 0;
+  for (int k = 0; k < kMaxChunks; k++) {
+    C += d.c_cnt[k];
+    d.c_cnt[k] = 0;
+  }
+  d.row_off[d.nall_launch] = C;   // the contact snapshot's count
   const unsigned long long cnsv = d.counters[0], pw = d.counters[1], ppg = d.counters[5], fx = d.counters[8],
                            cross = d.counters[9];
   const int n = *d.n, it = *d.iter + 1, next = *d.next_update;
@@ -1945,25 +1668,203 @@ __device__ void step_end_serial(const Dev& d, int* counters_out) {
   *d.wl_cnt = 0;
 }
 
-// The end of a step in one block: the serial delete passes (thread 0), the
-// moves they imply (all threads), the counters (thread 0), then a copy of the
-// device scalars (status, particle count, counters) into mapped host memory,
-// one word per thread, so that the host reads them after a stream
+// What the last block of a step's last kernel writes: the counters and a copy
+// of the device scalars (status, particle count, counters) in mapped host
+// memory, one word per thread, so that the host reads them after a stream
 // synchronisation without another copy.  Two mirror slots, by the parity of
 // the new iteration number: a step's copy survives while the next step runs.
-__global__ void k_finish(Dev d, int* counters_out, const int* scal, int* mirror, int nscal) {
-  if (threadIdx.x == 0) delete_serial(d);
+struct StepEnd {
+  int* counters;
+  const int* scal;
+  int* mirror;
+  int nscal;
+};
+
+// The end of a step, by the last block of the kernel that updates the
+// particles: the serial delete passes (thread 0), the moves they imply (all
+// threads), the counters (thread 0), the mirror.  As a kernel of its own it
+// cost a launch (4 us) of every step.
+__device__ void end_step(const Dev& d, const StepEnd& e) {
+  __shared__ int last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(d.ticket + 1, 1) == (int)gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  if (threadIdx.x == 0) {
+    d.ticket[1] = 0;
+    delete_serial(d);
+  }
   __syncthreads();
   apply_moves(d, threadIdx.x, blockDim.x);
   __syncthreads();
-  if (threadIdx.x == 0) step_end_serial(d, counters_out);
+  if (threadIdx.x == 0) step_end_serial(d, e.counters);
   __syncthreads();
-  if (mirror && threadIdx.x < nscal) {
-    int* slot = mirror + (*d.iter & 1) * nscal;
-    slot[threadIdx.x] = scal[threadIdx.x];
+  if (e.mirror && (int)threadIdx.x < e.nscal) {
+    int* slot = e.mirror + (*d.iter & 1) * e.nscal;
+    slot[threadIdx.x] = e.scal[threadIdx.x];
   }
 }
 
+// The update in index order, one thread per particle (coalesced records).
+__global__ void __launch_bounds__(kThreads) k_integrate(Dev d, StepEnd end) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p < *d.n) integrate_body(d, p, [&](int f) { return int_src(d, f)[p]; });
+  end_step(d, end);
+}
+
+// The sums of the particle at sort position s, and with kUpdate its update.
+template <bool kUpdate>
+__device__ __forceinline__ void gather_one(const Dev& d, const int s) {
+  const int p = d.sorted[s];
+  const int ncap = d.ncap;
+  const double rp = d.posr[p].w;
+  r3 F = sdem::mk3(0.0, 0.0, 0.0), T = sdem::mk3(0.0, 0.0, 0.0);
+
+  // The contact records of p in the reference's scatter order: in-list
+  // entries of earlier targets, p's own row, in-list entries of later
+  // targets, then wall contacts.  Their indices go to a small per-thread list
+  // first (integer work), so the FP64 additions run in one loop whose trip
+  // count is the warp's maximum, not once per branch.
+  const int own_a = d.row_off[s], own_n = d.row_cnt[s];
+  const int nin = min(d.in_cnt[s], d.Kin);
+  const int nwc = d.w_cnt[p];
+  const unsigned* __restrict__ inl = d.in_list + (size_t)s * d.Kin;
+  // entry: (contact index << 1) | (p is the row's target), or -(wall slot + 1)
+  int list[2 * kMaxK + kKw];
+  int nl = 0;
+  auto push_in = [&](unsigned key) { list[nl++] = (d.row_off[key >> 6] + (int)(key & 63u)) << 1; };
+  auto push_own = [&]() {
+    for (int j = 0; j < own_n; j++) list[nl++] = ((own_a + j) << 1) | 1;
+  };
+  if (nin <= 8) {
+    unsigned u[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) u[k] = k < nin ? inl[k] : 0xffffffffu;
+    sort_net<8>(u);
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+      if (k < nin && (int)(u[k] >> 6) < s) push_in(u[k]);
+    push_own();
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+      if (k < nin && (int)(u[k] >> 6) > s) push_in(u[k]);
+  } else if (nin <= 16) {
+    unsigned u[16];
+#pragma unroll
+    for (int k = 0; k < 16; k++) u[k] = k < nin ? inl[k] : 0xffffffffu;
+    sort_net<16>(u);
+#pragma unroll
+    for (int k = 0; k < 16; k++)
+      if (k < nin && (int)(u[k] >> 6) < s) push_in(u[k]);
+    push_own();
+#pragma unroll
+    for (int k = 0; k < 16; k++)
+      if (k < nin && (int)(u[k] >> 6) > s) push_in(u[k]);
+  } else {
+    unsigned e[kMaxK];
+    for (int k = 0; k < nin; k++) {
+      unsigned v = inl[k];
+      int j = k - 1;
+      while (j >= 0 && e[j] > v) { e[j + 1] = e[j]; j--; }
+      e[j + 1] = v;
+    }
+    int k = 0;
+    for (; k < nin && (int)(e[k] >> 6) < s; k++) push_in(e[k]);
+    push_own();
+    for (; k < nin; k++) push_in(e[k]);
+  }
+  for (int j = 0; j < nwc; j++) list[nl++] = -(j + 1);
+
+  for (int k = 0; k < nl; k++) {
+    const int e = list[k];
+    const int c = e >= 0 ? (e >> 1) : e;
+    const bool tgt = e < 0 || (e & 1);   // a wall record or p's own row: as stored
+    dbl4 S, Ms, Mr;
+    if (c >= 0) {
+      if (c >= d.ccap) continue;   // past the capacity: reported by k_force, nothing was computed
+      const ContactRec& rec = d.c_rec[c];
+      S = rec.S;
+      Ms = rec.M;
+      Mr = rec.Mr;
+    } else {
+      const size_t at = (size_t)(-c - 1) * ncap + p;
+      S = d.w_S[at];
+      Ms = d.w_M[at];
+      Mr = d.w_Mr[at];
+    }
+    // F(pid) + (Fnij+Ftij) / F(pjd) - (Fnij+Ftij);
+    // T + r*Moment + Mrij / T + r*Moment - Mrij  (Prtcl_ContactForce_inc.f90:69-86).
+    // The records are signed for the row's target; the partner adds their
+    // negations (x - y is x + (-y) in IEEE arithmetic), so that every lane
+    // runs the same FP64 additions.
+    const uint64_t sg = tgt ? 0ull : fpi::kSign;
+    auto flip = [sg](double v) { return fpi::from_bits(fpi::bits(v) ^ sg); };
+    F = sdem::add3(F, sdem::mk3(flip(S.x), flip(S.y), flip(S.z)));
+    // r*Moment with p's own radius (ri*Moment or rj*Moment of the reference)
+    T = sdem::add3(sdem::add3(T, sdem::scale3(sdem::xyz(Ms), rp)), sdem::mk3(flip(Mr.x), flip(Mr.y), flip(Mr.z)));
+  }
+  d.F[p] = sdem::d4(F, 0.0);
+  d.T[p] = sdem::d4(T, 0.0);
+  if (kUpdate)
+    integrate_body(d, p, [&](int f) { return f == IF_F ? sdem::d4(F, 0.0) : (f == IF_T ? sdem::d4(T, 0.0) : int_src(d, f)[p]); });
+}
+
+
+// One block takes kThreads consecutive sort positions, i.e. spheres that lie
+// side by side: the rows are read coalesced, and a contact's 96-byte record,
+// which its two spheres read, comes from DRAM once and from L2 the second
+// time.  Inside the block the spheres are ordered by their number of records
+// (a counting sort in shared memory), so that a warp's summation loops run
+// equal trip counts.
+// FP64-pipe bound (68% busy at 1M spheres, 1.5 contacts each; DRAM 3.5 TB/s):
+// 121 us there, as the gather over a global order by record count took, without
+// that order's kernel (24 us) and its share of the wall kernel; 423 B of DRAM a
+// sphere instead of 773.
+template <bool kUpdate>
+__global__ void __launch_bounds__(kThreads) k_gather(Dev d, StepEnd end) {
+  static_assert(kDegBuckets == 64, "two buckets per lane of one warp");
+  __shared__ int bucket[kDegBuckets];
+  __shared__ int order[kThreads];
+  __shared__ int members;
+  const int s0 = blockIdx.x * kThreads;
+  const int nloc = *d.n;
+  {
+    const int s = s0 + threadIdx.x;
+    if (threadIdx.x < kDegBuckets) bucket[threadIdx.x] = 0;
+    __syncthreads();
+    int deg = -1, rank = 0;
+    if (s < *d.nt) {
+      const int p = d.sorted[s];
+      if (p < nloc) {   // images and fixed spheres receive no force
+        deg = min(d.row_cnt[s] + min(d.in_cnt[s], d.Kin) + d.w_cnt[p], kDegBuckets - 1);
+        rank = atomicAdd(&bucket[deg], 1);
+      }
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {   // bucket starts, the most records first
+      const int l = threadIdx.x;
+      const int b0 = kDegBuckets - 1 - 2 * l, b1 = b0 - 1;
+      const int c0 = bucket[b0], v = c0 + bucket[b1];
+      int incl = v;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (l >= o) incl += t;
+      }
+      bucket[b0] = incl - v;
+      bucket[b1] = incl - v + c0;
+      if (l == 31) members = incl;
+    }
+    __syncthreads();
+    if (deg >= 0) order[bucket[deg] + rank] = s;
+    __syncthreads();
+  }
+  if ((int)threadIdx.x < members) gather_one<kUpdate>(d, order[threadIdx.x]);
+  if (kUpdate) end_step(d, end);
+}
 // ---------------------------------------------------------------------------
 // Allocation-free contact count (sdem_count_contacts_noalloc).
 //
@@ -1987,7 +1888,8 @@ struct NoAllocScratch {
   int sortpos[kNaMaxN];
   float4 spos[kNaMaxN];
   float4 pf[kNaMaxN];
-  int bsum[kNaBlocks];
+  ScanCtl ctl;
+  unsigned long long words[kNaBlocks];
   int n;
   int status[2];
   unsigned long long counts[2];   // exact contacts, candidate pairs
@@ -2000,6 +1902,8 @@ __global__ void k_na_begin(NoAllocScratch* S, int n) {
   S->status[1] = 0;
   S->counts[0] = 0ull;
   S->counts[1] = 0ull;
+  S->ctl.ticket = 0;
+  S->ctl.done = 0;
 }
 
 // The search of k_search without its rows: the same half shell, the same
@@ -2113,8 +2017,7 @@ struct sdem_h {
   double cell = 0, x0 = 0, y0 = 0, z0 = 0;
   int nx = 0, ny = 0, nz = 0;
   long long ncell = 0;
-  int *cell_cnt = nullptr, *cell_start = nullptr, *scan_tmp = nullptr;
-  size_t scan_tmp_n = 0;
+  int *cell_cnt = nullptr, *cell_start = nullptr;
   // particles
   int n_host = 0;  // count at upload (upper bound of the device count)
   int *gid = nullptr, *ptype = nullptr, *usrmark = nullptr;
@@ -2126,7 +2029,8 @@ struct sdem_h {
   int *row_cnt = nullptr, *row_partner = nullptr, *row_off = nullptr, *in_cnt = nullptr;
   unsigned* in_list = nullptr;
   int ccap = 0;
-  int *c_ogid = nullptr, *c_pgid[2] = {}, *own_cnt[2] = {}, *c_row = nullptr;
+  int *c_ogid = nullptr, *c_pgid[2] = {}, *own_cnt[2] = {}, *c_cnt = nullptr;
+  int2* c_pair = nullptr;
   int2* own_c[2] = {};
   int nall = 0, gcap = 0;
   int fcap = 0, nfix = 0;
@@ -2136,7 +2040,8 @@ struct sdem_h {
   int* type_lvl = nullptr;
   int *fix_gid = nullptr, *fix_ptype = nullptr;
   dbl4* fix_posr = nullptr;
-  int *gflag = nullptr, *goff = nullptr;
+  ScanCtl *gctl = nullptr, *cctl = nullptr;           // ghost passes; cell scan
+  unsigned long long *gwords = nullptr, *cwords = nullptr;
   // particle-particle records as uploaded (reported until the first step):
   // owner id, partner id, listed under the partner too
   struct UpRec { int owner, partner; bool both; dbl4 hist; };
@@ -2145,17 +2050,15 @@ struct sdem_h {
   ContactRec* c_rec = nullptr;
   int *wh_cnt[2] = {}, *wh_wall[2] = {};
   dbl4* wh_hist[2] = {};
-  int *w_cnt = nullptr, *w_wall = nullptr, *wl = nullptr;
+  int *w_cnt = nullptr, *w_wall = nullptr, *wl = nullptr, *near_list = nullptr;
   dbl4 *w_geo = nullptr, *w_S = nullptr, *w_M = nullptr, *w_Mr = nullptr;
   float4* spos = nullptr;
   float4* pf = nullptr;
   int4* pcell = nullptr;
   float pf_margin = 0.f;
-  int *deg_cnt = nullptr, *deg_of = nullptr, *deg_rank = nullptr;
-  GRec* gorder = nullptr;
   // second stream and events of the chunked search/force pipeline
   cudaStream_t stream2 = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_rows = nullptr, ev_chunk[kMaxChunks] = {};
+  cudaEvent_t ev_fork = nullptr, ev_cells = nullptr, ev_wall = nullptr, ev_chunk[kMaxChunks] = {};
   int nchunk = kChunks;                  // launch shape (sdem_set_launch); results do not depend on it
   int force_bps = kForceBlocksPerSM;
   int first_pct = 0;                     // percent of the targets in the first chunk (0: whole search waves)
@@ -2262,8 +2165,9 @@ int ensure_stage(sdem_h* h, size_t count) {
   return 0;
 }
 
-enum { S_N = 0, S_STATUS = 1, S_ITER = 3, S_NEXT = 4, S_OUTCNT = 5, S_WLCNT = 6, S_NG = 7, S_COUNTERS = 8,  // counters: 8..16
-       S_NT = 20, S_TICKET = 21, S_SIZE = 24 };
+enum { S_N = 0, S_STATUS = 1, S_ITER = 3, S_NEXT = 4, S_OUTCNT = 5, S_NEARCNT = 6, S_NG = 7, S_COUNTERS = 8,  // counters: 8..16
+       S_NT = 20, S_TICKET = 21,  // two tickets
+       S_STALE = 23, S_WLCNT = 24, S_SIZE = 28 };
 
 Dev make_dev(sdem_h* h) {
   Dev d{};
@@ -2290,8 +2194,8 @@ Dev make_dev(sdem_h* h) {
   d.lencs = h->cell;
   d.dmin = make_double3(c.dom_min[0], c.dom_min[1], c.dom_min[2]);
   d.dmax = make_double3(c.dom_max[0], c.dom_max[1], c.dom_max[2]);
-  d.gflag = h->gflag;
-  d.goff = h->goff;
+  d.gctl = h->gctl;
+  d.gwords = h->gwords;
   d.max_gid = c.max_gid;
   d.K = h->K;
   d.Kin = h->K;
@@ -2360,20 +2264,19 @@ Dev make_dev(sdem_h* h) {
   d.pf = h->pf;
   d.pcell = h->pcell;
   d.cdiv = fpi::divisor(h->cell);
-  d.deg_cnt = h->deg_cnt;
-  d.deg_of = h->deg_of;
-  d.deg_rank = h->deg_rank;
-  d.gorder = h->gorder;
   d.pf_margin = h->pf_margin;
   d.cellf = (float)h->cell;
   d.w_cnt = h->w_cnt;
-  d.w_wall = h->w_wall;
-  d.w_geo = h->w_geo;
   d.w_S = h->w_S;
   d.w_M = h->w_M;
   d.w_Mr = h->w_Mr;
+  d.w_wall = h->w_wall;
+  d.w_geo = h->w_geo;
   d.wl = h->wl;
   d.wl_cnt = h->scal + S_WLCNT;
+  d.near_list = h->near_list;
+  d.near_cnt = h->scal + S_NEARCNT;
+  d.near_stale = h->scal + S_STALE;
   d.row_cnt = h->row_cnt;
   d.row_partner = h->row_partner;
   d.row_off = h->row_off;
@@ -2387,7 +2290,8 @@ Dev make_dev(sdem_h* h) {
   d.c_hist_prev = h->c_hist[pv];
   d.c_rec = h->c_rec;
   d.Ko = h->K;
-  d.c_row = h->c_row;
+  d.c_cnt = h->c_cnt;
+  d.c_pair = h->c_pair;
   d.own_cnt = h->own_cnt[cu];
   d.own_c = h->own_c[cu];
   d.own_cnt_prev = h->own_cnt[pv];
@@ -2413,13 +2317,7 @@ Dev make_dev(sdem_h* h) {
 
 int grid_for(long long n) { return (int)std::max<long long>(1, (n + kThreads - 1) / kThreads); }
 
-void scan(sdem_h* h, const int* in, long long n, int* out, const int* offset = nullptr) {
-  int nb = (int)std::max<long long>(1, (n + kScanTile - 1) / kScanTile);
-  k_scan_reduce<<<nb, kScanThreads, 0, h->stream>>>(in, n, h->scan_tmp);
-  k_scan_blocks<<<1, 1024, 0, h->stream>>>(h->scan_tmp, nb);
-  k_scan_apply<<<nb, kScanThreads, 0, h->stream>>>(in, n, h->scan_tmp, out, offset);
-}
-
+constexpr int kUpdateTogether = 131072;   // most search positions whose sums and update share a kernel
 int enqueue_step(sdem_h* h) {
   Dev d = make_dev(h);
   int n = h->n_host;
@@ -2430,10 +2328,22 @@ int enqueue_step(sdem_h* h) {
     if (ev) cudaEventRecord(ev[ph], st);
   };
   long long L = 0;
+  // Profiling runs one chunk on one stream, so that every phase has its own
+  // events.
+  const int nchunk = ev ? 1 : h->nchunk;
+  cudaStream_t s2 = ev ? st : h->stream2;
   mark(PH_WALL);
-  // the refresh schedule (Next_iter_update) advances with or without walls
-  k_step_begin<<<h->num_sms * kBeginBlocksPerSM, kThreads, 0, st>>>(d);
-  L += 1;
+  // The walls need positions and velocities only: they run on the second
+  // stream beside the images, the binning and the sort.  The refresh schedule
+  // (Next_iter_update) advances with or without walls.
+  if (s2 != st) {
+    cudaEventRecord(h->ev_fork, st);
+    cudaStreamWaitEvent(s2, h->ev_fork, 0);
+  }
+  k_step_begin<<<h->num_sms * kBeginBlocksPerSM, kThreads, 0, s2>>>(d);
+  k_wall_detect<<<h->num_sms * 4, kWallThreads, 0, s2>>>(d);
+  if (s2 != st) cudaEventRecord(h->ev_wall, s2);
+  L += 2;
   mark(PH_BIN);
   const int na = n + h->gcap + h->nfix;   // search arrays: locals, periodic images, fixed spheres
   if (h->gcap > 0) {
@@ -2442,42 +2352,36 @@ int enqueue_step(sdem_h* h) {
     const int pdir[5] = {1, 0, 0, 2, 2};
     for (int k = 0; k < 5; k++) {
       if (!per[pdir[k]]) continue;
-      k_ghost_flag<<<grid_for(na), kThreads, 0, st>>>(d, passes[k]);
-      scan(h, h->gflag, na, h->goff);
-      k_ghost_scatter<<<grid_for(na), kThreads, 0, st>>>(d, passes[k]);
-      k_ghost_count<<<1, 1, 0, st>>>(d);
-      L += 6;
+      k_ghost<<<(na + kGhostTile - 1) / kGhostTile, kThreads, 0, st>>>(d, passes[k]);
+      L += 1;
     }
   }
   if (h->nfix > 0) {
     k_fixed_append<<<grid_for(h->nfix), kThreads, 0, st>>>(d);
     L += 1;
   }
-  cudaMemsetAsync(h->cell_cnt, 0, sizeof(int) * (size_t)h->ncell, st);
-  cudaMemsetAsync(h->in_cnt, 0, sizeof(int) * (size_t)std::max(n, 1), st);
   k_bin<<<grid_for(na), kThreads, 0, st>>>(d);
   mark(PH_SCAN_CELLS);
-  scan(h, h->cell_cnt, h->ncell, h->cell_start);
+  L += scan_cells(h->cell_cnt, h->ncell, h->cell_start, h->cctl, h->cwords, h->scal + S_STATUS, st);
   mark(PH_SCATTER);
   k_scatter<<<grid_for(na), kThreads, 0, st>>>(d);
   mark(PH_CELLORDER);
   k_cellorder<<<grid_for(na), kThreads, 0, st>>>(d);
   mark(PH_SEARCH);
-  // Chunked pipeline: the searches of all chunks, then wall detection and wall
-  // forces, run on the second stream; each chunk's row offsets (continuing
-  // the previous chunk's total), contact rows and forces run on the main
-  // stream as soon as its search is done.  Profiling runs one chunk on one
-  // stream, so that every phase has its own events.
-  const int nchunk = ev ? 1 : h->nchunk;
-  cudaStream_t s2 = ev ? st : h->stream2;
-  // chunk boundaries on scan tiles, so that each chunk's row scan moves whole
-  // aligned tiles
-  // The first chunk's search runs alone, before any force: by default it
-  // takes as many whole waves of resident search blocks as fit in an even
-  // share, when that trims the share by a quarter at most, so that its last
-  // wave is full (a partial last wave takes a whole wave's time); or
-  // first_pct percent of the targets.  The other chunks share the rest
-  // evenly.
+  // Chunked pipeline (more than one chunk): the searches of all chunks run on
+  // the second stream (after the walls) and lay out their rows' contacts; each
+  // chunk's forces run on the main stream as soon as its search is done.  With
+  // one chunk, the default, the search stays on the main stream and waits for
+  // nothing but the sort.  k_force holds every SM's registers, so a search
+  // gains little from running beside it, and every chunk adds a partial last
+  // round of forces: 1 / 2 / 3 chunks take 60 / 80 / 98 us per step at 20k
+  // spheres, 198 / 237 / 228 at 200k, 695 / 761 / 693 at 1M.
+  // Chunk boundaries lie on whole search blocks.  The first chunk's search
+  // runs alone, before any force: by default it takes as many whole waves of
+  // resident search blocks as fit in an even share, when that trims the share
+  // by a quarter at most, so that its last wave is full (a partial last wave
+  // takes a whole wave's time); or first_pct percent of the targets.  The other
+  // chunks share the rest evenly.
   long long first = -1;
   if (nchunk > 1) {
     const long long wave = (long long)h->num_sms * kSearchBlocksPerSM * kThreads;
@@ -2489,66 +2393,51 @@ int enqueue_step(sdem_h* h) {
     if (k == 0) return 0;
     if (k == nchunk) return na;
     const long long c = first < 0 ? (long long)na * k / nchunk : first + (na - first) * (k - 1) / (nchunk - 1);
-    return (int)(c & ~(long long)(kScanTile - 1));
+    return (int)(c & ~(long long)(kThreads - 1));
   };
-  if (s2 != st) {
-    cudaEventRecord(h->ev_fork, st);
-    cudaStreamWaitEvent(s2, h->ev_fork, 0);
+  const bool piped = nchunk > 1;
+  cudaStream_t sr = piped ? s2 : st;
+  if (piped) {
+    cudaEventRecord(h->ev_cells, st);
+    cudaStreamWaitEvent(s2, h->ev_cells, 0);
   }
   for (int k = 0; k < nchunk; k++) {
     const int a = cut(k), b = cut(k + 1);
-    if (h->hier) k_search<true><<<grid_for(std::max(b - a, 1)), kThreads, 0, s2>>>(d, a, b);
-    else if (!SDEM_SEARCH_WARP) k_search<false><<<grid_for(std::max(b - a, 1)), kThreads, 0, s2>>>(d, a, b);
-    else {
-      const long long warps = (std::max(b - a, 1) + 31) / 32;
-      k_search_warp<<<(int)((warps + kSearchWarps - 1) / kSearchWarps), kSearchWarps * 32, 0, s2>>>(d, a, b);
-    }
-    if (s2 != st) cudaEventRecord(h->ev_chunk[k], s2);
+    if (h->hier) k_search<true><<<grid_for(std::max(b - a, 1)), kThreads, 0, sr>>>(d, a, b, k);
+    else k_search<false><<<grid_for(std::max(b - a, 1)), kThreads, 0, sr>>>(d, a, b, k);
+    if (piped) cudaEventRecord(h->ev_chunk[k], s2);
   }
-  k_wall_detect<<<grid_for(n), kThreads, 0, s2>>>(d);
-  if (s2 == st) {
-    mark(PH_SCAN_ROWS);
-    scan(h, h->row_cnt, na, h->row_off);
-    mark(PH_ROW_FILL);
-    k_row_fill<<<grid_for(na), kThreads, 0, st>>>(d, 0, na);
-    mark(PH_FORCE);
-    if (h->gcap > 0 || h->nfix > 0) k_force<true><<<h->num_sms * 8, kThreads, 0, st>>>(d, 0, na);
-    else k_force<false><<<h->num_sms * 8, kThreads, 0, st>>>(d, 0, na);
-    mark(PH_WALL_FORCE);
-    k_wall_force<<<std::max(1, h->num_sms * 2), kThreads, 0, st>>>(d);
-  } else {
-    k_wall_force<<<std::max(1, h->num_sms * 2), kThreads, 0, s2>>>(d);
-    for (int k = 0; k < nchunk; k++) {
-      const int a = cut(k), b = cut(k + 1);
-      cudaStreamWaitEvent(st, h->ev_chunk[k], 0);
-      scan(h, h->row_cnt + a, b - a, h->row_off + a, k ? h->row_off + a : nullptr);
-      if (k == nchunk - 1) {
-        // every row offset is known: the gather order (which needs them and
-        // the wall contacts, not the forces) is built on the second stream
-        // beside the last forces
-        cudaEventRecord(h->ev_rows, st);
-        cudaStreamWaitEvent(s2, h->ev_rows, 0);
-        k_degree_scatter<<<grid_for(n), kThreads, 0, s2>>>(d);
-        cudaEventRecord(h->ev_join, s2);
-      }
-      k_row_fill<<<grid_for(std::max(b - a, 1)), kThreads, 0, st>>>(d, a, b);
-      if (h->gcap > 0 || h->nfix > 0) k_force<true><<<h->num_sms * h->force_bps, kThreads, 0, st>>>(d, a, b);
-      else k_force<false><<<h->num_sms * h->force_bps, kThreads, 0, st>>>(d, a, b);
-    }
-    cudaStreamWaitEvent(st, h->ev_join, 0);
+  mark(PH_SCAN_ROWS);   // rows and their contacts are laid out by the search: these two phases are empty
+  mark(PH_ROW_FILL);
+  mark(PH_FORCE);
+  if (s2 != st && !piped) cudaStreamWaitEvent(st, h->ev_wall, 0);
+  for (int k = 0; k < nchunk; k++) {
+    if (piped) cudaStreamWaitEvent(st, h->ev_chunk[k], 0);
+    const int blocks = h->num_sms * (ev ? 8 : h->force_bps);
+    if (h->gcap > 0 || h->nfix > 0) k_force<true><<<blocks, kThreads, 0, st>>>(d, k);
+    else k_force<false><<<blocks, kThreads, 0, st>>>(d, k);
   }
+  mark(PH_WALL_FORCE);   // wall forces are part of the force kernel: this phase is empty
   mark(PH_GATHER);
-  if (s2 == st) k_degree_scatter<<<grid_for(n), kThreads, 0, st>>>(d);
-  k_gather<<<grid_for(n), kThreads, 0, st>>>(d);
-  k_integrate<<<grid_for(n), kThreads, 0, st>>>(d);
-  mark(PH_DELETE);
-  k_finish<<<1, kThreads, 0, st>>>(d, h->scal + S_COUNTERS, h->scal, h->d_mirror, S_SIZE);
+  const StepEnd end{h->scal + S_COUNTERS, h->scal, h->d_mirror, S_SIZE};
+  // Sums and update in one kernel while the state (~640 B a sphere) sits in
+  // L2; beyond, the update in index order reads and writes whole lines where
+  // the sums' order would scatter 32-byte records.  One kernel against two,
+  // per step: 100k spheres 126 / 132 us, 20k 60.4 / 62.4, 200k 200.8 / 198.2,
+  // 400k 357 / 322, 1M 896 / 695.
+  const bool together = na <= kUpdateTogether;
+  if (together) {
+    k_gather<true><<<grid_for(na), kThreads, 0, st>>>(d, end);
+  } else {
+    k_gather<false><<<grid_for(na), kThreads, 0, st>>>(d, end);
+    k_integrate<<<grid_for(n), kThreads, 0, st>>>(d, end);
+  }
+  mark(PH_DELETE);   // the end of the step is part of the update kernel: these two phases are empty
   mark(PH_END);
   h->mirror_ok = true;
   mark(kPhases);
-  // bin, scan, scatter, cellorder, wall detect, wall force, degree scatter,
-  // gather, integrate, finish; per chunk search, scan (3), row fill, force
-  L += 1 + 3 + 1 + 1 + 1 + 1 + 3 + 1 + 6 * nchunk;
+  // bin, scatter, cellorder, gather, integrate; per chunk search, force
+  L += 1 + 1 + 1 + (together ? 1 : 2) + 2 * nchunk;
   h->launches += L;
   if (ev) h->prof_steps++;
   h->cur = 1 - h->cur;
@@ -2692,8 +2581,8 @@ int sdem_create(const sdem_cfg* cfg, sdem_h** out) {
   CK(cudaEventCreateWithFlags(&h->ev_snap, cudaEventDisableTiming));
   CK(cudaEventCreateWithFlags(&h->ev_snap_done, cudaEventDisableTiming));
   CK(cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming));
-  CK(cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming));
-  CK(cudaEventCreateWithFlags(&h->ev_rows, cudaEventDisableTiming));
+  CK(cudaEventCreateWithFlags(&h->ev_cells, cudaEventDisableTiming));
+  CK(cudaEventCreateWithFlags(&h->ev_wall, cudaEventDisableTiming));
   for (int k = 0; k < 6; k++) CK(cudaEventCreateWithFlags(&h->ev_xfer[k], cudaEventDisableTiming));
   for (int k = 0; k < kMaxChunks; k++) CK(cudaEventCreateWithFlags(&h->ev_chunk[k], cudaEventDisableTiming));
   int N = c.n_capacity;
@@ -2723,8 +2612,8 @@ int sdem_create(const sdem_cfg* cfg, sdem_h** out) {
     if (k < c.rsize) { rc |= dalloc(h, &h->rv[k], k == 0 ? NA : N); rc |= dalloc(h, &h->ra[k], N); }
   }
   if (h->gcap > 0) {
-    rc |= dalloc(h, &h->gflag, (size_t)NA);
-    rc |= dalloc(h, &h->goff, (size_t)NA + 1);
+    rc |= dalloc(h, &h->gctl, 1);
+    rc |= dalloc(h, &h->gwords, (size_t)NA / kGhostTile + 1);
   }
   if (h->fcap > 0) {
     rc |= dalloc(h, &h->fix_gid, (size_t)h->fcap);
@@ -2743,25 +2632,23 @@ int sdem_create(const sdem_cfg* cfg, sdem_h** out) {
   rc |= dalloc(h, &h->spos, NA);
   rc |= dalloc(h, &h->pf, NA);
   rc |= dalloc(h, &h->pcell, NA);
-  rc |= dalloc(h, &h->deg_cnt, kDegBuckets);
-  rc |= dalloc(h, &h->deg_of, N);
-  rc |= dalloc(h, &h->deg_rank, N);
-  rc |= dalloc(h, &h->gorder, N);
   rc |= dalloc(h, &h->w_cnt, N);
   rc |= dalloc(h, &h->w_wall, (size_t)N * kKw);
   rc |= dalloc(h, &h->wl, (size_t)N * kKw);
   rc |= dalloc(h, &h->w_geo, (size_t)N * kKw);
+  rc |= dalloc(h, &h->near_list, N);
   rc |= dalloc(h, &h->w_S, (size_t)N * kKw);
   rc |= dalloc(h, &h->w_M, (size_t)N * kKw);
   rc |= dalloc(h, &h->w_Mr, (size_t)N * kKw);
   rc |= dalloc(h, &h->row_cnt, NA);
   rc |= dalloc(h, &h->row_off, (size_t)NA + 1);
   rc |= dalloc(h, &h->row_partner, (size_t)NA * h->K);
-  rc |= dalloc(h, &h->in_cnt, N);
-  rc |= dalloc(h, &h->in_list, (size_t)N * h->K);
+  rc |= dalloc(h, &h->in_cnt, NA);
+  rc |= dalloc(h, &h->in_list, (size_t)NA * h->K);
   h->ccap = std::max(1, c.cntct_list_size) * N;
   rc |= dalloc(h, &h->c_ogid, h->ccap);
-  rc |= dalloc(h, &h->c_row, h->ccap);
+  rc |= dalloc(h, &h->c_pair, h->ccap);
+  rc |= dalloc(h, &h->c_cnt, kMaxChunks);
   rc |= dalloc(h, &h->c_rec, h->ccap);
   size_t G = (size_t)c.max_gid + 1;
   for (int b = 0; b < 2; b++) {
@@ -2780,7 +2667,6 @@ int sdem_create(const sdem_cfg* cfg, sdem_h** out) {
   rc |= dalloc(h, &h->moves, 1 + 2 * 5 * kOutCap + 5 * kOutCap);
   rc |= dalloc(h, &h->map_pos, 5 * kOutCap);
   rc |= dalloc(h, &h->map_id, 5 * kOutCap);
-  rc |= dalloc(h, &h->scan_tmp, 65536);
   if (rc) return SDEM_E_NOMEM;
   CK(cudaMallocHost(&h->h_counters, sizeof(int) * SDEM_CNT_SIZE));
   CK(cudaHostAlloc((void**)&h->h_mirror, sizeof(int) * 2 * S_SIZE, cudaHostAllocMapped));
@@ -2899,12 +2785,9 @@ int sdem_set_types(sdem_h* h, int nT, const double* radius, const double* mass, 
   if (h->ncell >= (1ll << 31) - 1) return set_err(h, SDEM_E_ARG, "search grid has more than 2^31 cells");
   rc |= dalloc(h, &h->cell_cnt, (size_t)h->ncell);
   rc |= dalloc(h, &h->cell_start, (size_t)h->ncell + 1);
+  rc |= dalloc(h, &h->cctl, 1);
+  rc |= dalloc(h, &h->cwords, (size_t)scan_tiles(h->ncell));
   if (rc) return SDEM_E_NOMEM;
-  long long nb = std::max<long long>((h->ncell + kScanTile - 1) / kScanTile, ((long long)h->nall + kScanTile - 1) / kScanTile);
-  if (nb > 65536) {
-    rc |= dalloc(h, &h->scan_tmp, (size_t)nb);
-    if (rc) return SDEM_E_NOMEM;
-  }
   CK(cudaStreamSynchronize(h->stream));
   h->have_types = true;
   return 0;
@@ -2937,9 +2820,11 @@ int sdem_set_walls(sdem_h* h, int nw, const double* wall, const int* flags) {
     CK(cudaMemcpyAsync(h->wflags, flags, sizeof(int) * nw * SDEM_WF_SIZE, cudaMemcpyHostToDevice, h->stream));
   }
   drop_graph(h);
-  // the near-wall list is rebuilt at the next step
-  int zero = 0;
+  // the near-wall masks and list are rebuilt at the next step
+  const int zero = 0, one = 1;
   CK(cudaMemcpyAsync(h->scal + S_NEXT, &zero, sizeof zero, cudaMemcpyHostToDevice, h->stream));
+  CK(cudaMemcpyAsync(h->scal + S_NEARCNT, &zero, sizeof zero, cudaMemcpyHostToDevice, h->stream));
+  CK(cudaMemcpyAsync(h->scal + S_STALE, &one, sizeof one, cudaMemcpyHostToDevice, h->stream));
   h->mirror_ok = false;
   CK(cudaStreamSynchronize(h->stream));
   return 0;
@@ -3048,6 +2933,7 @@ int sdem_upload_particles(sdem_h* h, int n, const int* id, const int* ptype, con
   int sc[S_SIZE] = {0};
   sc[S_N] = n;
   sc[S_NT] = n;
+  sc[S_STALE] = 1;
   CK(cudaMemcpyAsync(h->scal, sc, sizeof sc, cudaMemcpyHostToDevice, st));
   CK(cudaMemsetAsync(h->ull, 0, sizeof(unsigned long long) * 10, st));
   CK(cudaGetLastError());
@@ -3837,12 +3723,7 @@ int sdem_count_contacts_noalloc(const sdem_cfg* cfg, double max_radius, int n, c
   if (cudaMemsetAsync(S->cell_cnt, 0, sizeof(int) * (size_t)ncell, st) != cudaSuccess)
     return noalloc_fail(SDEM_E_CUDA, "sdem_count_contacts_noalloc: cudaMemsetAsync failed");
   k_bin<<<g, kThreads, 0, st>>>(d);
-  {
-    const int nb = (int)std::max<long long>(1, (ncell + kScanTile - 1) / kScanTile);
-    k_scan_reduce<<<nb, kScanThreads, 0, st>>>(S->cell_cnt, ncell, S->bsum);
-    k_scan_blocks<<<1, 1024, 0, st>>>(S->bsum, nb);
-    k_scan_apply<<<nb, kScanThreads, 0, st>>>(S->cell_cnt, ncell, S->bsum, S->cell_start, nullptr);
-  }
+  scan_cells(S->cell_cnt, ncell, S->cell_start, &S->ctl, S->words, S->status, st);
   k_scatter<<<g, kThreads, 0, st>>>(d);
   k_cellorder<<<g, kThreads, 0, st>>>(d);
   k_na_count<<<g, kThreads, 0, st>>>(d, S->counts);
@@ -3963,8 +3844,8 @@ void sdem_destroy(sdem_h* h) {
   if (h->ev_fork) cudaEventDestroy(h->ev_fork);
   for (int b = 0; b < 2; b++)
     if (h->ev_step[b]) cudaEventDestroy(h->ev_step[b]);
-  if (h->ev_join) cudaEventDestroy(h->ev_join);
-  if (h->ev_rows) cudaEventDestroy(h->ev_rows);
+  if (h->ev_cells) cudaEventDestroy(h->ev_cells);
+  if (h->ev_wall) cudaEventDestroy(h->ev_wall);
   for (int k = 0; k < 6; k++)
     if (h->ev_xfer[k]) cudaEventDestroy(h->ev_xfer[k]);
   for (int k = 0; k < kMaxChunks; k++)
