@@ -6,13 +6,14 @@
 //                                   order (neighbour cell, then sphere index);
 //   k_node_feat                     node features (velocity frames, spin,
 //                                   size, plane distances) as bf16;
-//   k_gemm                          one tensor-core GEMM for every layer of
-//                                   the network, forward and backward:
-//                                   C = A . B^T over operands that may be
+//   k_gemm_rows, k_gemm_wgrad       the network's layers on tcgen05, forward and
+//                                   backward: C = A . B^T over operands that may be
 //                                   row-gathered, split in column segments
 //                                   (concatenated edge/node inputs) and read
 //                                   transposed (weight gradients), with a
 //                                   fused bias/ReLU/mask/residual epilogue;
+//   k_gemm_tc, k_gemm               the same for other shapes: tcgen05 with B read
+//                                   per tile, and mma.sync for every form;
 //   k_split_reduce, k_colsum*       deterministic reductions (split-K weight
 //                                   gradients, bias gradients);
 //   k_segsum, k_gather_add          message aggregation and its adjoints;
@@ -28,6 +29,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <math.h>
+#include <algorithm>
 #include <stdint.h>
 
 #include "../../include/sdem_surrogate.h"
@@ -302,7 +304,7 @@ __global__ void __launch_bounds__(GT) k_gemm(int I, int J, int R, Operand A, Ope
 constexpr int TC_M = 128, TC_N = 128, TC_K = 32, TC_T = 256, TC_STAGES = 4;
 constexpr int TC_TILE = TC_M * TC_K * 2;          // bytes of one operand slice (8 KB)
 constexpr int TC_SMEM = TC_STAGES * 2 * TC_TILE;  // 64 KB: A and B slices of every stage
-constexpr long long TC_WAIT_LIMIT = 1ll << 26;
+constexpr int TC_WAIT_LIMIT = 1 << 22;
 constexpr uint32_t TC_IDESC = (1u << 4)                        // D: fp32
                               | (1u << 7) | (1u << 10)         // A, B: bf16
                               | ((uint32_t)(TC_N >> 3) << 17)  // N / 8
@@ -318,7 +320,7 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr) {
 }
 
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-    for (long long it = 0; it < TC_WAIT_LIMIT; ++it) {
+    for (int it = 0; it < TC_WAIT_LIMIT; ++it) {
         uint32_t done;
         asm volatile(
             "{\n .reg .pred P;\n mbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n selp.u32 %0, 1, 0, P;\n}\n"
@@ -481,12 +483,533 @@ __global__ void __launch_bounds__(TC_T, 1) k_gemm_tc(int I, int J, int R, Operan
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TC_N) : "memory");
 }
 
+// ------------------------------------------- tcgen05, weight kept in shared memory
+// The forms whose B fits in shared memory whole (every layer of the network:
+// forward C = [gathered rows] . W^T and input gradient C = dY . W): one
+// persistent CTA per SM keeps B there, K-major, for all its 128-row tiles, so
+// that a tile moves its A rows and nothing else (k_gemm_tc, which reads B anew
+// for every tile, moves twice as much).  Roles: warps 4-7 copy A slices of 64
+// reduction elements with cp.async into a ring of six (four to five in flight); one
+// thread of warp 8 issues the tcgen05.mma's into a ring of four 128-column
+// accumulators in tensor memory; warps 0-3 drain them, each thread one row,
+// with 32-byte global accesses straight from registers, while the next
+// accumulators fill.  Shared-memory operands are K-major with the 128-byte
+// swizzle: element (row, k) of a 64-wide slice at row * 128 bytes + ((k / 8) xor
+// (row mod 8)) * 16.  The reduction runs in the same order and steps of 16 as
+// in k_gemm_tc and k_gemm, and the results are the same bits.
+// Bound by L2 on the gathered forward form (600k rows, R = 384: 117 us, 5.9 TB/s
+// of L2; k_gemm_tc 328 us) and by HBM on the input gradient (J = 384, fp32 out:
+// 206 us, 5.0 TB/s; k_gemm 1150 us).
+constexpr int RW_M = 128, RW_K = 64, RW_STAGES = 6, RW_LAG = 5, RW_ACC = 4, RW_T = 288;
+constexpr int RW_SLICE = RW_M * RW_K * 2;              // 16 KB
+constexpr int RW_B_MAX = 98304;                        // bytes of B kept
+constexpr int RW_J_MAX = 384;
+
+__device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
+    return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(sbo >> 4) << 32) |
+           (1ull << 46) | (2ull << 61);
+}
+
+__device__ __forceinline__ void mbar_init(uint64_t* b, int count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(b)), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t* b) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(b)) : "memory");
+}
+__device__ __forceinline__ void tc_commit(uint64_t* b) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_u32(b))
+                 : "memory");
+}
+__device__ __forceinline__ void tc_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool acc) {
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
+        "l"(a), "l"(b), "r"(idesc), "r"(acc ? 1u : 0u)
+        : "memory");
+}
+// 32 accumulator columns of this warp's lane quarter
+__device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t (&r)[32]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+        "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+          "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+          "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+}
+// 32-byte global accesses (one sector a thread)
+__device__ __forceinline__ void st8(void* p, const uint32_t* v) {
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]),
+                 "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                 : "memory");
+}
+__device__ __forceinline__ void ld8(const void* p, uint32_t* v) {
+    asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "l"(p));
+}
+__device__ __forceinline__ uint32_t bf16_pair(float lo, float hi) {
+    return (uint32_t)bf16_bits(lo) | (uint32_t)bf16_bits(hi) << 16;
+}
+
+// The epilogue of 32 columns gj0.. of row gi, held by one thread.  `wide`: every
+// pointer and leading dimension allows 32-byte accesses, and all 32 columns exist.
+__device__ __forceinline__ void epilogue32(const sdem_sg_epilogue& ep, bool wide, const float* __restrict__ bias,
+                                           int gi, int gj0, int J, uint32_t (&r)[32]) {
+    if (wide) {
+        if (ep.bias) {
+#pragma unroll
+            for (int q = 0; q < 32; ++q) r[q] = __float_as_uint(__uint_as_float(r[q]) + bias[gj0 + q]);
+        }
+        if (ep.relu) {
+#pragma unroll
+            for (int q = 0; q < 32; ++q) r[q] = __float_as_uint(fmaxf(__uint_as_float(r[q]), 0.f));
+        }
+        if (ep.mask) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                uint32_t m[8];
+                ld8(ep.mask + (size_t)gi * ep.ld_mask + gj0 + 16 * h, m);
+#pragma unroll
+                for (int q = 0; q < 16; ++q)
+                    if (!bf16_positive((uint16_t)(m[q >> 1] >> (16 * (q & 1))))) r[16 * h + q] = 0u;
+            }
+        }
+        if (ep.out) {
+            float* o = ep.out + (size_t)gi * ep.ld_out + gj0;
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+                if (ep.accumulate) {
+                    uint32_t a[8];
+                    ld8(o + 8 * h, a);
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        a[q] = __float_as_uint(__uint_as_float(a[q]) + __uint_as_float(r[8 * h + q]));
+                    st8(o + 8 * h, a);
+                } else {
+                    st8(o + 8 * h, r + 8 * h);
+                }
+            }
+        }
+        if (ep.out_bf) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                uint32_t b[8];
+#pragma unroll
+                for (int q = 0; q < 8; ++q)
+                    b[q] = bf16_pair(__uint_as_float(r[16 * h + 2 * q]), __uint_as_float(r[16 * h + 2 * q + 1]));
+                st8(ep.out_bf + (size_t)gi * ep.ld_out_bf + gj0 + 16 * h, b);
+            }
+        }
+        if (ep.resid) {
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+                uint32_t a[8];
+                ld8(ep.resid + (size_t)gi * ep.ld_resid + gj0 + 8 * h, a);
+#pragma unroll
+                for (int q = 0; q < 8; ++q)
+                    r[8 * h + q] = __float_as_uint(__uint_as_float(a[q]) + __uint_as_float(r[8 * h + q]));
+                if (ep.res_out) st8(ep.res_out + (size_t)gi * ep.ld_res_out + gj0 + 8 * h, r + 8 * h);
+            }
+            if (ep.res_out_bf) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    uint32_t b[8];
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        b[q] = bf16_pair(__uint_as_float(r[16 * h + 2 * q]), __uint_as_float(r[16 * h + 2 * q + 1]));
+                    st8(ep.res_out_bf + (size_t)gi * ep.ld_res_out_bf + gj0 + 16 * h, b);
+                }
+            }
+        }
+        return;
+    }
+#pragma unroll
+    for (int q = 0; q < 32; ++q) {
+        const int gj = gj0 + q;
+        if (gj >= J) continue;
+        float v = __uint_as_float(r[q]);
+        if (ep.bias) v += bias[gj];
+        if (ep.relu) v = fmaxf(v, 0.f);
+        if (ep.mask && !bf16_positive(ep.mask[(size_t)gi * ep.ld_mask + gj])) v = 0.f;
+        if (ep.out) {
+            float* o = ep.out + (size_t)gi * ep.ld_out + gj;
+            *o = ep.accumulate ? *o + v : v;
+        }
+        if (ep.out_bf) ep.out_bf[(size_t)gi * ep.ld_out_bf + gj] = bf16_bits(v);
+        if (ep.resid) {
+            const float w = ep.resid[(size_t)gi * ep.ld_resid + gj] + v;
+            if (ep.res_out) ep.res_out[(size_t)gi * ep.ld_res_out + gj] = w;
+            if (ep.res_out_bf) ep.res_out_bf[(size_t)gi * ep.ld_res_out_bf + gj] = bf16_bits(w);
+        }
+    }
+}
+
+// B (J x R) into shared memory: 64-wide slices of jpad rows, 128-byte swizzle; zeros beyond J and R
+__device__ __forceinline__ void stage_b(uint8_t* Bs, const Operand& B, int J, int jpad, int R, int kslices) {
+    if (B.trans == 0) {
+        for (int c = threadIdx.x; c < jpad * kslices * 8; c += blockDim.x) {
+            const int j = c / (kslices * 8), kc = c % (kslices * 8);
+            uint4 v = make_uint4(0u, 0u, 0u, 0u);
+            if (j < J && kc * 8 < R) v = __ldg(chunk_addr(B, j, kc * 8));
+            *reinterpret_cast<uint4*>(Bs + (size_t)(kc >> 3) * jpad * 128 + j * 128 + (((kc & 7) ^ (j & 7)) << 4)) = v;
+        }
+    } else {
+        const int jc = jpad / 8;
+        for (int c = threadIdx.x; c < kslices * RW_K * jc; c += blockDim.x) {
+            const int r = c / jc, j0 = (c % jc) * 8;
+            uint4 v = make_uint4(0u, 0u, 0u, 0u);
+            if (r < R && j0 < J) v = __ldg(chunk_addr(B, r, j0));
+            const uint16_t* e = reinterpret_cast<const uint16_t*>(&v);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const int j = j0 + k;
+                *reinterpret_cast<uint16_t*>(Bs + (size_t)(r >> 6) * jpad * 128 + j * 128 +
+                                             ((((r >> 3) & 7) ^ (j & 7)) << 4) + (r & 7) * 2) = e[k];
+            }
+        }
+    }
+}
+
+__global__ void __launch_bounds__(RW_T, 1) k_gemm_rows(int I, int J, int R, Operand A, Operand B, sdem_sg_epilogue ep,
+                                                       int wide) {
+    extern __shared__ __align__(1024) uint8_t rw_smem[];
+    __shared__ __align__(8) uint64_t full[RW_STAGES], empty[RW_STAGES], accf[RW_ACC], acce[RW_ACC];
+    __shared__ uint32_t tmem_slot;
+    __shared__ float bias_s[RW_J_MAX];
+    const int jpad = (J + 15) / 16 * 16, kslices = (R + RW_K - 1) / RW_K, nb = (jpad + 127) / 128;
+    const int tiles = (I + RW_M - 1) / RW_M;
+    const bool by_segment = (A.nseg < 2 || A.c0[1] % RW_K == 0) && (A.nseg < 3 || A.c0[2] % RW_K == 0);
+    uint8_t* Bs = rw_smem;
+    const uint32_t Bs0 = smem_u32(Bs), As0 = Bs0 + (uint32_t)(kslices * jpad * 128);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&tmem_slot)),
+                     "r"(RW_ACC * 128)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+    }
+    if (threadIdx.x == 0) {
+        for (int k = 0; k < RW_STAGES; ++k) {
+            mbar_init(&full[k], 128);
+            mbar_init(&empty[k], 1);
+        }
+        for (int k = 0; k < RW_ACC; ++k) {
+            mbar_init(&accf[k], 1);
+            mbar_init(&acce[k], 128);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    for (int j = threadIdx.x; j < RW_J_MAX; j += RW_T) bias_s[j] = ep.bias && j < J ? ep.bias[j] : 0.f;
+    stage_b(Bs, B, J, jpad, R, kslices);
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    const uint32_t tmem = tmem_slot;
+    const int mine = tiles > (int)blockIdx.x ? (tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;   // this CTA's tiles
+    const int slices = mine * kslices;
+    if (warp >= 4 && warp < 8) {
+        // ---- copies: thread = (row mod 16, 16-byte chunk of the row's 128 bytes)
+        const int pt = threadIdx.x - 128, kc = pt & 7, r0 = pt >> 3;
+        bool ok = true;
+        int t = 0;   // slices issued
+        const uint32_t dst0 = As0 + r0 * 128 + ((kc ^ (r0 & 7)) << 4);
+        auto begin = [&]() -> uint32_t {   // the ring slot of slice t, free again
+            const int st = t % RW_STAGES, use = t / RW_STAGES;
+            if (use > 0 && ok) ok = mbar_wait(smem_u32(&empty[st]), (use - 1) & 1);
+            return dst0 + st * RW_SLICE;
+        };
+        auto finish = [&]() {
+            asm volatile("cp.async.commit_group;\n" ::: "memory");
+            if (t >= RW_LAG - 1) {   // the slice of RW_LAG - 1 rounds ago has landed: hand it to the tensor cores
+                asm volatile("cp.async.wait_group %0;\n" ::"n"(RW_LAG - 1) : "memory");
+                asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                if (t - (RW_LAG - 1) < slices) mbar_arrive(&full[(t - (RW_LAG - 1)) % RW_STAGES]);
+            }
+            ++t;
+        };
+        if (by_segment) {
+            // Whole slices lie in one segment: the rows' addresses are made once
+            // per segment, from indices that were requested a tile earlier (as a
+            // load beside each copy, their latency held every slice up: 342 us
+            // instead of 117 at 600k rows of 384).
+            int nxt[3][8];
+            auto fetch = [&](int m) {
+                const int i0 = ((int)blockIdx.x + m * (int)gridDim.x) * RW_M;
+#pragma unroll
+                for (int s = 0; s < 3; ++s)
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        const int gd = i0 + r0 + 16 * q;
+                        nxt[s][q] = -1;
+                        if (s < A.nseg && m < mine && gd < I) nxt[s][q] = A.idx[s] ? __ldg(A.idx[s] + gd) : gd;
+                    }
+            };
+            fetch(0);
+            for (int m = 0; m < mine; ++m) {
+                int cur[3][8];
+#pragma unroll
+                for (int s = 0; s < 3; ++s)
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) cur[s][q] = nxt[s][q];
+                fetch(m + 1);
+#pragma unroll
+                for (int s = 0; s < 3; ++s) {
+                    if (s >= A.nseg) break;
+                    const int w = (s + 1 < A.nseg ? A.c0[s + 1] : R) - A.c0[s];
+                    for (int c = 0; c < w; c += RW_K) {
+                        const uint32_t dst = begin();
+#pragma unroll
+                        for (int q = 0; q < 8; ++q) {
+                            const bool in = cur[s][q] >= 0 && c + kc * 8 < w;
+                            cp16(dst + q * 2048,
+                                 in ? A.ptr[s] + (size_t)cur[s][q] * A.ld[s] + c + kc * 8 : A.ptr[0], in ? 16u : 0u);
+                        }
+                        finish();
+                    }
+                }
+            }
+        } else {
+            while (t < slices) {
+                const int i0 = ((int)blockIdx.x + (t / kslices) * (int)gridDim.x) * RW_M;
+                const int gr = (t % kslices) * RW_K + kc * 8;
+                const uint32_t dst = begin();
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    const int gd = i0 + r0 + 16 * q;
+                    const bool in = gd < I && gr < R;
+                    cp16(dst + q * 2048, in ? (const void*)chunk_addr(A, gd, gr) : (const void*)A.ptr[0], in ? 16u : 0u);
+                }
+                finish();
+            }
+        }
+        while (t < slices + RW_LAG - 1) finish();
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        if (!ok && pt == 0) atomicAdd(&g_tc_timeouts, 1u);
+    } else if (warp == 8) {
+        if (lane == 0) {
+            bool ok = true;
+            for (int m = 0; m < mine && ok; ++m)
+                for (int n = 0; n < nb && ok; ++n) {
+                    const int u = m * nb + n, buf = u % RW_ACC, use = u / RW_ACC;
+                    if (use > 0) ok = mbar_wait(smem_u32(&acce[buf]), (use - 1) & 1);
+                    const int cols = min(128, jpad - n * 128);
+                    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(cols >> 3) << 17) |
+                                           ((uint32_t)(RW_M >> 4) << 24);
+                    for (int ks = 0; ks < kslices && ok; ++ks) {
+                        const int t = m * kslices + ks, st = t % RW_STAGES;
+                        if (n == 0) ok = mbar_wait(smem_u32(&full[st]), (t / RW_STAGES) & 1);
+                        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                        const int steps = (min(RW_K, R - ks * RW_K) + 15) / 16;
+                        for (int k = 0; k < steps; ++k)
+                            tc_mma(tmem + buf * 128,
+                                   umma_desc_sw128(As0 + st * RW_SLICE + k * 32, 16, 1024),
+                                   umma_desc_sw128(Bs0 + ks * jpad * 128 + n * 16384 + k * 32, 16, 1024), idesc,
+                                   ks > 0 || k > 0);
+                        if (n == nb - 1) tc_commit(&empty[st]);
+                    }
+                    if (ok) tc_commit(&accf[buf]);
+                }
+            if (!ok) atomicAdd(&g_tc_timeouts, 1u);
+        }
+        __syncwarp();
+    } else {
+        // ---- epilogue: warp w holds rows 32 w.. of the tile
+        bool ok = true;
+        for (int m = 0; m < mine; ++m) {
+            const int gi = ((int)blockIdx.x + m * (int)gridDim.x) * RW_M + warp * 32 + lane;
+            for (int n = 0; n < nb; ++n) {
+                const int u = m * nb + n, buf = u % RW_ACC;
+                if (ok) ok = mbar_wait(smem_u32(&accf[buf]), (u / RW_ACC) & 1);
+                ok = __all_sync(0xffffffffu, ok);
+                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                const int cols = min(128, jpad - n * 128);
+                for (int c = 0; c < cols; c += 32) {
+                    uint32_t r[32];
+                    tc_ld32(tmem + ((uint32_t)(warp * 32) << 16) + buf * 128 + c, r);
+                    if (!ok) {
+#pragma unroll
+                        for (int q = 0; q < 32; ++q) r[q] = 0u;
+                    }
+                    if (gi < I) epilogue32(ep, wide != 0, bias_s, gi, n * 128 + c, J, r);
+                }
+                asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+                mbar_arrive(&acce[buf]);
+            }
+        }
+        if (!ok && threadIdx.x == 0) atomicAdd(&g_tc_timeouts, 1u);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(RW_ACC * 128) : "memory");
+}
+
+// ------------------------------------------------ tcgen05, both operands transposed
+// The weight gradients: C (I x J) = sum over rows r of A(r, i) B(r, j), rows of
+// B gathered, the reduction split over blocks.  One CTA per (128 x 128 tile of
+// C, split); slices of 64 rows of both operands go to shared memory as they lie
+// in global memory, M- and N-major with the 128-byte swizzle -- element (r, i)
+// at (i / 64) * 8192 + (r / 8) * 1024 + (r mod 8) * 128 + ((i / 8 mod 8) xor (r mod
+// 8)) * 16 bytes -- where k_gemm transposed them element by element.  A ring of
+// six slices, five in flight, gated by the mbarriers that tcgen05.commit
+// arrives on.  Split boundaries, order and steps of the reduction are k_gemm's,
+// and the results are the same bits.
+// L2 bound: 600k rows, 128 x 384, 50 splits: 229 us (4.9 TB/s of L2; k_gemm 1150
+// us, the transposing 2-byte stores to shared memory).
+constexpr int WG_T = 256, WG_K = 64, WG_STAGES = 6;
+constexpr int WG_TILE = WG_K * 128 * 2;                   // 16 KB of one operand
+constexpr int WG_SMEM = WG_STAGES * 2 * WG_TILE;
+
+// The copies of one operand by one CTA: 16 threads a row (256 bytes), four rows a
+// thread.  Where the tile's columns lie in one segment, the rows' indices are
+// requested one slice ahead of their copies.
+struct WgSource {
+    const uint16_t* p;
+    const int* ix;
+    int ld, nxt[4];
+    bool one, in;
+    __device__ __forceinline__ void init(const Operand& op, int d0, int ndim) {
+        const int gd = d0 + (threadIdx.x & 15) * 8, last = min(d0 + 128, ndim) - 1;
+        const int s0 = (op.nseg > 2 && d0 >= op.c0[2]) ? 2 : (op.nseg > 1 && d0 >= op.c0[1]) ? 1 : 0;
+        const int s1 = (op.nseg > 2 && last >= op.c0[2]) ? 2 : (op.nseg > 1 && last >= op.c0[1]) ? 1 : 0;
+        one = s0 == s1;
+        in = gd < ndim;
+        p = (s0 == 2 ? op.ptr[2] : s0 == 1 ? op.ptr[1] : op.ptr[0]);
+        ix = (s0 == 2 ? op.idx[2] : s0 == 1 ? op.idx[1] : op.idx[0]);
+        ld = (s0 == 2 ? op.ld[2] : s0 == 1 ? op.ld[1] : op.ld[0]);
+        const int c0 = (s0 == 2 ? op.c0[2] : s0 == 1 ? op.c0[1] : 0);
+        if (in) p += gd - c0;
+    }
+    __device__ __forceinline__ void fetch(int r0, int rend) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int gr = r0 + (int)(threadIdx.x >> 4) + 16 * q;
+            nxt[q] = -1;
+            if (in && gr < rend) nxt[q] = ix ? __ldg(ix + gr) : gr;
+        }
+    }
+    __device__ __forceinline__ void copy(uint32_t S, const Operand& op, int d0, int r0, int rend) {
+        const int mc = threadIdx.x & 15, rr = threadIdx.x >> 4;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int r = rr + 16 * q;
+            const uint32_t dst = S + (mc >> 3) * 8192 + (r >> 3) * 1024 + (r & 7) * 128 + (((mc & 7) ^ (r & 7)) << 4);
+            const bool ok = nxt[q] >= 0;
+            const void* src = !ok ? (const void*)op.ptr[0]
+                              : one ? (const void*)(p + (size_t)nxt[q] * ld)
+                                    : (const void*)chunk_addr(op, r0 + r, d0 + mc * 8);
+            cp16(dst, src, ok ? 16u : 0u);
+        }
+        fetch(r0 + WG_K, rend);
+    }
+};
+
+__global__ void __launch_bounds__(WG_T, 1) k_gemm_wgrad(int I, int J, int R, Operand A, Operand B, float* __restrict__ out,
+                                                        int ld_out, int accumulate, int rchunk,
+                                                        float* __restrict__ partial) {
+    extern __shared__ __align__(1024) uint8_t wg_smem[];
+    __shared__ __align__(8) uint64_t done[WG_STAGES];
+    __shared__ uint32_t tmem_slot;
+    const uint32_t As0 = smem_u32(wg_smem), Bs0 = As0 + WG_STAGES * WG_TILE;
+    const int i0 = blockIdx.x * 128, j0 = blockIdx.y * 128;
+    const int rb = blockIdx.z * rchunk, re = min(R, rb + rchunk);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int cols = min(128, (J - j0 + 15) / 16 * 16);
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&tmem_slot)),
+                     "r"(128)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+    }
+    if (threadIdx.x == 0) {
+        for (int k = 0; k < WG_STAGES; ++k) mbar_init(&done[k], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    const uint32_t tmem = tmem_slot;
+    const int nch = re > rb ? (re - rb + WG_K - 1) / WG_K : 0;
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) |   // both operands MN-major
+                           ((uint32_t)(cols >> 3) << 17) | (8u << 24);
+    bool ok = true;
+    WgSource sa, sb;
+    sa.init(A, i0, I);
+    sb.init(B, j0, J);
+    sa.fetch(rb, re);
+    sb.fetch(rb, re);
+#pragma unroll
+    for (int k = 0; k < WG_STAGES - 1; ++k) {
+        if (k < nch) {
+            sa.copy(As0 + k * WG_TILE, A, i0, rb + k * WG_K, re);
+            sb.copy(Bs0 + k * WG_TILE, B, j0, rb + k * WG_K, re);
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    }
+    for (int c = 0; c < nch; ++c) {
+        const int b = c % WG_STAGES;
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(WG_STAGES - 2) : "memory");
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+            const int steps = (min(WG_K, re - rb - c * WG_K) + 15) / 16;
+            for (int k = 0; k < steps; ++k)
+                tc_mma(tmem, umma_desc_sw128(As0 + b * WG_TILE + k * 2048, 8192, 1024),
+                       umma_desc_sw128(Bs0 + b * WG_TILE + k * 2048, 8192, 1024), idesc, c > 0 || k > 0);
+            tc_commit(&done[b]);
+        }
+        // slice c + STAGES - 1 goes where slice c - 1 was: wait for its MMAs
+        const int nx = c + WG_STAGES - 1;
+        if (nx < nch) {
+            const int bx = nx % WG_STAGES;
+            if (c >= 1 && ok) ok = mbar_wait(smem_u32(&done[bx]), ((c - 1) / WG_STAGES) & 1);
+            sa.copy(As0 + bx * WG_TILE, A, i0, rb + nx * WG_K, re);
+            sb.copy(Bs0 + bx * WG_TILE, B, j0, rb + nx * WG_K, re);
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    }
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    if (nch > 0 && ok) ok = mbar_wait(smem_u32(&done[(nch - 1) % WG_STAGES]), ((nch - 1) / WG_STAGES) & 1);
+    if (!ok && lane == 0) atomicAdd(&g_tc_timeouts, 1u);
+    ok = __all_sync(0xffffffffu, ok);
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    const int gi = i0 + (warp & 3) * 32 + lane;   // warps w and w + 4 hold the same rows, alternate column groups
+    for (int c = (warp >> 2) * 32; c < cols; c += 64) {
+        uint32_t r[32];
+        tc_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + c, r);
+        if (gi >= I) continue;
+#pragma unroll
+        for (int q = 0; q < 32; ++q) {
+            const int gj = j0 + c + q;
+            if (gj >= J) continue;
+            const float v = nch > 0 && ok ? __uint_as_float(r[q]) : 0.f;
+            if (partial) {
+                partial[((size_t)blockIdx.z * I + gi) * J + gj] = v;
+            } else {
+                float* o = out + (size_t)gi * ld_out + gj;
+                *o = accumulate ? *o + v : v;
+            }
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(128) : "memory");
+}
+
 __global__ void k_split_reduce(int I, int J, int splits, const float* __restrict__ partial, float* __restrict__ out,
                                int ld_out, int accumulate) {
     const size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const size_t IJ = (size_t)I * J;
     if (k >= IJ) return;
     float s = 0.f;
+#pragma unroll 16
     for (int z = 0; z < splits; ++z) s += partial[z * IJ + k];
     const int i = (int)(k / J), j = (int)(k % J);
     float* o = out + (size_t)i * ld_out + j;
@@ -625,6 +1148,21 @@ inline int launched() { return cudaGetLastError() == cudaSuccess ? SDEM_SG_OK : 
 
 inline unsigned blocks(long long n, int t) { return (unsigned)((n + t - 1) / t); }
 
+inline bool aligned32(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 31u) == 0; }
+
+// The opt-in of a kernel to large dynamic shared memory, per device (idempotent,
+// a host-side attribute: cheap enough to set at every call).
+inline bool set_smem(const void* f, int bytes) {
+    return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
+}
+
+inline int sm_count() {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return 1;
+    return n;
+}
+
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 // Checks an operand against the dimension its columns cover (total width)
@@ -717,16 +1255,41 @@ int sdem_sg_gemm(int I, int J, int R, const sdem_sg_operand* a, const sdem_sg_op
     const int nsplit = R > 0 ? (int)((R + rchunk - 1) / rchunk) : 1;
     const dim3 grid(blocks(I, BM), blocks(J, BN), nsplit);
     if (grid.y > 65535 || grid.z > 65535) return SDEM_SG_E_ARG;
+    const int jpad = (J + 15) / 16 * 16, kslices = (R + RW_K - 1) / RW_K;
+    const size_t bbytes = (size_t)kslices * jpad * 128;
+    if (nsplit == 1 && g_tc_enabled && !A.trans && R > 0 && jpad <= RW_J_MAX && bbytes <= RW_B_MAX &&
+        (jpad <= 128 || kslices <= RW_STAGES / 2)) {
+        // B fits in shared memory (with more than one block of columns a tile's
+        // slices stay until the last block, so that two tiles must fit the ring)
+        const size_t smem = bbytes + RW_STAGES * RW_SLICE;
+        if (!set_smem((const void*)k_gemm_rows, RW_B_MAX + RW_STAGES * RW_SLICE)) return SDEM_SG_E_CUDA;
+        const bool wide = J % 32 == 0 && (!ep->out || (aligned32(ep->out) && ep->ld_out % 8 == 0)) &&
+                          (!ep->out_bf || (aligned32(ep->out_bf) && ep->ld_out_bf % 16 == 0)) &&
+                          (!ep->mask || (aligned32(ep->mask) && ep->ld_mask % 16 == 0)) &&
+                          (!ep->resid || (aligned32(ep->resid) && ep->ld_resid % 8 == 0)) &&
+                          (!ep->res_out || (aligned32(ep->res_out) && ep->ld_res_out % 8 == 0)) &&
+                          (!ep->res_out_bf || (aligned32(ep->res_out_bf) && ep->ld_res_out_bf % 16 == 0));
+        const int tiles = (I + RW_M - 1) / RW_M;
+        k_gemm_rows<<<std::min(tiles, sm_count()), RW_T, smem, st(stream)>>>(I, J, R, A, B, *ep, wide ? 1 : 0);
+        return launched();
+    }
     if (nsplit == 1 && g_tc_enabled && !A.trans && !B.trans) {
-        static bool attr = false;
-        if (!attr) {
-            if (cudaFuncSetAttribute(k_gemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM) != cudaSuccess)
-                return SDEM_SG_E_CUDA;
-            attr = true;
-        }
+        if (!set_smem((const void*)k_gemm_tc, TC_SMEM)) return SDEM_SG_E_CUDA;
         const dim3 tgrid(blocks(I, TC_M), blocks(J, TC_N));
         if (tgrid.y > 65535) return SDEM_SG_E_ARG;
         k_gemm_tc<<<tgrid, TC_T, TC_SMEM, st(stream)>>>(I, J, R, A, B, *ep);
+        return launched();
+    }
+    const bool only_out = ep->out && !ep->bias && !ep->relu && !ep->mask && !ep->out_bf && !ep->resid;
+    if (g_tc_enabled && A.trans && B.trans && R > 0 && only_out && (nsplit == 1 || partial)) {
+        if (!set_smem((const void*)k_gemm_wgrad, WG_SMEM)) return SDEM_SG_E_CUDA;
+        const dim3 wgrid(blocks(I, 128), blocks(J, 128), nsplit);
+        k_gemm_wgrad<<<wgrid, WG_T, WG_SMEM, st(stream)>>>(I, J, R, A, B, ep->out, ep->ld_out, ep->accumulate, (int)rchunk,
+                                                           nsplit > 1 ? partial : nullptr);
+        if (nsplit == 1) return launched();
+        if (cudaGetLastError() != cudaSuccess) return SDEM_SG_E_CUDA;
+        k_split_reduce<<<blocks((long long)I * J, 256), 256, 0, st(stream)>>>(I, J, nsplit, partial, ep->out, ep->ld_out,
+                                                                           ep->accumulate);
         return launched();
     }
     if (nsplit == 1) {
