@@ -115,6 +115,21 @@ typedef struct sdem_sg_epilogue {
 int sdem_sg_gemm(int I, int J, int R, const sdem_sg_operand* a, const sdem_sg_operand* b,
                  const sdem_sg_epilogue* ep, int splits, float* partial, void* stream);
 
+/* One two-layer MLP of the network in one kernel (hidden width 128):
+ *   z = bf16(relu(A w1^T + b1)),  v = z w2^T + b2,  w = resid ? resid + v : v.
+ * A (M x R, R a multiple of 8 up to 384, not transposed, segment widths but the
+ * last multiples of 64), w1 (128 x R) and w2 (J x 128, J = 128 or 16) as in
+ * sdem_sg_gemm.  z (M x 128), out = w (M x J floats) and out_bf = bf16(w) are
+ * written where given; resid (M x 128) may be out itself.  With agg_bf
+ * (nagg x 128): agg_bf[i] = bf16 of the sum, in row order, of v over the rows
+ * row_off[i] .. row_off[i+1]; dst[row] = i for those rows, row_off[nagg] = M;
+ * receivers without rows are left as they are.  Pointers of z, resid, out and
+ * out_bf are 32-byte aligned.  The results are the bits of the separate
+ * sdem_sg_gemm and sdem_sg_segsum calls. */
+int sdem_sg_mlp(int M, int R, const sdem_sg_operand* a, const uint16_t* w1, const float* b1, const uint16_t* w2,
+                const float* b2, int J, uint16_t* z, const float* resid, float* out, uint16_t* out_bf, int nagg,
+                const int* row_off, const int* dst, uint16_t* agg_bf, void* stream);
+
 /* Which tensor-core kernel sdem_sg_gemm uses for the forms without
  * transposed operands or split reductions: 1 (default) the tcgen05/TMEM
  * kernel, 0 the warp-level mma.sync kernel (kept for the other forms). */

@@ -6,6 +6,8 @@
 //                                   order (neighbour cell, then sphere index);
 //   k_node_feat                     node features (velocity frames, spin,
 //                                   size, plane distances) as bf16;
+//   k_mlp                           both layers of one MLP of the forward pass, with
+//                                   residual and message sums, on tcgen05;
 //   k_gemm_rows, k_gemm_wgrad       the network's layers on tcgen05, forward and
 //                                   backward: C = A . B^T over operands that may be
 //                                   row-gathered, split in column segments
@@ -835,6 +837,7 @@ __global__ void __launch_bounds__(RW_T, 1) k_gemm_rows(int I, int J, int R, Oper
                         for (int q = 0; q < 32; ++q) r[q] = 0u;
                     }
                     if (gi < I) epilogue32(ep, wide != 0, bias_s, gi, n * 128 + c, J, r);
+                    __syncwarp();   // tcgen05.ld takes whole warps
                 }
                 asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
                 mbar_arrive(&acce[buf]);
@@ -983,11 +986,10 @@ __global__ void __launch_bounds__(WG_T, 1) k_gemm_wgrad(int I, int J, int R, Ope
     for (int c = (warp >> 2) * 32; c < cols; c += 64) {
         uint32_t r[32];
         tc_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + c, r);
-        if (gi >= I) continue;
 #pragma unroll
         for (int q = 0; q < 32; ++q) {
             const int gj = j0 + c + q;
-            if (gj >= J) continue;
+            if (gi >= I || gj >= J) continue;
             const float v = nch > 0 && ok ? __uint_as_float(r[q]) : 0.f;
             if (partial) {
                 partial[((size_t)blockIdx.z * I + gi) * J + gj] = v;
@@ -996,11 +998,419 @@ __global__ void __launch_bounds__(WG_T, 1) k_gemm_wgrad(int I, int J, int R, Ope
                 *o = accumulate ? *o + v : v;
             }
         }
+        __syncwarp();   // tcgen05.ld takes whole warps
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(128) : "memory");
+}
+
+// ------------------------------------------------------- two layers in one kernel
+// One MLP of the network: z = relu(A W1^T + b1) (128 wide), v = z W2^T + b2, with
+// an optional residual and an optional sum of v over the rows of each receiver
+// (the messages of an edge block).  Both weights stay in shared memory; z goes
+// from tensor memory through registers into shared memory as the second
+// product's operand, and v from registers to its place, so that of the
+// intermediate values only what the caller asks for reaches HBM.  As separate
+// kernels an edge block moved 3 KB of HBM an edge (z twice, the messages twice,
+// the residual stream in two precisions); here it moves 1.5 KB.
+//
+// A CTA owns a contiguous range of rows, cut at receivers when there are sums,
+// and walks it in tiles of 128 rows.  Warps 12-15 copy A (ring of slices as in
+// k_gemm_rows), one thread of warp 16 issues the products -- the first layer of
+// tile m+1 before the second of tile m -- warps 4-7 make z in two halves of 64
+// columns, each handed over and given back by itself, warps 0-3 finish v, and
+// warps 8-11 read v from tensor memory once more and sum it.  The sums run
+// over the rows of a receiver one after another in row order (as k_segsum's),
+// from a 16-column strip in shared memory; the receiver that a tile leaves open
+// carries its sums to the next tile.  All results are the bits of the
+// separate kernels.
+// 974k edges of 50k receivers: 473 us for an edge block (511 with z), 250 us for
+// the products and a bf16 result alone, 264 with the sums alone: the roles share
+// the SM and none has slack enough to hide the others (HBM would take 230 us).
+// The forward pass of 50k spheres went from 5.84 ms of separate kernels to 3.27.
+constexpr int ML_T = 544, ML_LAG = 3, ML_MAX_STAGES = 6, ML_STRIP = 16;
+constexpr int ML_STRIP_LD = ML_STRIP + 1, ML_STRIP_BYTES = 128 * ML_STRIP_LD * 4;
+constexpr int ML_SMEM_MAX = 232448 - 3072;   // dynamic part beside the static arrays (below 3 KB)
+
+struct MlpArgs {
+    int M, R, J;
+    const uint16_t *w1, *w2;
+    const float *b1, *b2;
+    uint16_t* z;
+    const float* resid;
+    float* out;
+    uint16_t* out_bf;
+    int nagg;
+    const int *row_off, *dst;
+    uint16_t* agg;
+    int stages;
+};
+
+// first r in [0, n] with off[r] >= target (off ascending, off[n] >= target); one warp
+__device__ __forceinline__ int lower_bound32(const int* __restrict__ off, int n, int target) {
+    const int lane = threadIdx.x & 31;
+    int lo = 0, hi = n;
+    while (hi > lo) {
+        const int step = (hi - lo + 31) / 32, p = lo + lane * step;
+        const int c = __popc(__ballot_sync(0xffffffffu, p < hi && __ldg(off + p) < target));
+        if (c == 0) break;
+        hi = min(hi, lo + c * step);
+        lo = lo + (c - 1) * step + 1;
+    }
+    return lo;
+}
+
+__device__ __forceinline__ void bar_sums() { asm volatile("bar.sync 1, 128;\n" ::: "memory"); }
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p)); }
+
+__global__ void __launch_bounds__(ML_T, 1) k_mlp(Operand A, MlpArgs g) {
+    extern __shared__ __align__(1024) uint8_t ml_smem[];
+    __shared__ __align__(8) uint64_t full[ML_MAX_STAGES], empty[ML_MAX_STAGES], a1f[2], a1e[2], a2f[2], a2e[2], zf[2], ze[2];
+    __shared__ uint32_t tmem_slot;
+    __shared__ __align__(16) float b1s[128], b2s[128], carry[2][128];   // carry: sums of the open receiver, by tile parity
+    __shared__ int range[2], s_dst[128], s_after;
+    __shared__ uint8_t s_seg[132];   // rows where receivers start in the tile
+    __shared__ unsigned s_head[4];
+    const int kslices = (g.R + RW_K - 1) / RW_K, jpad = (g.J + 15) / 16 * 16;
+    const uint32_t W1 = smem_u32(ml_smem), W2 = W1 + kslices * 16384, Z = W2 + 2 * jpad * 128, ring = Z + 32768;
+    float* strip = reinterpret_cast<float*>(ml_smem + kslices * 16384 + 2 * jpad * 128 + 32768 + g.stages * RW_SLICE);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&tmem_slot)),
+                     "r"(512)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+    }
+    if (threadIdx.x == 0) {
+        for (int k = 0; k < ML_MAX_STAGES; ++k) {
+            mbar_init(&full[k], 128);
+            mbar_init(&empty[k], 1);
+        }
+        for (int k = 0; k < 2; ++k) {
+            mbar_init(&a1f[k], 1);
+            mbar_init(&a1e[k], 128);
+            mbar_init(&a2f[k], 1);
+            mbar_init(&a2e[k], g.agg ? 256 : 128);
+            mbar_init(&zf[k], 128);
+            mbar_init(&ze[k], 1);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    if (warp == 1 || warp == 2) {   // this CTA's rows
+        const int b = (int)blockIdx.x + (warp - 1), G = (int)gridDim.x;
+        int at;
+        if (g.agg) {
+            const int target = (int)((long long)g.M * b / G);
+            at = b == G ? g.M : g.row_off[lower_bound32(g.row_off, g.nagg, target)];
+        } else {
+            const long long tiles = (g.M + 127) / 128;
+            at = (int)min((long long)g.M, tiles * b / G * 128);
+        }
+        if (lane == 0) range[warp - 1] = at;
+    }
+    if (threadIdx.x < 128) {
+        b1s[threadIdx.x] = g.b1[threadIdx.x];
+        b2s[threadIdx.x] = (int)threadIdx.x < g.J ? g.b2[threadIdx.x] : 0.f;
+    }
+    {
+        Operand w;
+        w.ptr[0] = g.w1; w.ptr[1] = w.ptr[2] = nullptr;
+        w.idx[0] = w.idx[1] = w.idx[2] = nullptr;
+        w.ld[0] = g.R; w.ld[1] = w.ld[2] = 0;
+        w.c0[0] = 0; w.c0[1] = w.c0[2] = 1 << 30;
+        w.nseg = 1;
+        w.trans = 0;
+        stage_b(ml_smem, w, 128, 128, g.R, kslices);
+        w.ptr[0] = g.w2;
+        w.ld[0] = 128;
+        stage_b(ml_smem + kslices * 16384, w, g.J, jpad, 128, 2);
+    }
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    const uint32_t tmem = tmem_slot;
+    const int lo = range[0], hi = range[1];
+    const int mine = (hi - lo + 127) / 128, slices = mine * kslices;
+    bool ok = true;
+    if (warp >= 12 && warp < 16) {
+        // ---- copies of A
+        const int pt = threadIdx.x - 384, kc = pt & 7, r0 = pt >> 3, S = g.stages;
+        int t = 0, slot = 0, round = 0;
+        const uint32_t dst0 = ring + r0 * 128 + ((kc ^ (r0 & 7)) << 4);
+        int hand = 0;   // ring slot handed over next
+        auto finish = [&]() {
+            asm volatile("cp.async.commit_group;\n" ::: "memory");
+            if (t >= ML_LAG - 1) {
+                asm volatile("cp.async.wait_group %0;\n" ::"n"(ML_LAG - 1) : "memory");
+                asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                if (t - (ML_LAG - 1) < slices) mbar_arrive(&full[hand]);
+                hand = hand + 1 == S ? 0 : hand + 1;
+            }
+            ++t;
+            if (++slot == S) {
+                slot = 0;
+                ++round;
+            }
+        };
+        int nxt[3][8];
+        auto fetch = [&](int m) {
+#pragma unroll
+            for (int s = 0; s < 3; ++s)
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    const int gd = lo + m * 128 + r0 + 16 * q;
+                    nxt[s][q] = -1;
+                    if (s < A.nseg && gd < hi) nxt[s][q] = A.idx[s] ? __ldg(A.idx[s] + gd) : gd;
+                }
+        };
+        fetch(0);
+        for (int m = 0; m < mine; ++m) {
+            int cur[3][8];
+#pragma unroll
+            for (int s = 0; s < 3; ++s)
+#pragma unroll
+                for (int q = 0; q < 8; ++q) cur[s][q] = nxt[s][q];
+            fetch(m + 1);
+#pragma unroll
+            for (int s = 0; s < 3; ++s) {
+                if (s >= A.nseg) break;
+                const int w = (s + 1 < A.nseg ? A.c0[s + 1] : g.R) - A.c0[s];
+                for (int c = 0; c < w; c += RW_K) {
+                    if (round > 0 && ok) ok = mbar_wait(smem_u32(&empty[slot]), (round - 1) & 1);
+                    const uint32_t dst = dst0 + slot * RW_SLICE;
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        const bool in = cur[s][q] >= 0 && c + kc * 8 < w;
+                        cp16(dst + q * 2048, in ? A.ptr[s] + (size_t)cur[s][q] * A.ld[s] + c + kc * 8 : A.ptr[0],
+                             in ? 16u : 0u);
+                    }
+                    finish();
+                }
+            }
+        }
+        while (t < slices + ML_LAG - 1) finish();
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    } else if (warp == 16) {
+        if (lane == 0) {
+            const uint32_t id1 = (1u << 4) | (1u << 7) | (1u << 10) | (16u << 17) | (8u << 24);
+            const uint32_t id2 = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(jpad >> 3) << 17) | (8u << 24);
+            int slot = 0, round = 0;
+            auto first = [&](int m) {
+                const int b = m & 1;
+                if (m >= 2 && ok) ok = mbar_wait(smem_u32(&a1e[b]), ((m >> 1) - 1) & 1);
+                for (int ks = 0; ks < kslices && ok; ++ks) {
+                    ok = mbar_wait(smem_u32(&full[slot]), round & 1);
+                    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                    const int steps = (min(RW_K, g.R - ks * RW_K) + 15) / 16;
+                    for (int k = 0; k < steps; ++k)
+                        tc_mma(tmem + b * 128, umma_desc_sw128(ring + slot * RW_SLICE + k * 32, 16, 1024),
+                               umma_desc_sw128(W1 + ks * 16384 + k * 32, 16, 1024), id1, ks > 0 || k > 0);
+                    tc_commit(&empty[slot]);
+                    if (++slot == g.stages) {
+                        slot = 0;
+                        ++round;
+                    }
+                }
+                if (ok) tc_commit(&a1f[b]);
+            };
+            if (mine > 0) first(0);
+            for (int m = 0; m < mine && ok; ++m) {
+                if (m + 1 < mine) first(m + 1);
+                const int b = m & 1;
+                if (m >= 2 && ok) ok = mbar_wait(smem_u32(&a2e[b]), ((m >> 1) - 1) & 1);
+                for (int half = 0; half < 2 && ok; ++half) {
+                    ok = mbar_wait(smem_u32(&zf[half]), m & 1);
+                    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                    for (int k = 0; k < 4; ++k)
+                        tc_mma(tmem + 256 + b * 128, umma_desc_sw128(Z + half * 16384 + k * 32, 16, 1024),
+                               umma_desc_sw128(W2 + half * jpad * 128 + k * 32, 16, 1024), id2, half > 0 || k > 0);
+                    tc_commit(&ze[half]);
+                }
+                if (ok) tc_commit(&a2f[b]);
+            }
+        }
+        __syncwarp();
+    } else if (warp >= 8) {
+        // ---- sums: warp w holds rows 32 (w mod 4).. of the tile
+        const int w4 = warp & 3, row = w4 * 32 + lane;
+        // receivers of this tile and the next, requested two tiles ahead
+        int d0 = lo + row < hi && g.agg ? __ldg(g.dst + lo + row) : -1;
+        int d1 = lo + 128 + row < hi && g.agg ? __ldg(g.dst + lo + 128 + row) : -1;
+        for (int m = 0; g.agg && m < mine; ++m) {
+            const int b = m & 1, e0 = lo + m * 128, gi = e0 + row, rows = min(128, hi - e0);
+            const int before = s_dst[127];   // the tile before's last receiver
+            const int mydst = d0;
+            d0 = d1;
+            bar_sums();
+            s_dst[row] = mydst;
+            if (row == 0) s_after = d0;
+            d1 = gi + 256 < hi ? __ldg(g.dst + gi + 256) : -1;
+            int prev = __shfl_up_sync(0xffffffffu, mydst, 1);
+            bar_sums();
+            if (lane == 0 && row > 0) prev = s_dst[row - 1];
+            const bool head = gi < hi && (row == 0 || mydst != prev);
+            const unsigned hb = __ballot_sync(0xffffffffu, head);
+            if (lane == 0) s_head[w4] = hb;
+            bar_sums();
+            int rank = __popc(hb & ((1u << lane) - 1u)), nseg = 0;
+            for (int w = 0; w < 4; ++w) {
+                if (w < w4) rank += __popc(s_head[w]);
+                nseg += __popc(s_head[w]);
+            }
+            if (head) s_seg[rank] = (uint8_t)row;
+            if (row == 0) s_seg[nseg] = (uint8_t)rows;   // (the barrier before the first strip is read orders s_seg)
+            // the first receiver goes on from the tile before, the last into the next
+            const bool open_first = m > 0 && s_dst[0] == before;
+            const bool open_last = rows == 128 && e0 + 128 < hi && s_after == s_dst[127];
+            if (ok) ok = mbar_wait(smem_u32(&a2f[b]), (m >> 1) & 1);
+            ok = __all_sync(0xffffffffu, ok);
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+#pragma unroll 1
+            for (int c = 0; c < 128; c += 32) {
+                uint32_t r[32];
+                tc_ld32(tmem + 256 + ((uint32_t)(w4 * 32) << 16) + b * 128 + c, r);
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    float bias[ML_STRIP];
+#pragma unroll
+                    for (int q = 0; q < ML_STRIP / 4; ++q)
+                        reinterpret_cast<float4*>(bias)[q] = *reinterpret_cast<const float4*>(&b2s[c + half * ML_STRIP + 4 * q]);
+#pragma unroll
+                    for (int q = 0; q < ML_STRIP; ++q)
+                        strip[row * ML_STRIP_LD + q] = ok ? __uint_as_float(r[half * ML_STRIP + q]) + bias[q] : 0.f;
+                    bar_sums();
+                    // half a warp per receiver, a lane per column
+                    const int col = lane & 15, j = c + half * ML_STRIP + col;
+                    for (int k = w4 * 2 + (lane >> 4); k < nseg; k += 8) {
+                        const int r0 = s_seg[k];
+                        int left = s_seg[k + 1] - r0;
+                        const float* x = strip + r0 * ML_STRIP_LD + col;
+                        float sum = k == 0 && open_first ? carry[b][j] : 0.f;
+                        for (; left >= 8; left -= 8, x += 8 * ML_STRIP_LD) {
+                            float v[8];
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) v[i] = x[i * ML_STRIP_LD];
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) sum += v[i];
+                        }
+                        if (left > 0) {   // past the end +0, which leaves the sum (never -0) as it is
+                            float v[7];
+#pragma unroll
+                            for (int i = 0; i < 7; ++i) v[i] = i < left ? x[i * ML_STRIP_LD] : 0.f;
+#pragma unroll
+                            for (int i = 0; i < 7; ++i) sum += v[i];
+                        }
+                        if (k == nseg - 1 && open_last) carry[b ^ 1][j] = sum;
+                        else g.agg[(size_t)s_dst[r0] * 128 + j] = bf16_bits(sum);
+                    }
+                    __syncwarp();   // tcgen05.ld and the barrier take whole warps
+                    bar_sums();
+                }
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+            mbar_arrive(&a2e[b]);
+        }
+    } else if (warp >= 4) {
+        // ---- z: warp w holds rows 32 (w mod 4).. of the tile
+        const int row = (warp & 3) * 32 + lane;
+        uint8_t* zs = ml_smem + kslices * 16384 + 2 * jpad * 128 + row * 128;
+        for (int m = 0; m < mine; ++m) {
+            const int b = m & 1, gi = lo + m * 128 + row;
+            if (ok) ok = mbar_wait(smem_u32(&a1f[b]), (m >> 1) & 1);
+            ok = __all_sync(0xffffffffu, ok);
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                if (m >= 1 && ok) ok = mbar_wait(smem_u32(&ze[half]), (m - 1) & 1);
+                ok = __all_sync(0xffffffffu, ok);
+#pragma unroll
+                for (int c = half * 64; c < half * 64 + 64; c += 32) {
+                    uint32_t r[32], h[16];
+                    tc_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + b * 128 + c, r);
+#pragma unroll
+                    for (int q = 0; q < 16; ++q)
+                        h[q] = bf16_pair(fmaxf(__uint_as_float(r[2 * q]) + b1s[c + 2 * q], 0.f),
+                                         fmaxf(__uint_as_float(r[2 * q + 1]) + b1s[c + 2 * q + 1], 0.f));
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const int kc = ((c >> 3) + q) & 7;
+                        *reinterpret_cast<uint4*>(zs + half * 16384 + ((kc ^ (row & 7)) << 4)) =
+                            make_uint4(h[4 * q], h[4 * q + 1], h[4 * q + 2], h[4 * q + 3]);
+                    }
+                    if (g.z && gi < hi) {
+                        st8(g.z + (size_t)gi * 128 + c, h);
+                        st8(g.z + (size_t)gi * 128 + c + 16, h + 8);
+                    }
+                    __syncwarp();
+                }
+                asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+                if (half == 1) mbar_arrive(&a1e[b]);
+                mbar_arrive(&zf[half]);
+            }
+        }
+    } else {
+        // ---- v: warp w holds rows 32 w.. of the tile
+        const int row = warp * 32 + lane, J = g.J;
+        float res[32];   // the residual of the columns to come
+        auto load_res = [&](int gi, int c) {
+            if (g.resid && gi < hi) {
+#pragma unroll
+                for (int h = 0; h < 4; ++h) ld8(g.resid + (size_t)gi * 128 + c + 8 * h, reinterpret_cast<uint32_t*>(res) + 8 * h);
+            }
+        };
+        load_res(lo + row, 0);
+        for (int m = 0; m < mine; ++m) {
+            const int b = m & 1, gi = lo + m * 128 + row;
+            if (g.resid && gi + 128 < hi) {
+#pragma unroll
+                for (int h = 0; h < 4; ++h) prefetch_l2(g.resid + (size_t)(gi + 128) * 128 + 32 * h);
+            }
+            if (ok) ok = mbar_wait(smem_u32(&a2f[b]), (m >> 1) & 1);
+            ok = __all_sync(0xffffffffu, ok);
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+            if (g.out || g.out_bf) {
+#pragma unroll 1
+                for (int c = 0; c < J; c += 32) {
+                    uint32_t r[32];
+                    tc_ld32(tmem + 256 + ((uint32_t)(warp * 32) << 16) + b * 128 + c, r);
+                    float w[32];
+#pragma unroll
+                    for (int q = 0; q < 32; ++q) {
+                        const float v = ok ? __uint_as_float(r[q]) + b2s[c + q] : 0.f;
+                        w[q] = g.resid ? res[q] + v : v;
+                    }
+                    if (c + 32 < J) load_res(gi, c + 32);
+                    else load_res(gi + 128, 0);
+                    if (gi < hi && g.out) {
+#pragma unroll
+                        for (int h = 0; h < 4; ++h)
+                            if (c + 8 * h < J) st8(g.out + (size_t)gi * J + c + 8 * h, reinterpret_cast<const uint32_t*>(w) + 8 * h);
+                    }
+                    if (gi < hi && g.out_bf) {
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            uint32_t p[8];
+#pragma unroll
+                            for (int q = 0; q < 8; ++q) p[q] = bf16_pair(w[16 * h + 2 * q], w[16 * h + 2 * q + 1]);
+                            if (c + 16 * h < J) st8(g.out_bf + (size_t)gi * J + c + 16 * h, p);
+                        }
+                    }
+                    __syncwarp();   // tcgen05.ld takes whole warps
+                }
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+            mbar_arrive(&a2e[b]);
+        }
+    }
+    if (!ok && lane == 0) atomicAdd(&g_tc_timeouts, 1u);
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(512) : "memory");
 }
 
 __global__ void k_split_reduce(int I, int J, int splits, const float* __restrict__ partial, float* __restrict__ out,
@@ -1301,6 +1711,43 @@ int sdem_sg_gemm(int I, int J, int R, const sdem_sg_operand* a, const sdem_sg_op
     if (cudaGetLastError() != cudaSuccess) return SDEM_SG_E_CUDA;
     k_split_reduce<<<blocks((long long)I * J, 256), 256, 0, st(stream)>>>(I, J, nsplit, partial, ep->out, ep->ld_out,
                                                                        ep->accumulate);
+    return launched();
+}
+
+int sdem_sg_mlp(int M, int R, const sdem_sg_operand* a, const uint16_t* w1, const float* b1, const uint16_t* w2,
+                const float* b2, int J, uint16_t* z, const float* resid, float* out, uint16_t* out_bf, int nagg,
+                const int* row_off, const int* dst, uint16_t* agg_bf, void* stream) {
+    if (M < 0 || R < 8 || R > 384 || R % 8 || (J != 16 && J != 128) || !w1 || !b1 || !w2 || !b2 || !aligned16(w1) ||
+        !aligned16(w2) || nagg < 0)
+        return SDEM_SG_E_ARG;
+    if (M == 0) return SDEM_SG_OK;
+    Operand A;
+    if (!make_operand(a, R, &A) || A.trans) return SDEM_SG_E_ARG;
+    if ((A.nseg > 1 && A.c0[1] % RW_K) || (A.nseg > 2 && A.c0[2] % RW_K)) return SDEM_SG_E_ARG;
+    if ((z && !aligned32(z)) || (resid && (!aligned32(resid) || J != 128)) || (out && !aligned32(out)) ||
+        (out_bf && !aligned32(out_bf)) || (!out && !out_bf && !agg_bf))
+        return SDEM_SG_E_ARG;
+    if (agg_bf && (J != 128 || !row_off || !dst || nagg < 1)) return SDEM_SG_E_ARG;
+    MlpArgs g;
+    g.M = M;
+    g.R = R;
+    g.J = J;
+    g.w1 = w1;
+    g.b1 = b1;
+    g.w2 = w2;
+    g.b2 = b2;
+    g.z = z;
+    g.resid = resid;
+    g.out = out;
+    g.out_bf = out_bf;
+    g.nagg = nagg;
+    g.row_off = row_off;
+    g.dst = dst;
+    g.agg = agg_bf;
+    const int fixed = (R + RW_K - 1) / RW_K * 16384 + 2 * J * 128 + 32768 + (agg_bf ? ML_STRIP_BYTES : 0);
+    g.stages = std::min((int)ML_MAX_STAGES, (ML_SMEM_MAX - fixed) / RW_SLICE);   // 3 at R = 384
+    if (!set_smem((const void*)k_mlp, ML_SMEM_MAX)) return SDEM_SG_E_CUDA;
+    k_mlp<<<std::min((M + 127) / 128, sm_count()), ML_T, fixed + g.stages * RW_SLICE, st(stream)>>>(A, g);
     return launched();
 }
 

@@ -55,7 +55,7 @@ OVERLAP_GAIN = 100.0
 EXPORTED = ("sdem_sg_cells", "sdem_sg_edge_count", "sdem_sg_edge_fill", "sdem_sg_node_features", "sdem_sg_gemm",
             "sdem_sg_segsum", "sdem_sg_gather_add", "sdem_sg_colsum_blocks", "sdem_sg_colsum", "sdem_sg_mse",
             "sdem_sg_adam", "sdem_sg_to_bf16", "sdem_sg_advance", "sdem_sg_set_tensor_path",
-            "sdem_sg_tensor_timeouts")
+            "sdem_sg_tensor_timeouts", "sdem_sg_mlp")
 
 
 class SgGrid(C.Structure):
@@ -110,6 +110,7 @@ def load(path: str = LIB_PATH):
         "sdem_sg_advance": [I, P, I, D, D, D, D, D, C.POINTER(SgBox), P, P, P, P],
         "sdem_sg_set_tensor_path": [I],
         "sdem_sg_tensor_timeouts": [C.POINTER(C.c_uint)],
+        "sdem_sg_mlp": [I, I, C.POINTER(SgOperand), P, P, P, P, I, P, P, P, P, I, P, P, P, P],
     }
     for name, args in sig.items():
         fn = getattr(lib, name)
@@ -360,6 +361,9 @@ class Network:
         self.v = torch.zeros_like(self.p)
         self.step_count = 0
         self.device = device
+        # the library's two-layer kernel has the network's own width; other
+        # widths (and host memory, in the tests) take one call per layer
+        self.fused = latent == LATENT and torch.device(device).type == "cuda"
         self.colsum_partial = torch.empty(self.lib.sdem_sg_colsum_blocks() * 4 * latent, dtype=torch.float32,
                                           device=device)
         self.refresh_bf16()
@@ -412,8 +416,57 @@ class Network:
                                        _ptr(self.colsum_partial), _stream()), "sdem_sg_colsum")
 
     # -- forward
+    def _mlp(self, M: int, a: _Op, name: str, z=None, resid=None, out=None, out_bf=None, graph=None, agg=None) -> None:
+        """Both layers of MLP `name` over the M rows of a (sdem_sg_mlp)."""
+        kout, _ = self.shape(name + ".w2")
+        nagg, row_off, dst = (graph.n, graph.row_off, graph.dst) if graph is not None else (0, None, None)
+        _check(self.lib.sdem_sg_mlp(M, self.shape(name + ".w1")[1], C.byref(a.o), _ptr(self.pb, self.off(name + ".w1")),
+                                    _ptr(self.p, self.off(name + ".b1")), _ptr(self.pb, self.off(name + ".w2")),
+                                    _ptr(self.p, self.off(name + ".b2")), kout, _ptr(z), _ptr(resid), _ptr(out),
+                                    _ptr(out_bf), nagg, _ptr(row_off), _ptr(dst), _ptr(agg), _stream()), "sdem_sg_mlp")
+
+    def _forward_fused(self, g: Graph, xn: torch.Tensor, keep: bool) -> torch.Tensor:
+        """forward() with one kernel per MLP; the same bits."""
+        L, n, E, dev = self.latent, g.n, g.E, self.device
+
+        def new(rows, dtype=torch.bfloat16, width=L):
+            return torch.empty((max(rows, 1), width), dtype=dtype, device=dev)
+
+        def z(rows):
+            return new(rows) if keep else None
+
+        zn, ze = z(n), z(E)
+        h, hb, e, eb = new(n, torch.float32), new(n), new(E, torch.float32), new(E)
+        self._mlp(n, _Op(0, (xn, 0, NODE_IN, NODE_IN, None)), "enc_n", zn, out=h, out_bf=hb)
+        self._mlp(E, _Op(0, (g.efeat, 0, EDGE_IN, EDGE_IN, None)), "enc_e", ze, out=e, out_bf=eb)
+        saved = {"xn": xn, "zb_enc": zn, "zeb_enc": ze, "hb": [hb], "eb": [eb], "ze": [], "zn": [], "agg": []}
+        for l in range(self.layers):
+            last = l == self.layers - 1
+            ze, eb2 = z(E), None if last else new(E)
+            agg = torch.zeros((max(n, 1), L), dtype=torch.bfloat16, device=dev)
+            # the residual streams are updated in place: nothing reads their
+            # fp32 values again; the last layer's edges only feed the sums
+            self._mlp(E, _Op(0, (hb, 0, L, L, g.dst), (hb, 0, L, L, g.src), (eb, 0, L, L, None)), f"edge{l}", ze,
+                      resid=None if last else e, out=None if last else e, out_bf=eb2, graph=g, agg=agg)
+            zn, hb2 = z(n), new(n)
+            self._mlp(n, _Op(0, (hb, 0, L, L, None), (agg, 0, L, L, None)), f"node{l}", zn, resid=h,
+                      out=None if last else h, out_bf=hb2)
+            if keep:
+                for name, t in (("ze", ze), ("zn", zn), ("agg", agg), ("hb", hb2), ("eb", eb2)):
+                    saved[name].append(t)
+            hb, eb = hb2, eb2
+        zd = z(n)
+        y = torch.empty((n, OUT), dtype=torch.float32, device=dev)
+        self._mlp(n, _Op(0, (hb, 0, L, L, None)), "dec", zd, out=y)
+        saved["zd"] = zd
+        self.saved = saved if keep else None
+        self.graph = g if keep else None
+        return y
+
     def forward(self, g: Graph, xn: torch.Tensor, keep: bool = True) -> torch.Tensor:
         """(n, 16) fp32 predictions; keep=True saves what backward needs."""
+        if self.fused:
+            return self._forward_fused(g, xn, keep)
         L, n, E, dev = self.latent, g.n, g.E, self.device
         bf, f32 = torch.bfloat16, torch.float32
         zb = torch.empty((n, L), dtype=bf, device=dev)
