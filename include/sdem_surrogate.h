@@ -67,6 +67,19 @@ int sdem_sg_edge_fill(int n, const double* posR, const sdem_sg_grid* g, const in
                       const int* cell_start, const int* sorted, const int* row_off, int* dst, int* src,
                       uint16_t* efeat, void* stream);
 
+/* The same graph in two calls, sorted and counted on the device.  work:
+ * sdem_sg_graph_work(n, g) bytes (0: bad arguments), 256-byte aligned, the same
+ * for both calls, contents of no meaning to the caller but the first two
+ * words: after sdem_sg_graph_count the number of edges as an unsigned 64-bit
+ * integer, then an int status (0; otherwise a bounded device-side wait ran out
+ * and the graph is not valid).  row_off (n+1, 16-byte aligned) is exact while
+ * that number is below 2^31.  sdem_sg_graph_fill then writes dst, src and efeat
+ * as sdem_sg_edge_fill does; posR and g as in the first call.  n >= 1. */
+long long sdem_sg_graph_work(int n, const sdem_sg_grid* g);
+int sdem_sg_graph_count(int n, const double* posR, const sdem_sg_grid* g, void* work, int* row_off, void* stream);
+int sdem_sg_graph_fill(int n, const double* posR, const sdem_sg_grid* g, void* work, const int* row_off, int* dst,
+                       int* src, uint16_t* efeat, void* stream);
+
 /* Node features (32 bf16 per sphere): three velocity frames v(t), v(t-S),
  * v(t-2S) divided by vscale (9), omega r / vscale (3), 2r/scale, the signed
  * distances to up to 5 planes (n.x + d, planes: nw x 4 doubles nx ny nz d)

@@ -22,10 +22,11 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 SRC = os.path.join(HERE, "csrc", "sdem_gpu.cu")
 DEPS = [SRC, os.path.join(HERE, "csrc", "dem_device.cuh"), os.path.join(HERE, "csrc", "fp64_int.cuh"),
-        os.path.join(ROOT, "include", "sdem_gpu.h")]
+        os.path.join(HERE, "csrc", "scan.cuh"), os.path.join(ROOT, "include", "sdem_gpu.h")]
 LIB = os.path.join(HERE, "libsdem_gpu.so")
 SG_SRC = os.path.join(HERE, "csrc", "surrogate.cu")
-SG_DEPS = [SG_SRC, os.path.join(ROOT, "include", "sdem_surrogate.h")]
+SG_DEPS = [SG_SRC, os.path.join(HERE, "csrc", "fp64_int.cuh"), os.path.join(HERE, "csrc", "scan.cuh"),
+           os.path.join(ROOT, "include", "sdem_surrogate.h")]
 SG_LIB = os.path.join(HERE, "libsdem_surrogate.so")
 BG_SRC = os.path.join(HERE, "csrc", "bedgen.c")
 BG_LIB = os.path.join(HERE, "libsdem_bedgen.so")

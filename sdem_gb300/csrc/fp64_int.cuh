@@ -347,6 +347,19 @@ __host__ __device__ __forceinline__ float to_float_trunc(double x) {
   return (float)x;
 }
 
+// (float)x, round to nearest even, on the integer pipes where x rounds to a
+// normal float (the hardware conversion takes the FP64 pipe's rate on GB300);
+// zeros, other results, infinities and NaNs take the hardware conversion.
+__host__ __device__ __forceinline__ float to_float_rn(double x) {
+  const uint64_t u = bits(x);
+  const uint32_t e = (uint32_t)(u >> 52) & 0x7FFu;
+  if (e - 897u < 253u) {   // 2^-126 <= |x| < 2^127: rounding up a binade stays finite
+    const uint64_t m = (u & ~kSign) + 0x0FFFFFFFull + ((u >> 29) & 1ull);
+    return ffrom((uint32_t)(u >> 63) << 31 | ((uint32_t)(m >> 29) - (896u << 23)));
+  }
+  return (float)x;
+}
+
 // x * (-0.5), exact for every x whose half is a normal number or zero: the
 // exponent field drops by one and the sign flips.  Subnormal halves (which
 // round), infinities and NaNs take the hardware multiplication.

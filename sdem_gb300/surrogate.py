@@ -55,7 +55,7 @@ OVERLAP_GAIN = 100.0
 EXPORTED = ("sdem_sg_cells", "sdem_sg_edge_count", "sdem_sg_edge_fill", "sdem_sg_node_features", "sdem_sg_gemm",
             "sdem_sg_segsum", "sdem_sg_gather_add", "sdem_sg_colsum_blocks", "sdem_sg_colsum", "sdem_sg_mse",
             "sdem_sg_adam", "sdem_sg_to_bf16", "sdem_sg_advance", "sdem_sg_set_tensor_path",
-            "sdem_sg_tensor_timeouts", "sdem_sg_mlp")
+            "sdem_sg_tensor_timeouts", "sdem_sg_mlp", "sdem_sg_graph_work", "sdem_sg_graph_count", "sdem_sg_graph_fill")
 
 
 class SgGrid(C.Structure):
@@ -110,12 +110,15 @@ def load(path: str = LIB_PATH):
         "sdem_sg_advance": [I, P, I, D, D, D, D, D, C.POINTER(SgBox), P, P, P, P],
         "sdem_sg_set_tensor_path": [I],
         "sdem_sg_tensor_timeouts": [C.POINTER(C.c_uint)],
+        "sdem_sg_graph_work": [I, C.POINTER(SgGrid)],
+        "sdem_sg_graph_count": [I, P, C.POINTER(SgGrid), P, P, P],
+        "sdem_sg_graph_fill": [I, P, C.POINTER(SgGrid), P, P, P, P, P, P],
         "sdem_sg_mlp": [I, I, C.POINTER(SgOperand), P, P, P, P, I, P, P, P, P, I, P, P, P, P],
     }
     for name, args in sig.items():
         fn = getattr(lib, name)
         fn.argtypes = args
-        fn.restype = C.c_int
+        fn.restype = C.c_longlong if name == "sdem_sg_graph_work" else C.c_int
     _lib = lib
     return lib
 
@@ -227,10 +230,45 @@ def make_grid(lo, hi, d_max: float) -> SgGrid:
     return g
 
 
-def build_graph(posR: torch.Tensor, grid: SgGrid, sender_order: bool = True) -> Graph:
-    """Neighbour graph of the spheres in posR (cuda float64, n x 4); the
-    sender-ordered permutation (needed by the backward pass only) is built
-    when sender_order is set."""
+def _edge_arrays(E: int, dev):
+    # at least one row: an empty tensor has a null data pointer, which the
+    # library refuses even when there is nothing to write
+    return (torch.empty(max(E, 1), dtype=torch.int32, device=dev)[:E],
+            torch.empty(max(E, 1), dtype=torch.int32, device=dev)[:E],
+            torch.empty((max(E, 1), EDGE_IN), dtype=torch.bfloat16, device=dev))
+
+
+def _check_edges(E: int) -> None:
+    if E > 2**31 - 1:
+        # the CSR offsets and edge indices are int32 on the device
+        raise RuntimeError(f"{E} edges: more than the int32 offsets of the graph can address")
+
+
+def _edges_on_device(posR: torch.Tensor, grid: SgGrid):
+    """Sort, count, offsets and edges by the library alone; the one word that
+    comes back in between is the number of edges."""
+    lib = load()
+    n, dev, s = posR.shape[0], posR.device, _stream()
+    posR = posR.contiguous()
+    size = int(lib.sdem_sg_graph_work(n, C.byref(grid)))
+    if size <= 0:
+        raise RuntimeError("sdem_sg_graph_work failed (bad grid)")
+    work = torch.empty(size, dtype=torch.uint8, device=dev)
+    row_off = torch.empty(n + 1, dtype=torch.int32, device=dev)
+    _check(lib.sdem_sg_graph_count(n, _ptr(posR), C.byref(grid), _ptr(work), _ptr(row_off), s), "sdem_sg_graph_count")
+    E, status = (int(v) for v in work[:16].view(torch.int64).cpu())
+    if status & 0xFFFFFFFF:
+        raise RuntimeError("sdem_sg_graph_count: a device-side wait ran out")
+    _check_edges(E)
+    dst, src, efeat = _edge_arrays(E, dev)
+    if E:
+        _check(lib.sdem_sg_graph_fill(n, _ptr(posR), C.byref(grid), _ptr(work), _ptr(row_off), _ptr(dst), _ptr(src),
+                                      _ptr(efeat), s), "sdem_sg_graph_fill")
+    return row_off, dst, src, efeat, E
+
+
+def _edges_by_steps(posR: torch.Tensor, grid: SgGrid):
+    """The same from the library's single steps, sorts and prefix sums by torch."""
     lib = load()
     n = posR.shape[0]
     dev = posR.device
@@ -248,18 +286,25 @@ def build_graph(posR: torch.Tensor, grid: SgGrid, sender_order: bool = True) -> 
                                   _ptr(degree), s), "sdem_sg_edge_count")
     csum = torch.cumsum(degree.to(torch.int64), 0)
     E = int(csum[-1].item()) if n else 0
-    if E > 2**31 - 1:
-        # the CSR offsets and edge indices are int32 on the device
-        raise RuntimeError(f"{E} edges: more than the int32 offsets of the graph can address")
+    _check_edges(E)
     row_off = torch.zeros(n + 1, dtype=torch.int32, device=dev)
     row_off[1:] = csum.to(torch.int32)
-    # at least one row: an empty tensor has a null data pointer, which the
-    # library refuses even when there is nothing to write
-    dst = torch.empty(max(E, 1), dtype=torch.int32, device=dev)[:E]
-    src = torch.empty(max(E, 1), dtype=torch.int32, device=dev)[:E]
-    efeat = torch.empty((max(E, 1), EDGE_IN), dtype=torch.bfloat16, device=dev)
+    dst, src, efeat = _edge_arrays(E, dev)
     _check(lib.sdem_sg_edge_fill(n, _ptr(posR), C.byref(grid), _ptr(cell), _ptr(cell_start), _ptr(sorted_idx),
                                  _ptr(row_off), _ptr(dst), _ptr(src), _ptr(efeat), s), "sdem_sg_edge_fill")
+    return row_off, dst, src, efeat, E
+
+
+def build_graph(posR: torch.Tensor, grid: SgGrid, sender_order: bool = True) -> Graph:
+    """Neighbour graph of the spheres in posR (cuda float64, n x 4); the
+    sender-ordered permutation (needed by the backward pass only) is built
+    when sender_order is set."""
+    n = posR.shape[0]
+    dev = posR.device
+    if n and posR.is_cuda:
+        row_off, dst, src, efeat, E = _edges_on_device(posR, grid)
+    else:
+        row_off, dst, src, efeat, E = _edges_by_steps(posR, grid)
     src_perm = src_off = None
     if sender_order:
         skey = src.to(torch.int64) * max(E, 1) + torch.arange(E, device=dev, dtype=torch.int64)
