@@ -126,9 +126,9 @@ __global__ void k_edges(int n, const double* __restrict__ posR, sdem_sg_grid g, 
 // test (which k_edges runs for every candidate, twice, on GB300's two FP64
 // operations per SM per clock).  Square roots and divisions of the features run
 // on the integer pipes (fp64_int.cuh), bit-identical to the hardware's.
-// 200k spheres, 3.9M edges: 7.0 ms as k_edges twice with torch's sorts and prefix
-// sums in between, GRTOTAL here, of which the edges' features FILLUS (FP64 pipe
-// bound: 10 additions and multiplications an edge).
+// 200k spheres, 3.9M edges: 7.0 ms as k_edges twice with torch's sorts and
+// prefix sums in between, 0.36 ms here, of which the edges' features 192 us
+// (FP64 pipe 70% busy).
 constexpr int GR_CAP = 96;    // neighbours kept per sphere between the two calls; longer lists are searched again
 constexpr int GR_T = 256;
 
@@ -1616,7 +1616,8 @@ __global__ void k_split_reduce(int I, int J, int splits, const float* __restrict
     const size_t IJ = (size_t)I * J;
     if (k >= IJ) return;
     float s = 0.f;
-#pragma unroll 16
+    // many loads in flight, added in split order
+#pragma unroll 32
     for (int z = 0; z < splits; ++z) s += partial[z * IJ + k];
     const int i = (int)(k / J), j = (int)(k % J);
     float* o = out + (size_t)i * ld_out + j;
@@ -1644,6 +1645,33 @@ __global__ void k_segsum(int nrows, int J, const int* __restrict__ row_off, cons
     }
 }
 
+// rows of whole float4s, eight columns a thread (k_gather_add: one; 337k rows of
+// 128 columns with a gather, an addend and a bf16 copy: 210 us, 67 here at 6.5 TB/s
+// of HBM)
+__global__ void k_gather_add8(int rows, int J8, const int* __restrict__ idx, const float* __restrict__ x, int ldx,
+                              const float* __restrict__ y, int ldy, float* __restrict__ out, int ld_out,
+                              uint16_t* __restrict__ out_bf, int ld_out_bf) {
+    const size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= (size_t)rows * J8) return;
+    const size_t e = k / J8;
+    const int j = (int)(k % J8) * 8;
+    const size_t xr = idx ? (size_t)__ldg(idx + e) : e;
+    float4 v[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        v[h] = *reinterpret_cast<const float4*>(x + xr * ldx + j + 4 * h);
+        if (y) {
+            const float4 u = *reinterpret_cast<const float4*>(y + e * ldy + j + 4 * h);
+            v[h] = make_float4(u.x + v[h].x, u.y + v[h].y, u.z + v[h].z, u.w + v[h].w);
+        }
+        if (out) *reinterpret_cast<float4*>(out + e * ld_out + j + 4 * h) = v[h];
+    }
+    if (out_bf)
+        *reinterpret_cast<uint4*>(out_bf + e * ld_out_bf + j) =
+            make_uint4(bf16_pair(v[0].x, v[0].y), bf16_pair(v[0].z, v[0].w), bf16_pair(v[1].x, v[1].y),
+                       bf16_pair(v[1].z, v[1].w));
+}
+
 __global__ void k_gather_add(int rows, int J, const int* __restrict__ idx, const float* __restrict__ x, int ldx,
                              const float* __restrict__ y, int ldy, float* __restrict__ out, int ld_out,
                              uint16_t* __restrict__ out_bf, int ld_out_bf) {
@@ -1669,10 +1697,54 @@ __global__ void k_colsum_part(int M, int J, const float* __restrict__ x, int ldx
     }
 }
 
+// The same chunks and order of additions for rows of 128 floats: the rows of a
+// chunk come through shared memory, three tiles of 32 rows in flight (cp.async),
+// where one thread per column left one load in flight at a time (148 us for
+// 337k rows, 41 here).
+constexpr int CS_ROWS = 32, CS_STAGES = 4;
+__global__ void __launch_bounds__(256) k_colsum_part128(int M, const float* __restrict__ x, int ldx,
+                                                        float* __restrict__ partial) {
+    extern __shared__ __align__(16) float cs_tile[];   // CS_STAGES x CS_ROWS x 128
+    const int chunk = (M + kColsumBlocks - 1) / kColsumBlocks;
+    const int r0 = blockIdx.x * chunk, r1 = min(M, r0 + chunk);
+    const int tiles = r1 > r0 ? (r1 - r0 + CS_ROWS - 1) / CS_ROWS : 0;
+    auto copy = [&](int t) {
+        if (t < tiles) {
+            const uint32_t dst = smem_u32(cs_tile + (t % CS_STAGES) * CS_ROWS * 128);
+#pragma unroll
+            for (int q = 0; q < CS_ROWS * 32 / 256; ++q) {
+                const int c = threadIdx.x + q * 256, r = r0 + t * CS_ROWS + (c >> 5);
+                cp16(dst + c * 16, r < r1 ? x + (size_t)r * ldx + (c & 31) * 4 : x, r < r1 ? 16u : 0u);
+            }
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    for (int t = 0; t < CS_STAGES - 1; ++t) copy(t);
+    float s = 0.f;
+    for (int t = 0; t < tiles; ++t) {
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(CS_STAGES - 2) : "memory");
+        __syncthreads();
+        copy(t + CS_STAGES - 1);   // into the tile read in the last round
+        if (threadIdx.x < 128) {
+            const float* v = cs_tile + (t % CS_STAGES) * CS_ROWS * 128 + threadIdx.x;
+            const int rows = min(CS_ROWS, r1 - r0 - t * CS_ROWS);
+            if (rows == CS_ROWS) {
+#pragma unroll
+                for (int r = 0; r < CS_ROWS; ++r) s += v[r * 128];
+            } else {
+                for (int r = 0; r < rows; ++r) s += v[r * 128];
+            }
+        }
+    }
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    if (threadIdx.x < 128) partial[(size_t)blockIdx.x * 128 + threadIdx.x] = s;
+}
+
 __global__ void k_colsum_final(int J, const float* __restrict__ partial, float* __restrict__ out, int accumulate) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= J) return;
     float s = 0.f;
+#pragma unroll 32
     for (int b = 0; b < kColsumBlocks; ++b) s += partial[(size_t)b * J + j];
     out[j] = accumulate ? out[j] + s : s;
 }
@@ -2028,6 +2100,12 @@ int sdem_sg_gather_add(int rows, int J, const int* idx, const float* x, int ldx,
         return SDEM_SG_E_ARG;
     if (rows == 0 || J == 0) return SDEM_SG_OK;
     if (!x || (!out && !out_bf)) return SDEM_SG_E_ARG;
+    if (J % 8 == 0 && ldx % 4 == 0 && aligned16(x) && (!y || (aligned16(y) && ldy % 4 == 0)) &&
+        (!out || (aligned16(out) && ld_out % 4 == 0)) && (!out_bf || (aligned16(out_bf) && ld_out_bf % 8 == 0))) {
+        k_gather_add8<<<blocks((long long)rows * (J / 8), 256), 256, 0, st(stream)>>>(rows, J / 8, idx, x, ldx, y, ldy, out,
+                                                                                     ld_out, out_bf, ld_out_bf);
+        return launched();
+    }
     k_gather_add<<<blocks((long long)rows * J, 256), 256, 0, st(stream)>>>(rows, J, idx, x, ldx, y, ldy, out, ld_out,
                                                                           out_bf, ld_out_bf);
     return launched();
@@ -2039,7 +2117,13 @@ int sdem_sg_colsum(int M, int J, const float* x, int ldx, float* out, int accumu
     if (M < 0 || J < 0 || ldx < J) return SDEM_SG_E_ARG;
     if (J == 0) return SDEM_SG_OK;
     if (!out || !partial || (M > 0 && !x)) return SDEM_SG_E_ARG;
-    k_colsum_part<<<kColsumBlocks, 128, 0, st(stream)>>>(M, J, x, ldx, partial);
+    if (J == 128 && ldx % 4 == 0 && aligned16(x)) {
+        const int smem = CS_STAGES * CS_ROWS * 128 * 4;
+        if (!set_smem((const void*)k_colsum_part128, smem)) return SDEM_SG_E_CUDA;
+        k_colsum_part128<<<kColsumBlocks, 256, smem, st(stream)>>>(M, x, ldx, partial);
+    } else {
+        k_colsum_part<<<kColsumBlocks, 128, 0, st(stream)>>>(M, J, x, ldx, partial);
+    }
     if (cudaGetLastError() != cudaSuccess) return SDEM_SG_E_CUDA;
     k_colsum_final<<<blocks(J, 128), 128, 0, st(stream)>>>(J, partial, out, accumulate);
     return launched();

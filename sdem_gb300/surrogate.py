@@ -596,7 +596,8 @@ class Network:
         self._dgrad(n, _Op(0, (dzb, 0, L, L, None)), "dec.w1", out=dh, ld_out=L, out_bf=dhb, ld_out_bf=L)
         de = torch.zeros((max(E, 1), L), dtype=f32, device=dev)
         din_n = torch.empty((n, 2 * L), dtype=f32, device=dev)
-        din_e = torch.empty((max(E, 1), 3 * L), dtype=f32, device=dev)
+        din_e = torch.empty((max(E, 1), 2 * L), dtype=f32, device=dev)
+        deb = torch.empty((max(E, 1), L), dtype=bf, device=dev)
         dm = torch.empty((max(E, 1), L), dtype=f32, device=dev)
         dmb = torch.empty((max(E, 1), L), dtype=bf, device=dev)
         dze = torch.empty((max(E, 1), L), dtype=f32, device=dev)
@@ -627,15 +628,19 @@ class Network:
             self._wgrad(f"edge{l}.w1", E, _Op(1, (dzeb, 0, L, L, None)),
                         _Op(1, (hb_prev, 0, L, L, g.dst), (hb_prev, 0, L, L, g.src), (eb_prev, 0, L, L, None)))
             self._bgrad(f"edge{l}.b1", E, dze, L)
-            self._dgrad(E, _Op(0, (dzeb, 0, L, L, None)), f"edge{l}.w1", out=din_e, ld_out=3 * L)
-            de_prev = torch.empty_like(de)
-            _check(lib.sdem_sg_gather_add(E, L, None, _ptr(din_e, 2 * L), 3 * L, _ptr(de), L, _ptr(de_prev), L, None,
-                                          L, _stream()), "sdem_sg_gather_add")
-            _check(lib.sdem_sg_segsum(n, L, _ptr(g.row_off), None, _ptr(din_e), 3 * L, _ptr(dh_prev), L, 1, None, L,
+            # the input gradient by columns of W1: [h_dst, h_src] for the sums
+            # below, e straight onto its residual stream (in place)
+            w1 = self.off(f"edge{l}.w1")
+            dz_op = _Op(0, (dzeb, 0, L, L, None))
+            self._gemm(E, 2 * L, L, dz_op, _Op(1, (self.pb, w1, 3 * L, 2 * L, None)), _ep(out=din_e, ld_out=2 * L))
+            self._gemm(E, L, L, dz_op, _Op(1, (self.pb, w1 + 2 * L, 3 * L, L, None)),
+                       _ep(resid=de, ld_resid=L, res_out=de, ld_res_out=L, res_out_bf=deb if l == 0 else None,
+                           ld_res_out_bf=L))
+            _check(lib.sdem_sg_segsum(n, L, _ptr(g.row_off), None, _ptr(din_e), 2 * L, _ptr(dh_prev), L, 1, None, L,
                                       _stream()), "sdem_sg_segsum")
-            _check(lib.sdem_sg_segsum(n, L, _ptr(g.src_off), _ptr(g.src_perm), _ptr(din_e, L), 3 * L, _ptr(dh_prev),
+            _check(lib.sdem_sg_segsum(n, L, _ptr(g.src_off), _ptr(g.src_perm), _ptr(din_e, L), 2 * L, _ptr(dh_prev),
                                       L, 1, _ptr(dhb), L, _stream()), "sdem_sg_segsum")
-            dh, de = dh_prev, de_prev
+            dh = dh_prev
         # encoders
         self._wgrad("enc_n.w2", n, _Op(1, (dhb, 0, L, L, None)), _Op(1, (s["zb_enc"], 0, L, L, None)))
         self._bgrad("enc_n.b2", n, dh, L)
@@ -643,8 +648,8 @@ class Network:
                     out_bf=dzb, ld_out_bf=L)
         self._wgrad("enc_n.w1", n, _Op(1, (dzb, 0, L, L, None)), _Op(1, (s["xn"], 0, NODE_IN, NODE_IN, None)))
         self._bgrad("enc_n.b1", n, dz, L)
-        deb = torch.empty((max(E, 1), L), dtype=bf, device=dev)
-        _check(lib.sdem_sg_to_bf16(E * L, _ptr(de), _ptr(deb), _stream()), "sdem_sg_to_bf16")
+        if not self.layers:   # otherwise the first layer's input gradient wrote it
+            _check(lib.sdem_sg_to_bf16(E * L, _ptr(de), _ptr(deb), _stream()), "sdem_sg_to_bf16")
         self._wgrad("enc_e.w2", E, _Op(1, (deb, 0, L, L, None)), _Op(1, (s["zeb_enc"], 0, L, L, None)))
         self._bgrad("enc_e.b2", E, de, L)
         self._dgrad(E, _Op(0, (deb, 0, L, L, None)), "enc_e.w2", mask=s["zeb_enc"], ld_mask=L, out=dze, ld_out=L,
