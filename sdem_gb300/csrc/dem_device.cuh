@@ -46,8 +46,10 @@ __device__ __forceinline__ r3 add3(r3 a, r3 b) { return mk3(a.x + b.x, a.y + b.y
 __device__ __forceinline__ r3 sub3(r3 a, r3 b) { return mk3(a.x - b.x, a.y - b.y, a.z - b.z); }
 __device__ __forceinline__ r3 scale3(r3 p, double v) { return mk3(p.x * v, p.y * v, p.z * v); }
 __device__ __forceinline__ r3 div3(r3 p, double v) {
-  const fpi::Divisor dv = fpi::divisor(v);   // one reciprocal refinement for three quotients
-  return mk3(fpi::div_by(p.x, dv), fpi::div_by(p.y, dv), fpi::div_by(p.z, dv));
+  const double x[3] = {p.x, p.y, p.z};
+  double q[3];
+  fpi::div_three(x, fpi::divisor(v), q);   // one reciprocal refinement for three quotients
+  return mk3(q[0], q[1], q[2]);
 }
 __device__ __forceinline__ double dot3(r3 a, r3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
 __device__ __forceinline__ r3 cross3(r3 u, r3 v) {
@@ -186,6 +188,12 @@ struct LawCfg {
 // unfused ones' 8.3e-17.  The chain up to vrn keeps the reference's roundings:
 // where a new pair meets almost tangentially |vrn| is the small difference of
 // large terms, and it is kept for the contact's life as VelRel_Init.
+// In a small bed the kernel takes as long as one warp of it: 98 FP64
+// instructions of 64 cycles each, and the chains of the roots and quotients,
+// which therefore run in 32-bit products and side by side (fp64_int.cuh).  Per
+// step, before and after: linear spring 54.7 -> 43.7 us at 2k spheres and
+// 60.5 -> 49 at 20k (of it the powers without pow ~7), Hertz 64 -> 57 at 50k,
+// 206 -> 190 at 200k, 716 -> 648 at 1M.
 __device__ __forceinline__ void force_law(const LawCfg& L, const double* P, r3 Veli, r3 Velj,
                                           r3 Rvei, r3 Rvej, double ri, double rj, r3 Norm_v,
                                           double ovrlp, dbl4& hist, r3& S, r3& M, r3& Mr) {
@@ -198,12 +206,40 @@ __device__ __forceinline__ void force_law(const LawCfg& L, const double* P, r3 V
 
   r3 Vij_t = fma3(Norm_v, -vrn, Vrij);
 
+  // The lengths and the Hertz law's root of the overlap together, then the
+  // ratio of the two lengths, the rolling direction and the fourth root: a warp
+  // waits for the longest chain of each group, not for their sum.
   r3 Ovlp_t = mk3(hist.x, hist.y, hist.z);
-  double normTan1 = norm3f(Ovlp_t);
+  r3 W_hat = sub3(Rvei, Rvej);
+  const double tan1 = dot3f(Ovlp_t, Ovlp_t);
   Ovlp_t = fma3(Norm_v, -dot3f(Ovlp_t, Norm_v), Ovlp_t);
-  double normTan2 = norm3f(Ovlp_t);
-  if (fpi::gt(normTan2, 1.0E-10)) Ovlp_t = scale3(Ovlp_t, fpi::div_rn(normTan1, normTan2));
+  const bool lsd = L.cf_type == SDEM_CFT_LSD;
+  const double sq2[4] = {tan1, dot3f(Ovlp_t, Ovlp_t), dot3f(W_hat, W_hat), lsd ? 1.0 : ovrlp};
+  double len[4];   // |history|, |its tangential part|, |W_hat|, ovrlp**0.5
+  fpi::sqrt_many(sq2, len);
+  const bool t_on = fpi::gt(len[1], 1.0E-10), w_on = fpi::gt(len[2], 1.0E-10);
+  double ratio, o025;
+  {
+    const fpi::Divisor dt = fpi::divisor(len[1]), dw = fpi::divisor(len[2]);
+    bool st, sx, sy, sz;
+    ratio = fpi::from_bits(fpi::div_normal(fpi::bits(len[0]), dt, st));
+    const r3 w = W_hat;
+    W_hat.x = fpi::from_bits(fpi::div_normal(fpi::bits(w.x), dw, sx));
+    W_hat.y = fpi::from_bits(fpi::div_normal(fpi::bits(w.y), dw, sy));
+    W_hat.z = fpi::from_bits(fpi::div_normal(fpi::bits(w.z), dw, sz));
+    o025 = fpi::from_bits(fpi::sqrt_normal(fpi::bits(len[3])));
+    const bool so = fpi::sqrt_special(fpi::bits(len[3]));
+    if ((t_on && st) || (w_on && (sx || sy || sz)) || so) {
+      if (t_on && st) ratio = fpi::div_other(len[0], dt);
+      if (w_on && sx) W_hat.x = fpi::div_other(w.x, dw);
+      if (w_on && sy) W_hat.y = fpi::div_other(w.y, dw);
+      if (w_on && sz) W_hat.z = fpi::div_other(w.z, dw);
+      if (so) o025 = fpi::sqrt_other(len[3]);
+    }
+  }
+  if (t_on) Ovlp_t = scale3(Ovlp_t, ratio);
   else Ovlp_t = mk3(0.0, 0.0, 0.0);
+  if (!w_on) W_hat = mk3(0.0, 0.0, 0.0);
   Ovlp_t = fma3(Vij_t, L.dt, Ovlp_t);
 
   // Ftij = k_t*Ovlp_t + d_t*Vij_t with d_t = 0 (:29, :36): the second term is
@@ -212,20 +248,20 @@ __device__ __forceinline__ void force_law(const LawCfg& L, const double* P, r3 V
   // dropped (6 FP64 operations per contact).
   double fn, k_t;
   r3 Ftij;
-  if (L.cf_type == SDEM_CFT_LSD) {
+  if (lsd) {
     double Vel_in = fpi::gt(VelRel, 0.01) ? VelRel : 0.01;
-    double v04 = pow(Vel_in, 0.4);
+    double v02, v04;
+    fpi::fifth_powers(Vel_in, v02, v04);
     double k_n = -(P[SDEM_BP_KN] * v04);
-    double d_n = -(P[SDEM_BP_CN] * pow(Vel_in, 0.2));
+    double d_n = -(P[SDEM_BP_CN] * v02);
     fn = k_n * ovrlp + d_n * vrn;
     k_t = -(P[SDEM_BP_KT] * v04);
     Ftij = scale3(Ovlp_t, k_t);
   } else {
     double k_n = -P[SDEM_BP_KN];
     double d_n = -P[SDEM_BP_CN];
-    double sq = fpi::sqrt_rn(ovrlp);
+    double sq = len[3];
     double o15 = ovrlp * sq;   // ovrlp**1.5
-    double o025 = fpi::sqrt_rn(sq);    // ovrlp**0.25
     fn = k_n * o15 + d_n * o025 * vrn;
     k_t = -(P[SDEM_BP_KT] * sq);
     Ftij = scale3(Ovlp_t, k_t);
@@ -239,10 +275,6 @@ __device__ __forceinline__ void force_law(const LawCfg& L, const double* P, r3 V
     Ovlp_t = div3(Ftij, k_t);
   }
 
-  r3 W_hat = sub3(Rvei, Rvej);
-  double w_hat_mag = norm3f(W_hat);
-  if (fpi::gt(w_hat_mag, 1.0E-10)) W_hat = div3(W_hat, w_hat_mag);
-  else W_hat = mk3(0.0, 0.0, 0.0);
   if (L.ct_model == SDEM_CTM_CONSTANT)
     Mr = scale3(W_hat, -(P[SDEM_BP_MUR] * fabs(fn) * P[SDEM_BP_RADEFF]));
   else

@@ -5,9 +5,9 @@
 // holds an SM sub-partition's FP64 pipe for 64 cycles), against 64 integer
 // operations per SM per clock.  The hardware's correctly rounded sqrt and
 // division are sequences of ~10 and ~7 FP64-pipe operations; the force law
-// needs 7 of each per contact and is FP64-pipe bound with most issue slots
-// idle.  The versions here take an FP32 seed, refine it in 64-bit fixed point
-// and settle the last bit with an exact integer rounding test, so they run
+// needs 7 and more of them per contact and is FP64-pipe bound with most issue
+// slots idle.  The versions here take an FP32 seed, refine it in fixed point and
+// settle the last bit with an exact integer rounding test, so they run
 // beside the FP64 pipe instead of on it.  Results are bit-identical to the
 // hardware's __dsqrt_rn / __ddiv_rn for every input: normal operands and zeros
 // take the integer path; subnormal, infinite and NaN operands, and results
@@ -135,6 +135,28 @@ __host__ __device__ __forceinline__ float rcp_seed(float x) {
   return r;
 #endif
 }
+__host__ __device__ __forceinline__ float log2_seed(float x) {
+#ifdef __CUDA_ARCH__
+  float r;
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+#else
+  return __builtin_log2f(x);
+#endif
+}
+__host__ __device__ __forceinline__ float exp2_seed(float x) {
+#ifdef __CUDA_ARCH__
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+#else
+  float r = __builtin_exp2f(x);
+#ifdef FPI_HOST_SEED_HOOK
+  r = FPI_HOST_SEED_HOOK(r);
+#endif
+  return r;
+#endif
+}
 __host__ __device__ __forceinline__ int64_t smulhi(int64_t a, int64_t b) {
 #ifdef __CUDA_ARCH__
   return __mul64hi(a, b);
@@ -142,71 +164,76 @@ __host__ __device__ __forceinline__ int64_t smulhi(int64_t a, int64_t b) {
   return (int64_t)(((__int128)a * b) >> 64);
 #endif
 }
-// Q2.62 fixed point: value * 2^62 in a 64-bit word (values below 4)
-__host__ __device__ __forceinline__ uint64_t q62_from_seed(float r) {
-  // r = 1.m * 2^k, k in [-3, 1]: (2^23 + m) * 2^(39 + k) = r * 2^62
+// Q1.31 fixed point of a single-precision seed r in [1/4, 2)
+__host__ __device__ __forceinline__ uint32_t q31_from_seed(float r) {
   const uint32_t rb = fbits(r);
-  const int k = (int)(rb >> 23) - 127;
-  return ((uint64_t)((rb & 0x7FFFFFu) | 0x800000u)) << (39 + k);
+  return ((rb << 8) | 0x80000000u) >> (127u - (rb >> 23));
 }
+__host__ __device__ __forceinline__ uint64_t wide(uint32_t a, uint32_t b) { return (uint64_t)a * b; }
+__host__ __device__ __forceinline__ int64_t swide(int32_t a, int32_t b) { return (int64_t)a * b; }
 
-// sqrt(x), correctly rounded.  Positive normal x take the integer path:
-// x = M * 2^(2h) with M in [1, 4); a single-precision seed of 1/sqrt(M) is
-// refined by two coupled Newton (Goldschmidt) steps in Q3.61 fixed point,
-// g -> sqrt(M), h -> 1/(2 sqrt(M)), residual d = 1/2 - g*h (Goldschmidt,
-// 1964; Markstein, IBM J. Res. Dev. 34(1), 1990), which leave g within a
-// few 2^-58 of sqrt(M).  The candidate S = round(g * 2^52) is then settled by
-// the exact integer test of round-to-nearest, S^2 - S < M*2^104 <= S^2 + S,
-// and moved by one unit while it fails.  Other x take the hardware sqrt.
-__host__ __device__ __forceinline__ double sqrt_rn(double x) {
-  const uint64_t u = bits(x);
-  const uint32_t e = (uint32_t)(u >> 52);      // the sign bit makes negatives large
-  if (e - 1u >= 2046u) {
-    if ((u << 1) == 0) return x;               // sqrt(+-0) = +-0
-    return hw_sqrt(x);
-  }
+// The refinements below run in 32x32-bit products: an operand enters a step
+// with the bits the step's result can hold, and the residual of the last step
+// (A - g^2, a*2^30 - q*b) is exact modulo 2^64 and small.  One lane's chain is
+// what a small bed waits for (a warp of the force law runs 6 square roots and
+// 9 quotients, one after the other), and at 1M spheres fewer instructions leave
+// the FP64 pipe fewer gaps.
+// The errors, with e0 the seed's: 2^-22 on the GPU, and still sound at 2^-17.
+
+// sqrt(x), correctly rounded, for positive normal x: x = M * 2^(2h) with M in
+// [1, 4).  r, a single-precision seed of 1/sqrt(M), takes one Newton step
+// (r <- r + r*(1 - M r^2)/2) to within 2^-29; g = M r is corrected by the exact
+// residual, g <- g + r*(M - g^2)/2 (Markstein, IBM J. Res. Dev. 34(1), 1990),
+// to within 2^-56.  The candidate S = round(g * 2^52) is then settled by the
+// exact integer test of round-to-nearest, S^2 - S < M*2^104 <= S^2 + S, and
+// moved by one unit if it fails.
+__host__ __device__ __forceinline__ uint64_t sqrt_normal(uint64_t u) {
   const uint64_t f = u & kMant;
-  const int E = (int)e - 1023;
+  const int E = (int)((uint32_t)(u >> 52) & 0x7FFu) - 1023;
   const uint32_t odd = (uint32_t)E & 1u;
   const uint64_t A = ((f | kHid) << 10) << odd;            // M in Q2.62
-  const float fm = ffrom(((127u + odd) << 23) | (uint32_t)(f >> 29));
-  const uint64_t R0 = q62_from_seed(rsqrt_seed(fm));       // ~1/sqrt(M), Q2.62
-  // g and h in Q3.61: sqrt(M) reaches 2, and a seed error must not overflow
-  int64_t g = (int64_t)(mulhi(A, R0) << 1);                 // ~sqrt(M)
-  int64_t hh = (int64_t)(R0 >> 2);                          // ~1/(2 sqrt(M))
-#pragma unroll
-  for (int it = 0; it < 2; it++) {
-    const int64_t p = (int64_t)(mulhi((uint64_t)g, (uint64_t)hh) << 3);
-    const int64_t d = ((int64_t)1 << 60) - p;
-    g += (int64_t)((uint64_t)smulhi(g, d) << 3);
-    hh += (int64_t)((uint64_t)smulhi(hh, d) << 3);
-  }
-  uint64_t S = ((uint64_t)g + (1u << 8)) >> 9;              // ~sqrt(M) * 2^52
+  const uint32_t m = (uint32_t)(A >> 32);                  // M in Q2.30
+  const uint32_t r0 = q31_from_seed(rsqrt_seed(ffrom(((127u + odd) << 23) | (uint32_t)(f >> 29))));
+  const uint32_t p = (uint32_t)(wide(r0, r0) >> 31);       // r^2 in Q1.31
+  const int32_t d = (int32_t)((int64_t)((1ull << 61) - wide(m, p)) >> 16);   // 1 - M r^2 in Q.45
+  const uint32_t r = r0 + (uint32_t)(swide((int32_t)(r0 >> 1), d) >> 45);    // Q.75 / 2 to Q1.31
+  const uint32_t g = (uint32_t)(wide(m, r) >> 31);         // ~sqrt(M) in Q2.30
+  const int64_t res = (int64_t)(A - (wide(g, g) << 2));    // M - g^2 in Q.62, exact, below 2^37
+  const int64_t c = swide((int32_t)(res >> 7), (int32_t)(r >> 1));            // Q.85
+  uint64_t S = (((uint64_t)g << 31) + (uint64_t)(c >> 25) + (1u << 8)) >> 9;  // ~sqrt(M) * 2^52
   // D = M*2^104 - S^2, exact in 64 bits while S is within a few units
-  const uint64_t Nlo = A << 42;
-  int64_t D = (int64_t)(Nlo - S * S);
-#pragma unroll
-  for (int it = 0; it < 2; it++) {
-    if (D > (int64_t)S) { D -= (int64_t)(2 * S + 1); S += 1; }
-    else if (D <= -(int64_t)S) { D += (int64_t)(2 * S - 1); S -= 1; }
-  }
+  const int64_t D = (int64_t)((A << 42) - S * S);
+  S += (uint64_t)(D > (int64_t)S) - (uint64_t)(D <= -(int64_t)S);
   const int er = ((E - (int)odd) >> 1) + 1023;
-  return from_bits((((uint64_t)(er - 1)) << 52) + S);
+  return (((uint64_t)(er - 1)) << 52) + S;
+}
+// operands for sqrt_normal: positive and normal
+__host__ __device__ __forceinline__ bool sqrt_special(uint64_t u) { return (uint32_t)(u >> 52) - 1u >= 2046u; }
+// the others: zeros, subnormals, negatives, infinities, NaN
+__host__ __device__ __forceinline__ double sqrt_other(double x) {
+  return (bits(x) << 1) == 0 ? x : hw_sqrt(x);   // sqrt(+-0) = +-0
+}
+__host__ __device__ __forceinline__ double sqrt_rn(double x) {
+  const uint64_t u = bits(x);
+  if (sqrt_special(u)) return sqrt_other(x);
+  return from_bits(sqrt_normal(u));
 }
 
 // x / y, correctly rounded.  Normal x and y with a normal quotient take the
-// integer path: the significand ratio Q = (mx/my) * 2^k in [1, 2) comes from a
-// single-precision seed of 1/my refined by two Newton steps in Q2.62
-// (z <- z + z*(1 - my*z)), the candidate S = round(Q * 2^52) is settled by the
-// exact remainder R = mx*2^(52+k) - S*my (round to nearest: |R| <= my/2, ties
-// to the even S) and moved by one unit while the test fails.  Zeros,
-// subnormals, infinities, NaNs and quotients outside the normal range take
-// the hardware division.  The refined reciprocal depends on y only, so
-// several quotients by one divisor share it (Divisor).
+// integer path: the significand ratio Q = (mx/my) * 2^k in [1, 2) starts as
+// q = mx * z with z a reciprocal of my to within 2^-29, is corrected by the exact
+// remainder, q + (mx - q*my)*z, to within 2^-56, and the candidate
+// S = round(Q * 2^52) is settled by the exact remainder R = mx*2^(52+k) - S*my
+// (round to nearest: |R| < my/2; a quotient of two 53-bit significands never
+// lies half-way) and moved by one unit if the test fails.  Zeros, subnormals,
+// infinities, NaNs and quotients outside the normal range take the hardware
+// division.  The refined reciprocal depends on y only, so several quotients by
+// one divisor share it (Divisor).
 struct Divisor {
   double y;
   uint64_t mb;    // significand of y, [2^52, 2^53)
   int64_t z;      // ~1/my in Q2.62
+  uint32_t upper; // the same in Q1.31, within 2^-29
   uint32_t eb;    // biased exponent of y
   bool normal;
 };
@@ -218,45 +245,118 @@ __host__ __device__ __forceinline__ Divisor divisor(double y) {
   v.eb = (uint32_t)(b >> 52) & 0x7FFu;
   v.normal = v.eb - 1u < 2046u;
   v.mb = (b & kMant) | kHid;
-  const uint64_t B = v.mb << 10;                           // my in Q2.62, [1, 2)
+  const uint32_t b31 = (uint32_t)(v.mb >> 21);             // my in Q1.31
   const float fb = ffrom((127u << 23) | (uint32_t)((v.mb & kMant) >> 29));
-  int64_t z = (int64_t)q62_from_seed(rcp_seed(fb));
-#pragma unroll
-  for (int it = 0; it < 2; it++) {
-    const int64_t t = ((int64_t)1 << 62) - (int64_t)(mulhi(B, (uint64_t)z) << 2);   // 1 - my*z
-    z += (int64_t)((uint64_t)smulhi(z, t) << 2);
-  }
-  v.z = z;
+  const uint32_t z0 = q31_from_seed(rcp_seed(fb));
+  // two Newton steps z <- z + z*(1 - my*z), the first in 32 bits.  div_by reads
+  // the upper half only; where nothing else does, the second is not compiled.
+  const int32_t d0 = (int32_t)((int64_t)((1ull << 62) - wide(b31, z0)) >> 17);   // Q.45
+  const uint32_t z1 = z0 + (uint32_t)(swide((int32_t)(z0 >> 1), d0) >> 44);       // Q.75 to Q1.31
+  const uint64_t B = v.mb << 11;                           // my in Q1.63
+  const uint64_t t = wide((uint32_t)(B >> 32), z1) + (wide((uint32_t)B, z1) >> 32);   // my*z in Q2.62
+  const int32_t d1 = (int32_t)((int64_t)((1ull << 62) - t) >> 5);                 // Q.57
+  v.z = (int64_t)((uint64_t)z1 << 31) + (swide((int32_t)(z1 >> 1), d1) >> 25);    // Q.87 to Q2.62
+  v.upper = z1;
   return v;
 }
 
-__host__ __device__ __forceinline__ double div_by(double x, const Divisor& v) {
-  const uint64_t a = bits(x);
+// bits of x / v.y; special: the quotient is not one of the integer path's
+__host__ __device__ __forceinline__ uint64_t div_normal(uint64_t a, const Divisor& v, bool& special) {
   const uint32_t ea = (uint32_t)(a >> 52) & 0x7FFu;
-  if (ea - 1u >= 2046u || !v.normal) {
-    if ((a << 1) == 0 && v.normal) return from_bits((a ^ bits(v.y)) & kSign);   // +-0 / normal
-    return hw_div(x, v.y);
-  }
   const uint64_t ma = (a & kMant) | kHid, mb = v.mb;
   const uint32_t k = ma < mb ? 1u : 0u;                    // Q = ma*2^k/mb in [1, 2)
   const int eq = (int)ea - (int)v.eb + 1023 - (int)k;
-  if (eq < 1 || eq > 2046) return hw_div(x, v.y);
-  const uint64_t Aq = (ma << 10) << k;                     // mx*2^k in Q2.62 (below 4)
-  const uint64_t q = mulhi(Aq, (uint64_t)v.z) << 2;        // ~Q in Q2.62
-  uint64_t S = (q + (1u << 9)) >> 10;                      // ~Q * 2^52
+  special = ea - 1u >= 2046u || !v.normal || (uint32_t)(eq - 1) >= 2046u;
+  const uint64_t mx = ma << k;
+  const uint32_t q = (uint32_t)(wide((uint32_t)(mx >> 22), v.upper) >> 31);   // ~Q in Q2.30
+  const int64_t rem = (int64_t)((mx << 30) - mb * q);      // exact, below 2^56
+  const int64_t c = swide((int32_t)(rem >> 26), (int32_t)(v.upper >> 1));
+  uint64_t S = ((uint64_t)q << 22) + (uint64_t)((c + (1ll << 33)) >> 34);   // ~Q * 2^52
   // R = ma*2^(52+k) - S*mb, exact in 64 bits while S is within a few units
-  int64_t R = (int64_t)(((ma << 52) << k) - S * mb);
-  const int64_t hb = (int64_t)mb;
-#pragma unroll
-  for (int it = 0; it < 2; it++) {
-    if (2 * R > hb || (2 * R == hb && (S & 1u))) { R -= hb; S += 1; }
-    else if (2 * R < -hb || (2 * R == -hb && (S & 1u))) { R += hb; S -= 1; }
-  }
-  const uint64_t sg = (a ^ bits(v.y)) & kSign;
-  return from_bits(sg | ((((uint64_t)(eq - 1)) << 52) + S));
+  const int64_t R2 = (int64_t)((mx << 52) - S * mb) * 2, hb = (int64_t)mb;
+  S += (uint64_t)(R2 > hb) - (uint64_t)(R2 < -hb);
+  return ((a ^ bits(v.y)) & kSign) | ((((uint64_t)(eq - 1)) << 52) + S);
+}
+__host__ __device__ __forceinline__ double div_other(double x, const Divisor& v) {
+  const uint64_t a = bits(x);
+  if ((a << 1) == 0 && v.normal) return from_bits((a ^ bits(v.y)) & kSign);   // +-0 / normal
+  return hw_div(x, v.y);
+}
+__host__ __device__ __forceinline__ double div_by(double x, const Divisor& v) {
+  bool special;
+  const uint64_t q = div_normal(bits(x), v, special);
+  if (special) return div_other(x, v);
+  return from_bits(q);
+}
+
+// x^0.2 and x^0.4 (the exponents as the nearest doubles: 0.2 + 2^-54/5 and its
+// double), for positive normal x (+inf gives +inf).  x = M * 2^(5h) with M in
+// [1, 32); z, a single-precision seed of M^(-1/5), is within e = 2^-20, and
+// t = M z^4 is the root times (1 + e)^4.  d = 1 - t z = 1 - (1 + e)^5 gives the root
+// as t (1 - d)^(-4/5), by the binomial series to d^3: the next term is below
+// 2^-72.  The exponent's excess over 1/5 is the factor 1 + (2^-54/5) ln x.  The
+// root is held in 62 bits: the results are within 0.53 and 0.56 ulp.  Two calls
+// of pow keep a warp 11500 cycles (5760 each, measured).
+__host__ __device__ __forceinline__ void fifth_powers(double x, double& x02, double& x04) {
+  const uint64_t u = bits(x), f = u & kMant;
+  const int e = (int)((u >> 52) & 0x7FFu);
+  const int h5 = (e + 2) / 5, r = e + 2 - 5 * h5, h = h5 - 205;   // e - 1023 = 5 h + r
+  const float fm = ffrom((uint32_t)(127 + r) << 23 | (uint32_t)(f >> 29));
+  const float lg = log2_seed(fm);
+  const uint32_t z = q31_from_seed(exp2_seed(-0.2f * lg));       // 24 significant bits
+  const int s2 = r >= 3;                     // z^2 < 2^-s2: room for s2 more bits
+  const uint64_t z2 = wide(z, z) << (1 + s2);                    // z^2 2^s2 in Q1.63, exact
+  const uint64_t z4 = mulhi(z2, z2) << (r - 2 * s2);             // z^4 2^r in Q2.62
+  const uint64_t t = mulhi((f | kHid) << 11, z4) << 1;           // M z^4 in Q2.62
+  const uint64_t tz = (wide((uint32_t)(t >> 32), z) << 1) + (wide((uint32_t)t, z) >> 31);   // Q2.62
+  const int64_t d = (int64_t)((1ull << 62) - tz);                // below 2^-17
+  // s = d * (4/5 + d * (18/25 + d * 84/125)), Q2.62
+  const int32_t d31 = (int32_t)(d >> 15);                        // Q.47
+  const int32_t a = 1546188227 + (int32_t)(swide(d31, 1443109012) >> 47);      // 18/25 + .. in Q.31
+  const uint64_t b = 0x3333333333333333ull + (uint64_t)(swide(d31, a) >> 16);  // 4/5 + .. in Q2.62
+  const int64_t s = (int64_t)((uint64_t)smulhi(d, (int64_t)b) << 2);
+  // (2^-54/5) ln x in units of 2^-62: 256/5 ln 2 log2 x = 35.4891... (5h + lg)
+  const int32_t lx = h * 5 * 9085 + (int32_t)(fbits(lg * 9085.22f + 12582912.0f) - 0x4B400000u);   // 256 times
+  const int64_t corr = s + (lx >> 8);
+  const uint64_t T = t + ((uint64_t)smulhi((int64_t)(t >> 1), corr) << 3);   // root of M in Q2.62 (t may pass 2)
+  const uint64_t T2 = mulhi(T, T);                               // its square in Q4.60
+  // the binades (near a power of two the exponent's excess can cross one)
+  const int k1 = clz64(T) - 1, k2 = clz64(T2) - 3;
+  x02 = from_bits(((uint64_t)(h + 1022 - k1) << 52) + ((T + (1ull << (9 - k1))) >> (10 - k1)));
+  x04 = from_bits(((uint64_t)(2 * h + 1022 - k2) << 52) + ((T2 + (1ull << (7 - k2))) >> (8 - k2)));
+  if (e == 0x7FF) x02 = x04 = x;
 }
 
 __host__ __device__ __forceinline__ double div_rn(double x, double y) { return div_by(x, divisor(y)); }
+
+// Square roots of N operands, and quotients of three by one divisor: the
+// integer chains stand side by side, with one branch behind them for the
+// operands that the integer path leaves out, so that they overlap (the branch
+// of each call by itself keeps the compiler from that).
+template <int N>
+__host__ __device__ __forceinline__ void sqrt_many(const double (&x)[N], double (&r)[N]) {
+  bool special = false;
+#pragma unroll
+  for (int i = 0; i < N; i++) {
+    r[i] = from_bits(sqrt_normal(bits(x[i])));
+    special |= sqrt_special(bits(x[i]));
+  }
+  if (special) {
+#pragma unroll
+    for (int i = 0; i < N; i++)
+      if (sqrt_special(bits(x[i]))) r[i] = sqrt_other(x[i]);
+  }
+}
+__host__ __device__ __forceinline__ void div_three(const double (&x)[3], const Divisor& v, double (&r)[3]) {
+  bool sp[3];
+#pragma unroll
+  for (int i = 0; i < 3; i++) r[i] = from_bits(div_normal(bits(x[i]), v, sp[i]));
+  if (sp[0] || sp[1] || sp[2]) {
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+      if (sp[i]) r[i] = div_other(x[i], v);
+  }
+}
 
 // IEEE comparisons on the integer pipes (false with a NaN; +0 == -0): the
 // bit patterns, with the magnitude bits of negatives flipped, order like the

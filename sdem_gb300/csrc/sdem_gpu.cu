@@ -850,21 +850,12 @@ __global__ void __launch_bounds__(kThreads, SDEM_FORCE_MIN_BLOCKS) k_force(Dev d
       const int tm = tag_type(Vm.w), tq = tag_type(Vq.w);
       const int ta = img ? (m_loc ? tm : tq) : (m_lo ? tm : tq);
       const int tb = img ? (m_loc ? tq : tm) : (m_lo ? tq : tm);
-      {
-        const int2* oe = d.own_c_prev + (size_t)owner * d.Ko;
-        // the first entry is read beside the count (the table always holds Ko
-        // entries per owner; an entry past the count is not used)
-        const int2 e0 = oe[0];
-        const int k = d.own_cnt_prev[owner];
-        if (k > 0 && e0.y == partner) {
-          hist = d.c_hist_prev[e0.x];
-        } else {
-          for (int j = 1; j < k; j++) {
-            const int2 e = oe[j];
-            if (e.y == partner) { hist = d.c_hist_prev[e.x]; break; }
-          }
-        }
-      }
+      // Find_insert: the bucket's count and first entry are read here (the table
+      // always holds Ko entries per owner; an entry past the count is not used),
+      // looked at after the geometry, which does not wait for them
+      const int2* oe = d.own_c_prev + (size_t)owner * d.Ko;
+      const int2 e0 = oe[0];
+      const int k = d.own_cnt_prev[owner];
       P = d.bpp + ((size_t)(tb - 1) * d.nT + (ta - 1)) * SDEM_BP_SIZE;
       // Norm_v = Posj .nv. Posi (real4_nv, Prtcl_TypeDef.f90:268-281) and
       // ovrlp = dr - sqrt(d2sum) (NBSM_FineSearch2/3, Prtcl_NBS_Munjiza.f90:514-522)
@@ -877,6 +868,14 @@ __global__ void __launch_bounds__(kThreads, SDEM_FORCE_MIN_BLOCKS) k_force(Dev d
       rj = Pj.w;
       ovrlp = (ri + rj) - normv;
       Norm_v = fpi::gt(normv, 1.0000E-10) ? sdem::div3(sv, normv) : sdem::mk3(0.0, 0.0, 0.0);
+      if (k > 0 && e0.y == partner) {
+        hist = d.c_hist_prev[e0.x];
+      } else {
+        for (int j = 1; j < k; j++) {
+          const int2 e = oe[j];
+          if (e.y == partner) { hist = d.c_hist_prev[e.x]; break; }
+        }
+      }
     } else {
       // a wall contact: Find_insert on the particle's bucket (key = wall) +
       // ContactForce_PW (Prtcl_CL_and_CF.f90:227-249, 832-856)
@@ -1486,8 +1485,13 @@ __device__ void end_step(const Dev& d, const StepEnd& e) {
   }
 }
 
+// Blocks of the sums and of the update.  128 threads spread a small bed over
+// twice as many SMs as 256 do (60 -> 57 us a step at 50k spheres, 191 -> 188 at 200k, 650 -> 646
+// at 1M); with 64 the order by record count inside a block gets too short (661 at 1M).
+constexpr int kUpdateThreads = 128;
+
 // The update in index order, one thread per particle (coalesced records).
-__global__ void __launch_bounds__(kThreads) k_integrate(Dev d, StepEnd end) {
+__global__ void __launch_bounds__(kUpdateThreads) k_integrate(Dev d, StepEnd end) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p < *d.n) integrate_body(d, p, [&](int f) { return int_src(d, f)[p]; });
   end_step(d, end);
@@ -1591,7 +1595,7 @@ __device__ __forceinline__ void gather_one(const Dev& d, const int s) {
 }
 
 
-// One block takes kThreads consecutive sort positions, i.e. spheres that lie
+// One block takes kUpdateThreads consecutive sort positions, i.e. spheres that lie
 // side by side: the rows are read coalesced, and a contact's 96-byte record,
 // which its two spheres read, comes from DRAM once and from L2 the second
 // time.  Inside the block the spheres are ordered by their number of records
@@ -1602,12 +1606,12 @@ __device__ __forceinline__ void gather_one(const Dev& d, const int s) {
 // that order's kernel (24 us) and its share of the wall kernel; 423 B of DRAM a
 // sphere instead of 773.
 template <bool kUpdate>
-__global__ void __launch_bounds__(kThreads) k_gather(Dev d, StepEnd end) {
+__global__ void __launch_bounds__(kUpdateThreads) k_gather(Dev d, StepEnd end) {
   static_assert(kDegBuckets == 64, "two buckets per lane of one warp");
   __shared__ int bucket[kDegBuckets];
-  __shared__ int order[kThreads];
+  __shared__ int order[kUpdateThreads];
   __shared__ int members;
-  const int s0 = blockIdx.x * kThreads;
+  const int s0 = blockIdx.x * kUpdateThreads;
   const int nloc = *d.n;
   {
     const int s = s0 + threadIdx.x;
@@ -2092,7 +2096,7 @@ Dev make_dev(sdem_h* h) {
   return d;
 }
 
-int grid_for(long long n) { return (int)std::max<long long>(1, (n + kThreads - 1) / kThreads); }
+int grid_for(long long n, int width = kThreads) { return (int)std::max<long long>(1, (n + width - 1) / width); }
 
 constexpr int kUpdateTogether = 131072;   // most search positions whose sums and update share a kernel
 int enqueue_step(sdem_h* h) {
@@ -2204,10 +2208,10 @@ int enqueue_step(sdem_h* h) {
   // 400k 357 / 322, 1M 896 / 695.
   const bool together = na <= kUpdateTogether;
   if (together) {
-    k_gather<true><<<grid_for(na), kThreads, 0, st>>>(d, end);
+    k_gather<true><<<grid_for(na, kUpdateThreads), kUpdateThreads, 0, st>>>(d, end);
   } else {
-    k_gather<false><<<grid_for(na), kThreads, 0, st>>>(d, end);
-    k_integrate<<<grid_for(n), kThreads, 0, st>>>(d, end);
+    k_gather<false><<<grid_for(na, kUpdateThreads), kUpdateThreads, 0, st>>>(d, end);
+    k_integrate<<<grid_for(n, kUpdateThreads), kUpdateThreads, 0, st>>>(d, end);
   }
   mark(PH_DELETE);   // the end of the step is part of the update kernel: these two phases are empty
   mark(PH_END);
