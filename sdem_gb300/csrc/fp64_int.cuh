@@ -67,15 +67,7 @@ __host__ __device__ __forceinline__ int clz64(uint64_t v) {
   return v ? __builtin_clzll(v) : 64;
 #endif
 }
-// the hardware operation, for the rare operands the integer path leaves out
-__host__ __device__ __forceinline__ double hw_mul(double x, double y) {
-#ifdef __CUDA_ARCH__
-  return __dmul_rn(x, y);
-#else
-  return x * y;
-#endif
-}
-
+// the hardware operations, for the rare operands the integer paths leave out
 __host__ __device__ __forceinline__ double hw_sqrt(double x) {
 #ifdef __CUDA_ARCH__
   return __dsqrt_rn(x);
@@ -460,15 +452,18 @@ __host__ __device__ __forceinline__ float to_float_rn(double x) {
   return (float)x;
 }
 
-// x * (-0.5), exact for every x whose half is a normal number or zero: the
-// exponent field drops by one and the sign flips.  Subnormal halves (which
-// round), infinities and NaNs take the hardware multiplication.
+// x * (-0.5): the exponent field drops by one and the sign flips; a subnormal
+// half is the rounded half of the bits (to even), infinities and NaN keep
+// theirs.  No instruction of the FP64 pipe: the hardware multiplication for the
+// rare operands was predicated, not branched over, and kept the pipe all the
+// same (12 a sphere beside the update's 30: k_integrate at 1M spheres, AB2,
+// NEWFIG).
 __host__ __device__ __forceinline__ double mul_neg_half(double x) {
-  const uint64_t u = bits(x);
-  const uint32_t e = (uint32_t)(u >> 52) & 0x7FFu;
-  if (e - 2u < 2045u) return from_bits((u - (1ull << 52)) ^ kSign);
-  if ((u << 1) == 0) return from_bits(u ^ kSign);
-  return hw_mul(x, -0.5);
+  const uint64_t u = bits(x), m = u & ~kSign;
+  const uint32_t e = (uint32_t)(m >> 52);
+  const uint64_t low = (m >> 1) + (m & (m >> 1) & 1ull);   // e < 2: bits are multiples of the least subnormal
+  const uint64_t half = e >= 2047u ? m : (e >= 2u ? m - (1ull << 52) : low);
+  return from_bits(half | ((u ^ kSign) & kSign));
 }
 
 }  // namespace fpi
