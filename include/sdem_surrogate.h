@@ -162,6 +162,21 @@ int sdem_sg_segsum(int nrows, int J, const int* row_off, const int* perm, const 
 int sdem_sg_gather_add(int rows, int J, const int* idx, const float* x, int ldx, const float* y, int ldy,
                        float* out, int ld_out, uint16_t* out_bf, int ld_out_bf, void* stream);
 
+/* The gradient of every sphere's state (rows of 128): out[i] = y[i] + x[i]
+ * (leading dimension ldx), then, one after the other, d[e][0..127] for e in
+ * row_off[i] .. row_off[i+1] and d[src_perm[k]][128..255] for k in src_off[i] ..
+ * src_off[i+1] (d: rows of 256) added to it; out_bf = bf16(out).  The bits of
+ * sdem_sg_gather_add and two sdem_sg_segsum calls.  16-byte aligned. */
+int sdem_sg_sphere_grad(int n, const int* row_off, const int* src_off, const int* src_perm, const float* x, int ldx,
+                        const float* y, const float* d, float* out, uint16_t* out_bf, void* stream);
+
+/* out_bf[e] = bf16(v) with v = y[e] + x[idx[e]] (128 columns; y and out_bf
+ * dense, x with leading dimension ldx), and sum[j] += sum over e of v[j]; partial
+ * holds sdem_sg_colsum_blocks() x 128 floats.  The bits of sdem_sg_gather_add and
+ * sdem_sg_colsum.  16-byte aligned. */
+int sdem_sg_gather_add_sum(int rows, const int* idx, const float* x, int ldx, const float* y, uint16_t* out_bf,
+                           float* sum, float* partial, void* stream);
+
 /* Column sums of x (M x J, fp32): out[j] (+)= sum_i x[i][j], in a fixed
  * order; partial holds sdem_sg_colsum_blocks() x J floats. */
 int sdem_sg_colsum_blocks(void);

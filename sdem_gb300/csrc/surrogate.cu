@@ -699,7 +699,13 @@ __global__ void __launch_bounds__(TC_T, 1) k_gemm_tc(int I, int J, int R, Operan
 // Bound by L2 on the gathered forward form (600k rows, R = 384: 117 us, 5.9 TB/s
 // of L2; k_gemm_tc 328 us) and by HBM on the input gradient (J = 384, fp32 out:
 // 206 us, 5.0 TB/s; k_gemm 1150 us).
-constexpr int RW_M = 128, RW_K = 64, RW_STAGES = 6, RW_LAG = 5, RW_ACC = 4, RW_T = 288;
+// An epilogue that reads a mask or a residual (kReads) has eight warps, two to a
+// row quarter, and requests what it reads before it waits for the products: with
+// four warps that read behind the wait, a residual update of 330k rows took 140 us
+// (85 here; 62 for its bytes), a masked gradient 104 (92).  Without reads the four
+// warps are better (fp32 out, J = 384: 206 against 245 us; the copying warps lose
+// registers to the others).
+constexpr int RW_M = 128, RW_K = 64, RW_STAGES = 6, RW_LAG = 5, RW_ACC = 4, RW_T = 288, RW_T_READS = 416;
 constexpr int RW_SLICE = RW_M * RW_K * 2;              // 16 KB
 constexpr int RW_B_MAX = 98304;                        // bytes of B kept
 constexpr int RW_J_MAX = 384;
@@ -755,8 +761,11 @@ __device__ __forceinline__ uint32_t bf16_pair(float lo, float hi) {
 
 // The epilogue of 32 columns gj0.. of row gi, held by one thread.  `wide`: every
 // pointer and leading dimension allows 32-byte accesses, and all 32 columns exist.
+// kPre (wide only): pre holds the residual (32 floats) where ep.resid is given,
+// else the mask (32 bf16 in its first half), read before the accumulator was ready.
+template <bool kPre>
 __device__ __forceinline__ void epilogue32(const sdem_sg_epilogue& ep, bool wide, const float* __restrict__ bias,
-                                           int gi, int gj0, int J, uint32_t (&r)[32]) {
+                                           int gi, int gj0, int J, uint32_t (&r)[32], const uint32_t (&pre)[32]) {
     if (wide) {
         if (ep.bias) {
 #pragma unroll
@@ -770,7 +779,12 @@ __device__ __forceinline__ void epilogue32(const sdem_sg_epilogue& ep, bool wide
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 uint32_t m[8];
-                ld8(ep.mask + (size_t)gi * ep.ld_mask + gj0 + 16 * h, m);
+                if (!kPre || ep.resid) {
+                    ld8(ep.mask + (size_t)gi * ep.ld_mask + gj0 + 16 * h, m);
+                } else {
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) m[q] = pre[8 * h + q];
+                }
 #pragma unroll
                 for (int q = 0; q < 16; ++q)
                     if (!bf16_positive((uint16_t)(m[q >> 1] >> (16 * (q & 1))))) r[16 * h + q] = 0u;
@@ -806,10 +820,10 @@ __device__ __forceinline__ void epilogue32(const sdem_sg_epilogue& ep, bool wide
 #pragma unroll
             for (int h = 0; h < 4; ++h) {
                 uint32_t a[8];
-                ld8(ep.resid + (size_t)gi * ep.ld_resid + gj0 + 8 * h, a);
+                if (!kPre) ld8(ep.resid + (size_t)gi * ep.ld_resid + gj0 + 8 * h, a);
 #pragma unroll
                 for (int q = 0; q < 8; ++q)
-                    r[8 * h + q] = __float_as_uint(__uint_as_float(a[q]) + __uint_as_float(r[8 * h + q]));
+                    r[8 * h + q] = __float_as_uint(__uint_as_float(kPre ? pre[8 * h + q] : a[q]) + __uint_as_float(r[8 * h + q]));
                 if (ep.res_out) st8(ep.res_out + (size_t)gi * ep.ld_res_out + gj0 + 8 * h, r + 8 * h);
             }
             if (ep.res_out_bf) {
@@ -872,8 +886,9 @@ __device__ __forceinline__ void stage_b(uint8_t* Bs, const Operand& B, int J, in
     }
 }
 
-__global__ void __launch_bounds__(RW_T, 1) k_gemm_rows(int I, int J, int R, Operand A, Operand B, sdem_sg_epilogue ep,
-                                                       int wide) {
+template <bool kReads>
+__global__ void __launch_bounds__(kReads ? RW_T_READS : RW_T, 1) k_gemm_rows(int I, int J, int R, Operand A, Operand B,
+                                                                             sdem_sg_epilogue ep, int wide) {
     extern __shared__ __align__(1024) uint8_t rw_smem[];
     __shared__ __align__(8) uint64_t full[RW_STAGES], empty[RW_STAGES], accf[RW_ACC], acce[RW_ACC];
     __shared__ uint32_t tmem_slot;
@@ -897,11 +912,11 @@ __global__ void __launch_bounds__(RW_T, 1) k_gemm_rows(int I, int J, int R, Oper
         }
         for (int k = 0; k < RW_ACC; ++k) {
             mbar_init(&accf[k], 1);
-            mbar_init(&acce[k], 128);
+            mbar_init(&acce[k], kReads ? 256 : 128);
         }
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
-    for (int j = threadIdx.x; j < RW_J_MAX; j += RW_T) bias_s[j] = ep.bias && j < J ? ep.bias[j] : 0.f;
+    for (int j = threadIdx.x; j < RW_J_MAX; j += blockDim.x) bias_s[j] = ep.bias && j < J ? ep.bias[j] : 0.f;
     stage_b(Bs, B, J, jpad, R, kslices);
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
@@ -1016,24 +1031,47 @@ __global__ void __launch_bounds__(RW_T, 1) k_gemm_rows(int I, int J, int R, Oper
         }
         __syncwarp();
     } else {
-        // ---- epilogue: warp w holds rows 32 w.. of the tile
+        // ---- epilogue: a warp holds rows 32 (w mod 4).. of the tile; kReads: warps 0-3
+        // the first 64 of a block's columns, 9-12 the others
+        constexpr int kChunks = kReads ? 2 : 4;
+        const int quarter = warp & 3, half = warp > 8 ? 64 : 0;
         bool ok = true;
         for (int m = 0; m < mine; ++m) {
-            const int gi = ((int)blockIdx.x + m * (int)gridDim.x) * RW_M + warp * 32 + lane;
+            const int gi = ((int)blockIdx.x + m * (int)gridDim.x) * RW_M + quarter * 32 + lane;
             for (int n = 0; n < nb; ++n) {
                 const int u = m * nb + n, buf = u % RW_ACC;
+                const int cols = min(128, jpad - n * 128);
+                // what the epilogue reads does not wait for the products
+                uint32_t pre[kChunks][32];
+                if (kReads && gi < I) {
+#pragma unroll
+                    for (int c = 0; c < kChunks; ++c) {
+                        const int gj = n * 128 + half + 32 * c;
+                        if (half + 32 * c < cols) {
+                            if (ep.resid) {
+#pragma unroll
+                                for (int h = 0; h < 4; ++h) ld8(ep.resid + (size_t)gi * ep.ld_resid + gj + 8 * h, pre[c] + 8 * h);
+                            } else {
+#pragma unroll
+                                for (int h = 0; h < 2; ++h) ld8(ep.mask + (size_t)gi * ep.ld_mask + gj + 16 * h, pre[c] + 8 * h);
+                            }
+                        }
+                    }
+                }
                 if (ok) ok = mbar_wait(smem_u32(&accf[buf]), (u / RW_ACC) & 1);
                 ok = __all_sync(0xffffffffu, ok);
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                const int cols = min(128, jpad - n * 128);
-                for (int c = 0; c < cols; c += 32) {
+#pragma unroll (kReads ? 2 : 1)
+                for (int c = 0; c < kChunks; ++c) {
+                    const int col = half + 32 * c;
+                    if (col >= cols) continue;
                     uint32_t r[32];
-                    tc_ld32(tmem + ((uint32_t)(warp * 32) << 16) + buf * 128 + c, r);
+                    tc_ld32(tmem + ((uint32_t)(quarter * 32) << 16) + buf * 128 + col, r);
                     if (!ok) {
 #pragma unroll
                         for (int q = 0; q < 32; ++q) r[q] = 0u;
                     }
-                    if (gi < I) epilogue32(ep, wide != 0, bias_s, gi, n * 128 + c, J, r);
+                    if (gi < I) epilogue32<kReads>(ep, wide != 0, bias_s, gi, n * 128 + col, J, r, pre[c]);
                     __syncwarp();   // tcgen05.ld takes whole warps
                 }
                 asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
@@ -1610,15 +1648,31 @@ __global__ void __launch_bounds__(ML_T, 1) k_mlp(Operand A, MlpArgs g) {
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(512) : "memory");
 }
 
-__global__ void k_split_reduce(int I, int J, int splits, const float* __restrict__ partial, float* __restrict__ out,
-                               int ld_out, int accumulate) {
-    const size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t IJ = (size_t)I * J;
-    if (k >= IJ) return;
+// Partial products of a split reduction, added in split order.  A block stages
+// SR_SPLITS splits of 32 outputs in shared memory, all loads in flight, and one
+// warp adds them.  One thread per output left 64 blocks with a thread's 152 loads
+// in rounds of latency (11 us a weight gradient of the network's edges, 7 here).
+constexpr int SR_SPLITS = 160;
+__global__ void __launch_bounds__(256) k_split_reduce(int I, int J, int splits, const float* __restrict__ partial,
+                                                      float* __restrict__ out, int ld_out, int accumulate) {
+    __shared__ float tile[SR_SPLITS][32];
+    const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
+    const size_t IJ = (size_t)I * J, k = (size_t)blockIdx.x * 32 + lane;
     float s = 0.f;
-    // many loads in flight, added in split order
+    for (int z0 = 0; z0 < splits; z0 += SR_SPLITS) {
+        const int m = min(SR_SPLITS, splits - z0);
+        __syncthreads();
+        if (k < IJ) {
+#pragma unroll 20
+            for (int z = g; z < m; z += 8) tile[z][lane] = partial[(z0 + z) * IJ + k];
+        }
+        __syncthreads();
+        if (g == 0) {
 #pragma unroll 32
-    for (int z = 0; z < splits; ++z) s += partial[z * IJ + k];
+            for (int z = 0; z < m; ++z) s += tile[z][lane];
+        }
+    }
+    if (g > 0 || k >= IJ) return;
     const int i = (int)(k / J), j = (int)(k % J);
     float* o = out + (size_t)i * ld_out + j;
     *o = accumulate ? *o + s : s;
@@ -1643,6 +1697,45 @@ __global__ void k_segsum(int nrows, int J, const int* __restrict__ row_off, cons
         if (out) out[(size_t)row * ld_out + j] = s;
         if (out_bf) out_bf[(size_t)row * ld_out_bf + j] = bf16_bits(s);
     }
+}
+
+// The gradient of h of every sphere (rows of 128): out[i] = y[i] + x[i], then the
+// rows off0[i] .. of d (columns 0..127) and the rows perm1[off1[i]] .. (columns
+// 128..255) added in list order, and its bf16 copy: the additions of
+// sdem_sg_gather_add and two sdem_sg_segsum calls, in their order.
+// Bound by HBM (d, 1 KB an edge, once).  k_segsum keeps one row in flight a warp;
+// here eight: 330k edges of 16k spheres 73 us (4.6 TB/s) instead of 108 in three kernels.
+__global__ void __launch_bounds__(256) k_sphere_grad(int n, const int* __restrict__ off0, const int* __restrict__ off1,
+                                                     const int* __restrict__ perm1, const float* __restrict__ x, int ldx,
+                                                     const float* __restrict__ y, const float* __restrict__ d,
+                                                     float* __restrict__ out, uint16_t* __restrict__ out_bf) {
+    const int i = (int)(((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (i >= n) return;
+    const float4 a = *reinterpret_cast<const float4*>(x + (size_t)i * ldx + lane * 4);
+    const float4 u = *reinterpret_cast<const float4*>(y + (size_t)i * 128 + lane * 4);
+    float4 s = make_float4(u.x + a.x, u.y + a.y, u.z + a.z, u.w + a.w);
+#pragma unroll
+    for (int side = 0; side < 2; ++side) {
+        const int* __restrict__ off = side ? off1 : off0;
+        const int e0 = off[i], e1 = off[i + 1];
+        const float* __restrict__ dc = d + side * 128 + lane * 4;
+        for (int b = e0; b < e1; b += 32) {
+            const int mine = b + lane < e1 ? (side ? perm1[b + lane] : b + lane) : 0, m = min(32, e1 - b);
+            for (int k = 0; k < m; k += 8) {
+                float4 v[8];
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    const int row = __shfl_sync(0xffffffffu, mine, (k + q) & 31);
+                    if (k + q < m) v[q] = __ldcs(reinterpret_cast<const float4*>(dc + (size_t)row * 256));
+                }
+#pragma unroll
+                for (int q = 0; q < 8; ++q)
+                    if (k + q < m) s = make_float4(s.x + v[q].x, s.y + v[q].y, s.z + v[q].z, s.w + v[q].w);
+            }
+        }
+    }
+    *reinterpret_cast<float4*>(out + (size_t)i * 128 + lane * 4) = s;
+    *reinterpret_cast<uint2*>(out_bf + (size_t)i * 128 + lane * 4) = make_uint2(bf16_pair(s.x, s.y), bf16_pair(s.z, s.w));
 }
 
 // rows of whole float4s, eight columns a thread (k_gather_add: one; 337k rows of
@@ -1737,6 +1830,75 @@ __global__ void __launch_bounds__(256) k_colsum_part128(int M, const float* __re
         }
     }
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    if (threadIdx.x < 128) partial[(size_t)blockIdx.x * 128 + threadIdx.x] = s;
+}
+
+// out_bf[e] = bf16(v), v = y[e] + x[idx[e]] (rows of 128), and the column sums of v
+// in k_colsum_part128's chunks and order, so that v is neither written nor read
+// back for the bias gradient.  A block takes tiles of 64 rows of its chunk: the
+// next tile's rows are on their way while this one's go to shared memory, where
+// 128 threads add them.  Bound by HBM (768 B a row).  330k rows: 55 us (4.6 TB/s)
+// instead of 67 and 36 in two kernels; with the gather's indices loaded beside the
+// rows they point to, 83.
+constexpr int GS_ROWS = 64, GS_T = 512;
+constexpr int GS_SMEM = 2 * GS_ROWS * 128 * 4;
+__global__ void __launch_bounds__(GS_T) k_gather_add_sum(int M, const int* __restrict__ idx, const float* __restrict__ x,
+                                                         int ldx, const float* __restrict__ y, uint16_t* __restrict__ out_bf,
+                                                         float* __restrict__ partial) {
+    extern __shared__ __align__(16) float gs_tile[];   // two of GS_ROWS x 128
+    const int chunk = (M + kColsumBlocks - 1) / kColsumBlocks;
+    const int r0 = blockIdx.x * chunk, r1 = min(M, r0 + chunk);
+    const int tiles = r1 > r0 ? (r1 - r0 + GS_ROWS - 1) / GS_ROWS : 0;
+    // 32 consecutive threads take a row, four columns each; four rows a thread, 16 apart
+    const int j = (threadIdx.x & 31) * 4, g = threadIdx.x >> 5;
+    constexpr int kPer = GS_ROWS / (GS_T / 32);
+    float4 a[kPer], u[kPer];
+    int ids[kPer];   // of the tile after the one in a and u
+    auto load_ids = [&](int t) {
+#pragma unroll
+        for (int q = 0; q < kPer; ++q) {
+            const int e = r0 + t * GS_ROWS + q * (GS_T / 32) + g;
+            ids[q] = e < r1 ? __ldg(idx + e) : 0;
+        }
+    };
+    auto load = [&](int t) {
+#pragma unroll
+        for (int q = 0; q < kPer; ++q) {
+            const int e = r0 + t * GS_ROWS + q * (GS_T / 32) + g;
+            if (e < r1) {
+                u[q] = __ldcs(reinterpret_cast<const float4*>(y + (size_t)e * 128 + j));
+                a[q] = *reinterpret_cast<const float4*>(x + (size_t)ids[q] * ldx + j);
+            }
+        }
+        load_ids(t + 1);
+    };
+    load_ids(0);
+    load(0);
+    float s = 0.f;
+    for (int t = 0; t < tiles; ++t) {
+        float* tile = gs_tile + (t & 1) * GS_ROWS * 128;
+#pragma unroll
+        for (int q = 0; q < kPer; ++q) {
+            const int r = q * (GS_T / 32) + g, e = r0 + t * GS_ROWS + r;
+            if (e < r1) {
+                const float4 v = make_float4(u[q].x + a[q].x, u[q].y + a[q].y, u[q].z + a[q].z, u[q].w + a[q].w);
+                *reinterpret_cast<float4*>(tile + r * 128 + j) = v;
+                *reinterpret_cast<uint2*>(out_bf + (size_t)e * 128 + j) = make_uint2(bf16_pair(v.x, v.y), bf16_pair(v.z, v.w));
+            }
+        }
+        load(t + 1);
+        __syncthreads();   // the tile is whole; the other one is read no more
+        if (threadIdx.x < 128) {
+            const float* v = tile + threadIdx.x;
+            const int rows = min(GS_ROWS, r1 - r0 - t * GS_ROWS);
+            if (rows == GS_ROWS) {
+#pragma unroll
+                for (int r = 0; r < GS_ROWS; ++r) s += v[r * 128];
+            } else {
+                for (int r = 0; r < rows; ++r) s += v[r * 128];
+            }
+        }
+    }
     if (threadIdx.x < 128) partial[(size_t)blockIdx.x * 128 + threadIdx.x] = s;
 }
 
@@ -1993,7 +2155,6 @@ int sdem_sg_gemm(int I, int J, int R, const sdem_sg_operand* a, const sdem_sg_op
         // B fits in shared memory (with more than one block of columns a tile's
         // slices stay until the last block, so that two tiles must fit the ring)
         const size_t smem = bbytes + RW_STAGES * RW_SLICE;
-        if (!set_smem((const void*)k_gemm_rows, RW_B_MAX + RW_STAGES * RW_SLICE)) return SDEM_SG_E_CUDA;
         const bool wide = J % 32 == 0 && (!ep->out || (aligned32(ep->out) && ep->ld_out % 8 == 0)) &&
                           (!ep->out_bf || (aligned32(ep->out_bf) && ep->ld_out_bf % 16 == 0)) &&
                           (!ep->mask || (aligned32(ep->mask) && ep->ld_mask % 16 == 0)) &&
@@ -2001,7 +2162,10 @@ int sdem_sg_gemm(int I, int J, int R, const sdem_sg_operand* a, const sdem_sg_op
                           (!ep->res_out || (aligned32(ep->res_out) && ep->ld_res_out % 8 == 0)) &&
                           (!ep->res_out_bf || (aligned32(ep->res_out_bf) && ep->ld_res_out_bf % 16 == 0));
         const int tiles = (I + RW_M - 1) / RW_M;
-        k_gemm_rows<<<std::min(tiles, sm_count()), RW_T, smem, st(stream)>>>(I, J, R, A, B, *ep, wide ? 1 : 0);
+        const bool reads = wide && (ep->resid || ep->mask);
+        const auto kernel = reads ? k_gemm_rows<true> : k_gemm_rows<false>;
+        if (!set_smem((const void*)kernel, RW_B_MAX + RW_STAGES * RW_SLICE)) return SDEM_SG_E_CUDA;
+        kernel<<<std::min(tiles, sm_count()), reads ? RW_T_READS : RW_T, smem, st(stream)>>>(I, J, R, A, B, *ep, wide ? 1 : 0);
         return launched();
     }
     if (nsplit == 1 && g_tc_enabled && !A.trans && !B.trans) {
@@ -2019,7 +2183,7 @@ int sdem_sg_gemm(int I, int J, int R, const sdem_sg_operand* a, const sdem_sg_op
                                                            nsplit > 1 ? partial : nullptr);
         if (nsplit == 1) return launched();
         if (cudaGetLastError() != cudaSuccess) return SDEM_SG_E_CUDA;
-        k_split_reduce<<<blocks((long long)I * J, 256), 256, 0, st(stream)>>>(I, J, nsplit, partial, ep->out, ep->ld_out,
+        k_split_reduce<<<blocks((long long)I * J, 32), 256, 0, st(stream)>>>(I, J, nsplit, partial, ep->out, ep->ld_out,
                                                                            ep->accumulate);
         return launched();
     }
@@ -2030,7 +2194,7 @@ int sdem_sg_gemm(int I, int J, int R, const sdem_sg_operand* a, const sdem_sg_op
     if (!partial || !ep->out || ep->bias || ep->relu || ep->mask || ep->out_bf || ep->resid) return SDEM_SG_E_ARG;
     k_gemm<<<grid, GT, 0, st(stream)>>>(I, J, R, A, B, *ep, (int)rchunk, partial);
     if (cudaGetLastError() != cudaSuccess) return SDEM_SG_E_CUDA;
-    k_split_reduce<<<blocks((long long)I * J, 256), 256, 0, st(stream)>>>(I, J, nsplit, partial, ep->out, ep->ld_out,
+    k_split_reduce<<<blocks((long long)I * J, 32), 256, 0, st(stream)>>>(I, J, nsplit, partial, ep->out, ep->ld_out,
                                                                        ep->accumulate);
     return launched();
 }
@@ -2108,6 +2272,31 @@ int sdem_sg_gather_add(int rows, int J, const int* idx, const float* x, int ldx,
     }
     k_gather_add<<<blocks((long long)rows * J, 256), 256, 0, st(stream)>>>(rows, J, idx, x, ldx, y, ldy, out, ld_out,
                                                                           out_bf, ld_out_bf);
+    return launched();
+}
+
+int sdem_sg_sphere_grad(int n, const int* row_off, const int* src_off, const int* src_perm, const float* x, int ldx,
+                        const float* y, const float* d, float* out, uint16_t* out_bf, void* stream) {
+    if (n < 0 || ldx < 128 || ldx % 4) return SDEM_SG_E_ARG;
+    if (n == 0) return SDEM_SG_OK;
+    // (without edges there is no src_perm)
+    if (!row_off || !src_off || !x || !y || !d || !out || !out_bf || !aligned16(x) || !aligned16(y) ||
+        !aligned16(d) || !aligned16(out) || !aligned16(out_bf))
+        return SDEM_SG_E_ARG;
+    k_sphere_grad<<<blocks((long long)n * 32, 256), 256, 0, st(stream)>>>(n, row_off, src_off, src_perm, x, ldx, y, d, out,
+                                                                         out_bf);
+    return launched();
+}
+
+int sdem_sg_gather_add_sum(int rows, const int* idx, const float* x, int ldx, const float* y, uint16_t* out_bf, float* sum,
+                           float* partial, void* stream) {
+    if (rows < 0 || ldx < 128 || ldx % 4) return SDEM_SG_E_ARG;
+    if (!sum || !partial || (rows > 0 && (!idx || !x || !y || !out_bf || !aligned16(x) || !aligned16(y) || !aligned16(out_bf))))
+        return SDEM_SG_E_ARG;
+    if (!set_smem((const void*)k_gather_add_sum, GS_SMEM)) return SDEM_SG_E_CUDA;
+    k_gather_add_sum<<<kColsumBlocks, GS_T, GS_SMEM, st(stream)>>>(rows, idx, x, ldx, y, out_bf, partial);
+    if (cudaGetLastError() != cudaSuccess) return SDEM_SG_E_CUDA;
+    k_colsum_final<<<1, 128, 0, st(stream)>>>(128, partial, sum, 1);
     return launched();
 }
 

@@ -55,7 +55,8 @@ OVERLAP_GAIN = 100.0
 EXPORTED = ("sdem_sg_cells", "sdem_sg_edge_count", "sdem_sg_edge_fill", "sdem_sg_node_features", "sdem_sg_gemm",
             "sdem_sg_segsum", "sdem_sg_gather_add", "sdem_sg_colsum_blocks", "sdem_sg_colsum", "sdem_sg_mse",
             "sdem_sg_adam", "sdem_sg_to_bf16", "sdem_sg_advance", "sdem_sg_set_tensor_path",
-            "sdem_sg_tensor_timeouts", "sdem_sg_mlp", "sdem_sg_graph_work", "sdem_sg_graph_count", "sdem_sg_graph_fill")
+            "sdem_sg_tensor_timeouts", "sdem_sg_mlp", "sdem_sg_graph_work", "sdem_sg_graph_count", "sdem_sg_graph_fill",
+            "sdem_sg_sphere_grad", "sdem_sg_gather_add_sum")
 
 
 class SgGrid(C.Structure):
@@ -102,6 +103,8 @@ def load(path: str = LIB_PATH):
         "sdem_sg_gemm": [I, I, I, C.POINTER(SgOperand), C.POINTER(SgOperand), C.POINTER(SgEpilogue), I, P, P],
         "sdem_sg_segsum": [I, I, P, P, P, I, P, I, I, P, I, P],
         "sdem_sg_gather_add": [I, I, P, P, I, P, I, P, I, P, I, P],
+        "sdem_sg_sphere_grad": [I, P, P, P, P, I, P, P, P, P, P],
+        "sdem_sg_gather_add_sum": [I, P, P, I, P, P, P, P, P],
         "sdem_sg_colsum_blocks": [],
         "sdem_sg_colsum": [I, I, P, I, P, I, P, P],
         "sdem_sg_mse": [I, I, P, I, P, P, P, P, P],
@@ -411,6 +414,8 @@ class Network:
         self.fused = latent == LATENT and torch.device(device).type == "cuda"
         self.colsum_partial = torch.empty(self.lib.sdem_sg_colsum_blocks() * 4 * latent, dtype=torch.float32,
                                           device=device)
+        # ... and the gathers and sums of the backward pass
+        self.wide_rows = latent == LATENT and torch.device(device).type == "cuda"
         self.refresh_bf16()
         self.saved = None
 
@@ -598,7 +603,7 @@ class Network:
         din_n = torch.empty((n, 2 * L), dtype=f32, device=dev)
         din_e = torch.empty((max(E, 1), 2 * L), dtype=f32, device=dev)
         deb = torch.empty((max(E, 1), L), dtype=bf, device=dev)
-        dm = torch.empty((max(E, 1), L), dtype=f32, device=dev)
+        dm = None if self.wide_rows else torch.empty((max(E, 1), L), dtype=f32, device=dev)
         dmb = torch.empty((max(E, 1), L), dtype=bf, device=dev)
         dze = torch.empty((max(E, 1), L), dtype=f32, device=dev)
         dzeb = torch.empty((max(E, 1), L), dtype=bf, device=dev)
@@ -614,20 +619,22 @@ class Network:
                         _Op(1, (hb_prev, 0, L, L, None), (aggb, 0, L, L, None)))
             self._bgrad(f"node{l}.b1", n, dz, L)
             self._dgrad(n, _Op(0, (dzb, 0, L, L, None)), f"node{l}.w1", out=din_n, ld_out=2 * L)
-            dh_prev = torch.empty_like(dh)
-            _check(lib.sdem_sg_gather_add(n, L, None, _ptr(din_n), 2 * L, _ptr(dh), L, _ptr(dh_prev), L, None, L,
-                                          _stream()), "sdem_sg_gather_add")
             # messages: dm = de_l + dagg[dst]
-            _check(lib.sdem_sg_gather_add(E, L, _ptr(g.dst), _ptr(din_n, L), 2 * L, _ptr(de), L, _ptr(dm), L,
-                                          _ptr(dmb), L, _stream()), "sdem_sg_gather_add")
+            if self.wide_rows:
+                _check(lib.sdem_sg_gather_add_sum(E, _ptr(g.dst), _ptr(din_n, L), 2 * L, _ptr(de), _ptr(dmb),
+                                                  _ptr(self.grad, self.off(f"edge{l}.b2")), _ptr(self.colsum_partial),
+                                                  _stream()), "sdem_sg_gather_add_sum")
+            else:
+                _check(lib.sdem_sg_gather_add(E, L, _ptr(g.dst), _ptr(din_n, L), 2 * L, _ptr(de), L, _ptr(dm), L,
+                                              _ptr(dmb), L, _stream()), "sdem_sg_gather_add")
+                self._bgrad(f"edge{l}.b2", E, dm, L)
             # edge MLP: m = W2 relu(W1 [h_dst, h_src, e] + b1) + b2
             self._wgrad(f"edge{l}.w2", E, _Op(1, (dmb, 0, L, L, None)), _Op(1, (ze, 0, L, L, None)))
-            self._bgrad(f"edge{l}.b2", E, dm, L)
             self._dgrad(E, _Op(0, (dmb, 0, L, L, None)), f"edge{l}.w2", mask=ze, ld_mask=L, out=dze, ld_out=L,
                         out_bf=dzeb, ld_out_bf=L)
+            self._bgrad(f"edge{l}.b1", E, dze, L)
             self._wgrad(f"edge{l}.w1", E, _Op(1, (dzeb, 0, L, L, None)),
                         _Op(1, (hb_prev, 0, L, L, g.dst), (hb_prev, 0, L, L, g.src), (eb_prev, 0, L, L, None)))
-            self._bgrad(f"edge{l}.b1", E, dze, L)
             # the input gradient by columns of W1: [h_dst, h_src] for the sums
             # below, e straight onto its residual stream (in place)
             w1 = self.off(f"edge{l}.w1")
@@ -636,10 +643,18 @@ class Network:
             self._gemm(E, L, L, dz_op, _Op(1, (self.pb, w1 + 2 * L, 3 * L, L, None)),
                        _ep(resid=de, ld_resid=L, res_out=de, ld_res_out=L, res_out_bf=deb if l == 0 else None,
                            ld_res_out_bf=L))
-            _check(lib.sdem_sg_segsum(n, L, _ptr(g.row_off), None, _ptr(din_e), 2 * L, _ptr(dh_prev), L, 1, None, L,
-                                      _stream()), "sdem_sg_segsum")
-            _check(lib.sdem_sg_segsum(n, L, _ptr(g.src_off), _ptr(g.src_perm), _ptr(din_e, L), 2 * L, _ptr(dh_prev),
-                                      L, 1, _ptr(dhb), L, _stream()), "sdem_sg_segsum")
+            dh_prev = torch.empty_like(dh)
+            if self.wide_rows:
+                _check(lib.sdem_sg_sphere_grad(n, _ptr(g.row_off), _ptr(g.src_off), _ptr(g.src_perm), _ptr(din_n), 2 * L,
+                                               _ptr(dh), _ptr(din_e), _ptr(dh_prev), _ptr(dhb), _stream()),
+                       "sdem_sg_sphere_grad")
+            else:
+                _check(lib.sdem_sg_gather_add(n, L, None, _ptr(din_n), 2 * L, _ptr(dh), L, _ptr(dh_prev), L, None, L,
+                                              _stream()), "sdem_sg_gather_add")
+                _check(lib.sdem_sg_segsum(n, L, _ptr(g.row_off), None, _ptr(din_e), 2 * L, _ptr(dh_prev), L, 1, None, L,
+                                          _stream()), "sdem_sg_segsum")
+                _check(lib.sdem_sg_segsum(n, L, _ptr(g.src_off), _ptr(g.src_perm), _ptr(din_e, L), 2 * L,
+                                          _ptr(dh_prev), L, 1, _ptr(dhb), L, _stream()), "sdem_sg_segsum")
             dh = dh_prev
         # encoders
         self._wgrad("enc_n.w2", n, _Op(1, (dhb, 0, L, L, None)), _Op(1, (s["zb_enc"], 0, L, L, None)))
