@@ -1255,18 +1255,20 @@ __global__ void __launch_bounds__(WG_T, 1) k_gemm_wgrad(int I, int J, int R, Ope
 // and walks it in tiles of 128 rows.  Warps 12-15 copy A (ring of slices as in
 // k_gemm_rows), one thread of warp 16 issues the products -- the first layer of
 // tile m+1 before the second of tile m -- warps 4-7 make z in two halves of 64
-// columns, each handed over and given back by itself, warps 0-3 finish v, and
-// warps 8-11 read v from tensor memory once more and sum it.  The sums run
-// over the rows of a receiver one after another in row order (as k_segsum's),
-// from a 16-column strip in shared memory; the receiver that a tile leaves open
-// carries its sums to the next tile.  All results are the bits of the
-// separate kernels.
-// 974k edges of 50k receivers: 473 us for an edge block (511 with z), 250 us for
-// the products and a bf16 result alone, 264 with the sums alone: the roles share
-// the SM and none has slack enough to hide the others (HBM would take 230 us).
-// The forward pass of 50k spheres went from 5.84 ms of separate kernels to 3.27.
-constexpr int ML_T = 544, ML_LAG = 3, ML_MAX_STAGES = 6, ML_STRIP = 16;
-constexpr int ML_STRIP_LD = ML_STRIP + 1, ML_STRIP_BYTES = 128 * ML_STRIP_LD * 4;
+// columns, each handed over and given back by itself, warps 8-11 put v into
+// strips of 32 columns in shared memory and sum the rows of each receiver there,
+// one after another in row order (as k_segsum's), and warps 0-3 store the strips
+// with their residuals.  The receiver that a tile leaves open carries its sums to
+// the next tile.  All results are the bits of the separate kernels.
+// The strips turn v by rows into whole lines: with a thread per row, storing 32
+// bytes of 32 rows at a time, the storing warps were the slowest role (an edge
+// block of 974k edges 473 us, 402 without sums; 373 and 354 here, 230 for its HBM
+// bytes).  What remains at R = 384 is the ring of three slices that fits beside
+// the weights (291 us for a bf16 result alone, 158 at R = 128) and the sums (266 us
+// alone).
+// The forward pass of 50k spheres went from 5.84 ms of separate kernels to 2.67.
+constexpr int ML_T = 544, ML_LAG = 3, ML_MAX_STAGES = 6, ML_STRIP = 32;
+constexpr int ML_STRIP_BYTES = 128 * ML_STRIP * 4;   // 16-byte chunk q of a row at q xor (row mod 8)
 constexpr int ML_SMEM_MAX = 232448 - 3072;   // dynamic part beside the static arrays (below 3 KB)
 
 struct MlpArgs {
@@ -1298,6 +1300,16 @@ __device__ __forceinline__ int lower_bound32(const int* __restrict__ off, int n,
 }
 
 __device__ __forceinline__ void bar_sums() { asm volatile("bar.sync 1, 128;\n" ::: "memory"); }
+// the strip between its writers (warps 8-11) and the warps that store v (0-3): each
+// side arrives where it has nothing to wait for
+__device__ __forceinline__ void bar_strip_full(bool writer) {
+    if (writer) asm volatile("bar.arrive 2, 256;\n" ::: "memory");
+    else asm volatile("bar.sync 2, 256;\n" ::: "memory");
+}
+__device__ __forceinline__ void bar_strip_free(bool writer) {
+    if (writer) asm volatile("bar.sync 3, 256;\n" ::: "memory");
+    else asm volatile("bar.arrive 3, 256;\n" ::: "memory");
+}
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p)); }
 
 __global__ void __launch_bounds__(ML_T, 1) k_mlp(Operand A, MlpArgs g) {
@@ -1311,6 +1323,8 @@ __global__ void __launch_bounds__(ML_T, 1) k_mlp(Operand A, MlpArgs g) {
     const int kslices = (g.R + RW_K - 1) / RW_K, jpad = (g.J + 15) / 16 * 16;
     const uint32_t W1 = smem_u32(ml_smem), W2 = W1 + kslices * 16384, Z = W2 + 2 * jpad * 128, ring = Z + 32768;
     float* strip = reinterpret_cast<float*>(ml_smem + kslices * 16384 + 2 * jpad * 128 + 32768 + g.stages * RW_SLICE);
+    const bool stored = g.out || g.out_bf;              // v goes to HBM
+    const int strips = g.J > ML_STRIP ? g.J / ML_STRIP : 1;   // a tile's
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&tmem_slot)),
@@ -1327,7 +1341,7 @@ __global__ void __launch_bounds__(ML_T, 1) k_mlp(Operand A, MlpArgs g) {
             mbar_init(&a1f[k], 1);
             mbar_init(&a1e[k], 128);
             mbar_init(&a2f[k], 1);
-            mbar_init(&a2e[k], g.agg ? 256 : 128);
+            mbar_init(&a2e[k], 128);
             mbar_init(&zf[k], 128);
             mbar_init(&ze[k], 1);
         }
@@ -1469,84 +1483,100 @@ __global__ void __launch_bounds__(ML_T, 1) k_mlp(Operand A, MlpArgs g) {
         }
         __syncwarp();
     } else if (warp >= 8) {
-        // ---- sums: warp w holds rows 32 (w mod 4).. of the tile
+        // ---- strips and sums: warp w holds rows 32 (w mod 4).. of the tile
         const int w4 = warp & 3, row = w4 * 32 + lane;
         // receivers of this tile and the next, requested two tiles ahead
         int d0 = lo + row < hi && g.agg ? __ldg(g.dst + lo + row) : -1;
         int d1 = lo + 128 + row < hi && g.agg ? __ldg(g.dst + lo + 128 + row) : -1;
-        for (int m = 0; g.agg && m < mine; ++m) {
+        for (int m = 0; m < mine; ++m) {
             const int b = m & 1, e0 = lo + m * 128, gi = e0 + row, rows = min(128, hi - e0);
-            const int before = s_dst[127];   // the tile before's last receiver
-            const int mydst = d0;
-            d0 = d1;
-            bar_sums();
-            s_dst[row] = mydst;
-            if (row == 0) s_after = d0;
-            d1 = gi + 256 < hi ? __ldg(g.dst + gi + 256) : -1;
-            int prev = __shfl_up_sync(0xffffffffu, mydst, 1);
-            bar_sums();
-            if (lane == 0 && row > 0) prev = s_dst[row - 1];
-            const bool head = gi < hi && (row == 0 || mydst != prev);
-            const unsigned hb = __ballot_sync(0xffffffffu, head);
-            if (lane == 0) s_head[w4] = hb;
-            bar_sums();
-            int rank = __popc(hb & ((1u << lane) - 1u)), nseg = 0;
-            for (int w = 0; w < 4; ++w) {
-                if (w < w4) rank += __popc(s_head[w]);
-                nseg += __popc(s_head[w]);
+            int nseg = 0;
+            bool open_first = false, open_last = false;
+            if (g.agg) {
+                const int before = s_dst[127];   // the tile before's last receiver
+                const int mydst = d0;
+                d0 = d1;
+                bar_sums();
+                s_dst[row] = mydst;
+                if (row == 0) s_after = d0;
+                d1 = gi + 256 < hi ? __ldg(g.dst + gi + 256) : -1;
+                int prev = __shfl_up_sync(0xffffffffu, mydst, 1);
+                bar_sums();
+                if (lane == 0 && row > 0) prev = s_dst[row - 1];
+                const bool head = gi < hi && (row == 0 || mydst != prev);
+                const unsigned hb = __ballot_sync(0xffffffffu, head);
+                if (lane == 0) s_head[w4] = hb;
+                bar_sums();
+                int rank = __popc(hb & ((1u << lane) - 1u));
+                for (int w = 0; w < 4; ++w) {
+                    if (w < w4) rank += __popc(s_head[w]);
+                    nseg += __popc(s_head[w]);
+                }
+                if (head) s_seg[rank] = (uint8_t)row;
+                if (row == 0) s_seg[nseg] = (uint8_t)rows;   // (the barrier before the first strip is read orders s_seg)
+                // the first receiver goes on from the tile before, the last into the next
+                open_first = m > 0 && s_dst[0] == before;
+                open_last = rows == 128 && e0 + 128 < hi && s_after == s_dst[127];
             }
-            if (head) s_seg[rank] = (uint8_t)row;
-            if (row == 0) s_seg[nseg] = (uint8_t)rows;   // (the barrier before the first strip is read orders s_seg)
-            // the first receiver goes on from the tile before, the last into the next
-            const bool open_first = m > 0 && s_dst[0] == before;
-            const bool open_last = rows == 128 && e0 + 128 < hi && s_after == s_dst[127];
             if (ok) ok = mbar_wait(smem_u32(&a2f[b]), (m >> 1) & 1);
             ok = __all_sync(0xffffffffu, ok);
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
 #pragma unroll 1
-            for (int c = 0; c < 128; c += 32) {
+            for (int p = 0; p < strips; ++p) {
+                const int c = p * ML_STRIP;
                 uint32_t r[32];
                 tc_ld32(tmem + 256 + ((uint32_t)(w4 * 32) << 16) + b * 128 + c, r);
-#pragma unroll
-                for (int half = 0; half < 2; ++half) {
-                    float bias[ML_STRIP];
-#pragma unroll
-                    for (int q = 0; q < ML_STRIP / 4; ++q)
-                        reinterpret_cast<float4*>(bias)[q] = *reinterpret_cast<const float4*>(&b2s[c + half * ML_STRIP + 4 * q]);
-#pragma unroll
-                    for (int q = 0; q < ML_STRIP; ++q)
-                        strip[row * ML_STRIP_LD + q] = ok ? __uint_as_float(r[half * ML_STRIP + q]) + bias[q] : 0.f;
-                    bar_sums();
-                    // half a warp per receiver, a lane per column
-                    const int col = lane & 15, j = c + half * ML_STRIP + col;
-                    for (int k = w4 * 2 + (lane >> 4); k < nseg; k += 8) {
-                        const int r0 = s_seg[k];
-                        int left = s_seg[k + 1] - r0;
-                        const float* x = strip + r0 * ML_STRIP_LD + col;
-                        float sum = k == 0 && open_first ? carry[b][j] : 0.f;
-                        for (; left >= 8; left -= 8, x += 8 * ML_STRIP_LD) {
-                            float v[8];
-#pragma unroll
-                            for (int i = 0; i < 8; ++i) v[i] = x[i * ML_STRIP_LD];
-#pragma unroll
-                            for (int i = 0; i < 8; ++i) sum += v[i];
-                        }
-                        if (left > 0) {   // past the end +0, which leaves the sum (never -0) as it is
-                            float v[7];
-#pragma unroll
-                            for (int i = 0; i < 7; ++i) v[i] = i < left ? x[i * ML_STRIP_LD] : 0.f;
-#pragma unroll
-                            for (int i = 0; i < 7; ++i) sum += v[i];
-                        }
-                        if (k == nseg - 1 && open_last) carry[b ^ 1][j] = sum;
-                        else g.agg[(size_t)s_dst[r0] * 128 + j] = bf16_bits(sum);
-                    }
-                    __syncwarp();   // tcgen05.ld and the barrier take whole warps
-                    bar_sums();
+                // the strip before has been read
+                if (m > 0 || p > 0) {
+                    if (stored) bar_strip_free(true);
+                    else bar_sums();
                 }
+#pragma unroll
+                for (int q = 0; q < ML_STRIP / 4; ++q) {
+                    const float4 bias = *reinterpret_cast<const float4*>(&b2s[c + 4 * q]);
+                    float4 v = make_float4(__uint_as_float(r[4 * q]) + bias.x, __uint_as_float(r[4 * q + 1]) + bias.y,
+                                           __uint_as_float(r[4 * q + 2]) + bias.z, __uint_as_float(r[4 * q + 3]) + bias.w);
+                    if (!ok) v = make_float4(0.f, 0.f, 0.f, 0.f);
+                    *reinterpret_cast<float4*>(strip + row * ML_STRIP + ((q ^ (row & 7)) << 2)) = v;
+                }
+                if (p == strips - 1) {
+                    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+                    mbar_arrive(&a2e[b]);
+                }
+                if (stored) bar_strip_full(true);
+                if (!g.agg) continue;
+                bar_sums();
+                // a warp per receiver, a lane per column
+                const int j = c + lane;
+                for (int k = w4; k < nseg; k += 4) {
+                    const int r0 = s_seg[k];
+                    int left = s_seg[k + 1] - r0;
+                    const int to = s_dst[r0];
+                    float sum = k == 0 && open_first ? carry[b][j] : 0.f;
+                    // where this column lies in eight rows on end; eight rows further it is the same
+                    const float* x[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) x[i] = strip + (r0 + i) * ML_STRIP + (lane ^ (((r0 + i) & 7) << 2));
+                    int at = 0;
+                    for (; left >= 8; left -= 8, at += 8 * ML_STRIP) {
+                        float v[8];
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) v[i] = x[i][at];
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) sum += v[i];
+                    }
+                    if (left > 0) {   // past the end +0, which leaves the sum (never -0) as it is
+                        float v[7];
+#pragma unroll
+                        for (int i = 0; i < 7; ++i) v[i] = i < left ? x[i][at] : 0.f;
+#pragma unroll
+                        for (int i = 0; i < 7; ++i) sum += v[i];
+                    }
+                    if (k == nseg - 1 && open_last) carry[b ^ 1][j] = sum;
+                    else g.agg[(size_t)to * 128 + j] = bf16_bits(sum);
+                }
+                __syncwarp();   // tcgen05.ld and the barrier take whole warps
             }
-            asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-            mbar_arrive(&a2e[b]);
         }
     } else if (warp >= 4) {
         // ---- z: warp w holds rows 32 (w mod 4).. of the tile
@@ -1588,57 +1618,57 @@ __global__ void __launch_bounds__(ML_T, 1) k_mlp(Operand A, MlpArgs g) {
             }
         }
     } else {
-        // ---- v: warp w holds rows 32 w.. of the tile
-        const int row = warp * 32 + lane, J = g.J;
-        float res[32];   // the residual of the columns to come
-        auto load_res = [&](int gi, int c) {
-            if (g.resid && gi < hi) {
+        // ---- v: warp w stores rows 32 w.. of the tile from the strips, eight lanes a
+        // row (whole lines), four columns a lane
+        const int q = lane & 7, J = g.J, total = stored ? mine * strips : 0;
+        // row of this lane's k-th four columns of strip P, and its place in v
+        auto gi_of = [&](int P, int k) { return lo + P / strips * 128 + warp * 32 + 4 * k + (lane >> 3); };
+        auto col_of = [&](int P) { return P % strips * ML_STRIP + 4 * q; };
+        float4 r[8];   // residual of the strip to come
+        auto load_res = [&](int P) {
+            if (!g.resid || P >= total) return;
 #pragma unroll
-                for (int h = 0; h < 4; ++h) ld8(g.resid + (size_t)gi * 128 + c + 8 * h, reinterpret_cast<uint32_t*>(res) + 8 * h);
-            }
+            for (int k = 0; k < 8; ++k)
+                if (gi_of(P, k) < hi) r[k] = __ldcs(reinterpret_cast<const float4*>(g.resid + (size_t)gi_of(P, k) * 128 + col_of(P)));
         };
-        load_res(lo + row, 0);
-        for (int m = 0; m < mine; ++m) {
-            const int b = m & 1, gi = lo + m * 128 + row;
-            if (g.resid && gi + 128 < hi) {
+        auto finish = [&](int P) {
+            __syncwarp();   // the barriers take whole warps
+            bar_strip_full(false);
+            float4 v[8];
 #pragma unroll
-                for (int h = 0; h < 4; ++h) prefetch_l2(g.resid + (size_t)(gi + 128) * 128 + 32 * h);
+            for (int k = 0; k < 8; ++k) {
+                const int row = warp * 32 + 4 * k + (lane >> 3);
+                v[k] = *reinterpret_cast<const float4*>(strip + row * ML_STRIP + ((q ^ (row & 7)) << 2));
             }
-            if (ok) ok = mbar_wait(smem_u32(&a2f[b]), (m >> 1) & 1);
-            ok = __all_sync(0xffffffffu, ok);
-            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            if (g.out || g.out_bf) {
-#pragma unroll 1
-                for (int c = 0; c < J; c += 32) {
-                    uint32_t r[32];
-                    tc_ld32(tmem + 256 + ((uint32_t)(warp * 32) << 16) + b * 128 + c, r);
-                    float w[32];
+            __syncwarp();
+            if (P + 1 < total) bar_strip_free(false);
 #pragma unroll
-                    for (int q = 0; q < 32; ++q) {
-                        const float v = ok ? __uint_as_float(r[q]) + b2s[c + q] : 0.f;
-                        w[q] = g.resid ? res[q] + v : v;
-                    }
-                    if (c + 32 < J) load_res(gi, c + 32);
-                    else load_res(gi + 128, 0);
-                    if (gi < hi && g.out) {
+            for (int k = 0; k < 8; ++k)
+                if (g.resid) v[k] = make_float4(r[k].x + v[k].x, r[k].y + v[k].y, r[k].z + v[k].z, r[k].w + v[k].w);
+            load_res(P + 1);
+            if (col_of(P) < J) {
 #pragma unroll
-                        for (int h = 0; h < 4; ++h)
-                            if (c + 8 * h < J) st8(g.out + (size_t)gi * J + c + 8 * h, reinterpret_cast<const uint32_t*>(w) + 8 * h);
-                    }
-                    if (gi < hi && g.out_bf) {
-#pragma unroll
-                        for (int h = 0; h < 2; ++h) {
-                            uint32_t p[8];
-#pragma unroll
-                            for (int q = 0; q < 8; ++q) p[q] = bf16_pair(w[16 * h + 2 * q], w[16 * h + 2 * q + 1]);
-                            if (c + 16 * h < J) st8(g.out_bf + (size_t)gi * J + c + 16 * h, p);
-                        }
-                    }
-                    __syncwarp();   // tcgen05.ld takes whole warps
+                for (int k = 0; k < 8; ++k) {
+                    const int gi = gi_of(P, k);
+                    if (gi >= hi) continue;
+                    if (g.out) *reinterpret_cast<float4*>(g.out + (size_t)gi * J + col_of(P)) = v[k];
+                    if (g.out_bf)
+                        *reinterpret_cast<uint2*>(g.out_bf + (size_t)gi * J + col_of(P)) =
+                            make_uint2(bf16_pair(v[k].x, v[k].y), bf16_pair(v[k].z, v[k].w));
                 }
             }
-            asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-            mbar_arrive(&a2e[b]);
+        };
+        load_res(0);
+#pragma unroll 1
+        for (int P = 0; P < total; ++P) {
+            if (g.resid && P % strips == 0) {   // the next tile's residual on its way to L2
+                const int gi = lo + (P / strips + 1) * 128 + warp * 32 + lane;
+                if (gi < hi) {
+#pragma unroll
+                    for (int h = 0; h < 4; ++h) prefetch_l2(g.resid + (size_t)gi * 128 + 32 * h);
+                }
+            }
+            finish(P);
         }
     }
     if (!ok && lane == 0) atomicAdd(&g_tc_timeouts, 1u);
@@ -2229,7 +2259,7 @@ int sdem_sg_mlp(int M, int R, const sdem_sg_operand* a, const uint16_t* w1, cons
     g.row_off = row_off;
     g.dst = dst;
     g.agg = agg_bf;
-    const int fixed = (R + RW_K - 1) / RW_K * 16384 + 2 * J * 128 + 32768 + (agg_bf ? ML_STRIP_BYTES : 0);
+    const int fixed = (R + RW_K - 1) / RW_K * 16384 + 2 * J * 128 + 32768 + (agg_bf || out || out_bf ? ML_STRIP_BYTES : 0);
     g.stages = std::min((int)ML_MAX_STAGES, (ML_SMEM_MAX - fixed) / RW_SLICE);   // 3 at R = 384
     if (!set_smem((const void*)k_mlp, ML_SMEM_MAX)) return SDEM_SG_E_CUDA;
     k_mlp<<<std::min((M + 127) / 128, sm_count()), ML_T, fixed + g.stages * RW_SLICE, st(stream)>>>(A, g);
