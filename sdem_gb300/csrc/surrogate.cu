@@ -732,6 +732,22 @@ __device__ __forceinline__ void tc_mma(uint32_t d, uint64_t a, uint64_t b, uint3
         "l"(a), "l"(b), "r"(idesc), "r"(acc ? 1u : 0u)
         : "memory");
 }
+// the same with A in tensor memory (K-major, two 16-bit elements a column)
+__device__ __forceinline__ void tc_mma_ta(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, bool acc) {
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d),
+        "r"(a), "l"(b), "r"(idesc), "r"(acc ? 1u : 0u)
+        : "memory");
+}
+// 16 columns of this warp's lane quarter
+__device__ __forceinline__ void tc_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n" ::"r"(taddr),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+        "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
+}
 // 32 accumulator columns of this warp's lane quarter
 __device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t (&r)[32]) {
     asm volatile(
@@ -1245,28 +1261,29 @@ __global__ void __launch_bounds__(WG_T, 1) k_gemm_wgrad(int I, int J, int R, Ope
 // One MLP of the network: z = relu(A W1^T + b1) (128 wide), v = z W2^T + b2, with
 // an optional residual and an optional sum of v over the rows of each receiver
 // (the messages of an edge block).  Both weights stay in shared memory; z goes
-// from tensor memory through registers into shared memory as the second
-// product's operand, and v from registers to its place, so that of the
+// from tensor memory through registers back into tensor memory as the second
+// product's operand, and v through shared memory to its place, so that of the
 // intermediate values only what the caller asks for reaches HBM.  As separate
 // kernels an edge block moved 3 KB of HBM an edge (z twice, the messages twice,
 // the residual stream in two precisions); here it moves 1.5 KB.
 //
 // A CTA owns a contiguous range of rows, cut at receivers when there are sums,
 // and walks it in tiles of 128 rows.  Warps 12-15 copy A (ring of slices as in
-// k_gemm_rows), one thread of warp 16 issues the products -- the first layer of
-// tile m+1 before the second of tile m -- warps 4-7 make z in two halves of 64
-// columns, each handed over and given back by itself, warps 8-11 put v into
+// k_gemm_rows), one thread of warp 16 issues the products -- the second layer of
+// tile m, then the first of tile m+1 -- warps 4-7 make z, warps 8-11 put v into
 // strips of 32 columns in shared memory and sum the rows of each receiver there,
 // one after another in row order (as k_segsum's), and warps 0-3 store the strips
 // with their residuals.  The receiver that a tile leaves open carries its sums to
 // the next tile.  All results are the bits of the separate kernels.
-// The strips turn v by rows into whole lines: with a thread per row, storing 32
-// bytes of 32 rows at a time, the storing warps were the slowest role (an edge
-// block of 974k edges 473 us, 402 without sums; 373 and 354 here, 230 for its HBM
-// bytes).  What remains at R = 384 is the ring of three slices that fits beside
-// the weights (291 us for a bf16 result alone, 158 at R = 128) and the sums (266 us
-// alone).
-// The forward pass of 50k spheres went from 5.84 ms of separate kernels to 2.67.
+// Tensor memory (512 columns): one accumulator of the first layer, two of the
+// second, whose readers are the slower ones, and two of z.
+// Two things bound it, measured on an edge block of 974k edges (326 us, 364 with z
+// kept; its HBM bytes would take 230): the sums (252 us alone) and the copies (242
+// for a bf16 result alone; 158 at R = 128).  A thread per row storing 32 bytes of
+// 32 rows at a time instead of strips, which make whole lines: 473.  z in shared
+// memory, which leaves room for a ring of three slices instead of five: 373.
+// Slices are handed over two behind the copies (3 behind: 346, 1: 355).
+// The forward pass of 50k spheres went from 5.84 ms of separate kernels to 2.42.
 constexpr int ML_T = 544, ML_LAG = 3, ML_MAX_STAGES = 6, ML_STRIP = 32;
 constexpr int ML_STRIP_BYTES = 128 * ML_STRIP * 4;   // 16-byte chunk q of a row at q xor (row mod 8)
 constexpr int ML_SMEM_MAX = 232448 - 3072;   // dynamic part beside the static arrays (below 3 KB)
@@ -1314,15 +1331,15 @@ __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefe
 
 __global__ void __launch_bounds__(ML_T, 1) k_mlp(Operand A, MlpArgs g) {
     extern __shared__ __align__(1024) uint8_t ml_smem[];
-    __shared__ __align__(8) uint64_t full[ML_MAX_STAGES], empty[ML_MAX_STAGES], a1f[2], a1e[2], a2f[2], a2e[2], zf[2], ze[2];
+    __shared__ __align__(8) uint64_t full[ML_MAX_STAGES], empty[ML_MAX_STAGES], a1f, a1e, a2f[2], a2e[2], zf[2], ze[2];
     __shared__ uint32_t tmem_slot;
     __shared__ __align__(16) float b1s[128], b2s[128], carry[2][128];   // carry: sums of the open receiver, by tile parity
     __shared__ int range[2], s_dst[128], s_after;
     __shared__ uint8_t s_seg[132];   // rows where receivers start in the tile
     __shared__ unsigned s_head[4];
     const int kslices = (g.R + RW_K - 1) / RW_K, jpad = (g.J + 15) / 16 * 16;
-    const uint32_t W1 = smem_u32(ml_smem), W2 = W1 + kslices * 16384, Z = W2 + 2 * jpad * 128, ring = Z + 32768;
-    float* strip = reinterpret_cast<float*>(ml_smem + kslices * 16384 + 2 * jpad * 128 + 32768 + g.stages * RW_SLICE);
+    const uint32_t W1 = smem_u32(ml_smem), W2 = W1 + kslices * 16384, ring = W2 + 2 * jpad * 128;
+    float* strip = reinterpret_cast<float*>(ml_smem + kslices * 16384 + 2 * jpad * 128 + g.stages * RW_SLICE);
     const bool stored = g.out || g.out_bf;              // v goes to HBM
     const int strips = g.J > ML_STRIP ? g.J / ML_STRIP : 1;   // a tile's
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1337,9 +1354,9 @@ __global__ void __launch_bounds__(ML_T, 1) k_mlp(Operand A, MlpArgs g) {
             mbar_init(&full[k], 128);
             mbar_init(&empty[k], 1);
         }
+        mbar_init(&a1f, 1);
+        mbar_init(&a1e, 128);
         for (int k = 0; k < 2; ++k) {
-            mbar_init(&a1f[k], 1);
-            mbar_init(&a1e[k], 128);
             mbar_init(&a2f[k], 1);
             mbar_init(&a2e[k], 128);
             mbar_init(&zf[k], 128);
@@ -1448,14 +1465,13 @@ __global__ void __launch_bounds__(ML_T, 1) k_mlp(Operand A, MlpArgs g) {
             const uint32_t id2 = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(jpad >> 3) << 17) | (8u << 24);
             int slot = 0, round = 0;
             auto first = [&](int m) {
-                const int b = m & 1;
-                if (m >= 2 && ok) ok = mbar_wait(smem_u32(&a1e[b]), ((m >> 1) - 1) & 1);
+                if (m >= 1 && ok) ok = mbar_wait(smem_u32(&a1e), (m - 1) & 1);
                 for (int ks = 0; ks < kslices && ok; ++ks) {
                     ok = mbar_wait(smem_u32(&full[slot]), round & 1);
                     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                     const int steps = (min(RW_K, g.R - ks * RW_K) + 15) / 16;
                     for (int k = 0; k < steps; ++k)
-                        tc_mma(tmem + b * 128, umma_desc_sw128(ring + slot * RW_SLICE + k * 32, 16, 1024),
+                        tc_mma(tmem, umma_desc_sw128(ring + slot * RW_SLICE + k * 32, 16, 1024),
                                umma_desc_sw128(W1 + ks * 16384 + k * 32, 16, 1024), id1, ks > 0 || k > 0);
                     tc_commit(&empty[slot]);
                     if (++slot == g.stages) {
@@ -1463,22 +1479,22 @@ __global__ void __launch_bounds__(ML_T, 1) k_mlp(Operand A, MlpArgs g) {
                         ++round;
                     }
                 }
-                if (ok) tc_commit(&a1f[b]);
+                if (ok) tc_commit(&a1f);
             };
             if (mine > 0) first(0);
             for (int m = 0; m < mine && ok; ++m) {
-                if (m + 1 < mine) first(m + 1);
                 const int b = m & 1;
                 if (m >= 2 && ok) ok = mbar_wait(smem_u32(&a2e[b]), ((m >> 1) - 1) & 1);
-                for (int half = 0; half < 2 && ok; ++half) {
-                    ok = mbar_wait(smem_u32(&zf[half]), m & 1);
+                if (ok) ok = mbar_wait(smem_u32(&zf[b]), (m >> 1) & 1);
+                if (ok) {
                     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                    for (int k = 0; k < 4; ++k)
-                        tc_mma(tmem + 256 + b * 128, umma_desc_sw128(Z + half * 16384 + k * 32, 16, 1024),
-                               umma_desc_sw128(W2 + half * jpad * 128 + k * 32, 16, 1024), id2, half > 0 || k > 0);
-                    tc_commit(&ze[half]);
+                    for (int k = 0; k < 8; ++k)
+                        tc_mma_ta(tmem + 128 + b * 128, tmem + 384 + b * 64 + k * 8,
+                                  umma_desc_sw128(W2 + (k >> 2) * jpad * 128 + (k & 3) * 32, 16, 1024), id2, k > 0);
+                    tc_commit(&ze[b]);
                 }
                 if (ok) tc_commit(&a2f[b]);
+                if (m + 1 < mine) first(m + 1);
             }
         }
         __syncwarp();
@@ -1525,7 +1541,7 @@ __global__ void __launch_bounds__(ML_T, 1) k_mlp(Operand A, MlpArgs g) {
             for (int p = 0; p < strips; ++p) {
                 const int c = p * ML_STRIP;
                 uint32_t r[32];
-                tc_ld32(tmem + 256 + ((uint32_t)(w4 * 32) << 16) + b * 128 + c, r);
+                tc_ld32(tmem + 128 + ((uint32_t)(w4 * 32) << 16) + b * 128 + c, r);
                 // the strip before has been read
                 if (m > 0 || p > 0) {
                     if (stored) bar_strip_free(true);
@@ -1581,41 +1597,32 @@ __global__ void __launch_bounds__(ML_T, 1) k_mlp(Operand A, MlpArgs g) {
     } else if (warp >= 4) {
         // ---- z: warp w holds rows 32 (w mod 4).. of the tile
         const int row = (warp & 3) * 32 + lane;
-        uint8_t* zs = ml_smem + kslices * 16384 + 2 * jpad * 128 + row * 128;
+        const uint32_t quarter = (uint32_t)((warp & 3) * 32) << 16;
         for (int m = 0; m < mine; ++m) {
             const int b = m & 1, gi = lo + m * 128 + row;
-            if (ok) ok = mbar_wait(smem_u32(&a1f[b]), (m >> 1) & 1);
+            if (m >= 2 && ok) ok = mbar_wait(smem_u32(&ze[b]), ((m >> 1) - 1) & 1);
+            if (ok) ok = mbar_wait(smem_u32(&a1f), m & 1);
             ok = __all_sync(0xffffffffu, ok);
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
 #pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                if (m >= 1 && ok) ok = mbar_wait(smem_u32(&ze[half]), (m - 1) & 1);
-                ok = __all_sync(0xffffffffu, ok);
+            for (int c = 0; c < 128; c += 32) {
+                uint32_t r[32], h[16];
+                tc_ld32(tmem + quarter + c, r);
 #pragma unroll
-                for (int c = half * 64; c < half * 64 + 64; c += 32) {
-                    uint32_t r[32], h[16];
-                    tc_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + b * 128 + c, r);
-#pragma unroll
-                    for (int q = 0; q < 16; ++q)
-                        h[q] = bf16_pair(fmaxf(__uint_as_float(r[2 * q]) + b1s[c + 2 * q], 0.f),
-                                         fmaxf(__uint_as_float(r[2 * q + 1]) + b1s[c + 2 * q + 1], 0.f));
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const int kc = ((c >> 3) + q) & 7;
-                        *reinterpret_cast<uint4*>(zs + half * 16384 + ((kc ^ (row & 7)) << 4)) =
-                            make_uint4(h[4 * q], h[4 * q + 1], h[4 * q + 2], h[4 * q + 3]);
-                    }
-                    if (g.z && gi < hi) {
-                        st8(g.z + (size_t)gi * 128 + c, h);
-                        st8(g.z + (size_t)gi * 128 + c + 16, h + 8);
-                    }
-                    __syncwarp();
+                for (int q = 0; q < 16; ++q)
+                    h[q] = bf16_pair(fmaxf(__uint_as_float(r[2 * q]) + b1s[c + 2 * q], 0.f),
+                                     fmaxf(__uint_as_float(r[2 * q + 1]) + b1s[c + 2 * q + 1], 0.f));
+                tc_st16(tmem + 384 + quarter + b * 64 + c / 2, h);
+                if (g.z && gi < hi) {
+                    st8(g.z + (size_t)gi * 128 + c, h);
+                    st8(g.z + (size_t)gi * 128 + c + 16, h + 8);
                 }
-                asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-                asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-                if (half == 1) mbar_arrive(&a1e[b]);
-                mbar_arrive(&zf[half]);
+                __syncwarp();
             }
+            asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+            mbar_arrive(&a1e);
+            mbar_arrive(&zf[b]);
         }
     } else {
         // ---- v: warp w stores rows 32 w.. of the tile from the strips, eight lanes a
@@ -2259,8 +2266,8 @@ int sdem_sg_mlp(int M, int R, const sdem_sg_operand* a, const uint16_t* w1, cons
     g.row_off = row_off;
     g.dst = dst;
     g.agg = agg_bf;
-    const int fixed = (R + RW_K - 1) / RW_K * 16384 + 2 * J * 128 + 32768 + (agg_bf || out || out_bf ? ML_STRIP_BYTES : 0);
-    g.stages = std::min((int)ML_MAX_STAGES, (ML_SMEM_MAX - fixed) / RW_SLICE);   // 3 at R = 384
+    const int fixed = (R + RW_K - 1) / RW_K * 16384 + 2 * J * 128 + (agg_bf || out || out_bf ? ML_STRIP_BYTES : 0);
+    g.stages = std::min((int)ML_MAX_STAGES, (ML_SMEM_MAX - fixed) / RW_SLICE);   // 5 at R = 384
     if (!set_smem((const void*)k_mlp, ML_SMEM_MAX)) return SDEM_SG_E_CUDA;
     k_mlp<<<std::min((M + 127) / 128, sm_count()), ML_T, fixed + g.stages * RW_SLICE, st(stream)>>>(A, g);
     return launched();
