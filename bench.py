@@ -45,14 +45,14 @@ METRIC = "particle-steps/s, 1M Hertz spheres"
 UNIT = "particle-steps/s"
 # From the ncu captures in profiles/ (each file gives its command):
 # profiles/kernels_hertz_poly_settled_1m.txt, one step of the settled 1M bed.
-FORCE_DRAM_BYTES_PER_CONTACT = 401.4     # k_force: dram__bytes_read.sum + dram__bytes_write.sum per contact
+FORCE_DRAM_BYTES_PER_CONTACT = 509.6     # k_force: dram__bytes_read.sum + dram__bytes_write.sum per contact
 FP64_INST_PER_SM_CLK = 2.0               # DADD/DMUL/DFMA thread operations per SM per clock (FP64 pipe)
 NUM_SMS = 152
 # Executed DADD + DMUL + DFMA thread instructions of the step's kernels,
 # modelled per particle-particle contact, per sphere and per wall contact.
-FP64_PER_CONTACT = {"k_force": 120.1, "k_gather": 24.2}
-FP64_PER_SPHERE = {"k_integrate": 51.0, "k_bin": 3.0, "k_wall_detect": 0.74}
-FP64_PER_WALL_CONTACT = {"k_wall_force": 123.3, "k_gather": 12.0}
+FP64_PER_CONTACT = {"k_force": 95.0, "k_gather": 18.0}
+FP64_PER_SPHERE = {"k_integrate": 27.0, "k_bin": 3.0, "k_wall_detect": 0.74}
+FP64_PER_WALL_CONTACT = {"k_force": 95.0, "k_gather": 9.0}
 
 # name -> (metric, default particles, base seed)
 WORKLOADS = {
@@ -411,7 +411,8 @@ def our_arm(args):
     traffic = FORCE_DRAM_BYTES_PER_CONTACT * C
     # algorithmic FP64 operations of k_force per Hertz contact (force law + normal
     # vector; the two r*Moment scalings are the gather's): 121 add/sub/mul,
-    # 8 sqrt, 7 divisions, each sqrt/div counted as one operation
+    # 8 sqrt, 7 divisions, each sqrt/div counted as one operation, and fused
+    # multiply-adds (most of the law) as two
     fp64_per_contact = 136
     t_step = ms / K * 1e-3
     step_bytes = n * 352.0 + C * 80.0   # per-step algorithmic bytes of the whole path
@@ -491,9 +492,10 @@ def our_arm(args):
                               "frac": step_bytes / t_step / 1e9 / hbm,
                               "algorithmic_bytes": "352 B per particle + 80 B per contact per step"},
             "phases_ms_per_step": {k: v / nprof for k, v in phases.items()},
-            "phases_note": "separate window of %d steps with events between phases, search/force chunks in one "
-                           "stream; the timed steps overlap each chunk's search with the previous chunk's forces "
-                           "on two streams" % nprof,
+            "phases_note": "separate window of %d steps with events between phases, one chunk on one stream; the "
+                           "timed steps run the wall kernels on a second stream beside the binning and the sort "
+                           "(scan_rows, row_fill, wall_force, delete and step_end are parts of other kernels: "
+                           "their times are the events')" % nprof,
             "dominant_phase": dom,
             "cpu_baseline": cpu,
             "clocks": clocks,
@@ -656,10 +658,12 @@ def surrogate_arm(args):
 
     runner._surrogate_stride(runner.posR, runner.vel, runner.omega)     # warm-up
     phases, E = surrogate_phases(runner, net, sg, torch, reset)
-    # the same forward on the warp-level mma.sync kernel, for comparison
+    # the same forward layer by layer on the warp-level mma.sync kernel, for comparison
+    fused, net.fused = net.fused, False
     assert net.lib.sdem_sg_set_tensor_path(0) == 0
     phases_mma, _ = surrogate_phases(runner, net, sg, torch, reset)
     assert net.lib.sdem_sg_set_tensor_path(1) == 0
+    net.fused = fused
     t_sur = 0.0
     for _ in range(K):
         reset()
