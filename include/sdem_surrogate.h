@@ -17,7 +17,8 @@
  * row-major; bf16 values travel as uint16_t bit patterns.
  *
  * Network arithmetic: BF16 operands, FP32 accumulation on the tensor cores
- * (mma m16n8k16), FP32 bias/ReLU/residual epilogues, FP32 master weights and
+ * (tcgen05 with accumulators in tensor memory, mma m16n8k16 for the remaining
+ * forms; the same bits), FP32 bias/ReLU/residual epilogues, FP32 master weights and
  * Adam state.  Graph construction and features are FP64 (positions) rounded
  * once to FP32 and once to BF16 (round to nearest even).
  */
@@ -143,9 +144,10 @@ int sdem_sg_mlp(int M, int R, const sdem_sg_operand* a, const uint16_t* w1, cons
                 const float* b2, int J, uint16_t* z, const float* resid, float* out, uint16_t* out_bf, int nagg,
                 const int* row_off, const int* dst, uint16_t* agg_bf, void* stream);
 
-/* Which tensor-core kernel sdem_sg_gemm uses for the forms without
- * transposed operands or split reductions: 1 (default) the tcgen05/TMEM
- * kernel, 0 the warp-level mma.sync kernel (kept for the other forms). */
+/* Which tensor-core kernels sdem_sg_gemm uses: 1 (default) the tcgen05 ones
+ * where one takes the form (second operand within 96 KB; no transposed operand;
+ * both transposed), 0 the warp-level mma.sync kernel for every form.  The
+ * results are the same bits.  sdem_sg_mlp is always tcgen05. */
 int sdem_sg_set_tensor_path(int use_tcgen05);
 /* Number of tcgen05 GEMM blocks whose bounded mbarrier wait expired (0
  * expected; such a block writes zeros instead of its products). */

@@ -1088,7 +1088,7 @@ __device__ __forceinline__ void integrate_body(const Dev& d, const int p, const 
 
   // Comm_For_Exchange, y pencil, one rank (Prtcl_Comm.f90:1569-1840): a periodic
   // direction wraps the position (passes y, +x, -x, +z, -z); the others delete
-  // what left [min, max), in the delete passes (k_finish).
+  // what left [min, max), in the delete passes (end_step).
   if (d.per[0] || d.per[1] || d.per[2]) {
     dbl4 Q = sdem::d4(x, Pp.w);
     if (d.per[1]) {

@@ -1,9 +1,11 @@
 // Learned surrogate of the particle step (include/sdem_surrogate.h), sm_103a.
 //
 // Kernels:
-//   k_cells / k_edges<count|fill>   cell-grid neighbour graph at radius
+//   k_graph_bin, scan, k_graph_scatter, k_graph_order, k_graph_count,
+//   k_graph_fill                    cell-grid neighbour graph at radius
 //                                   1.5 d_max, CSR by receiver, deterministic
 //                                   order (neighbour cell, then sphere index);
+//   k_cells / k_edges<count|fill>   the same step by step;
 //   k_node_feat                     node features (velocity frames, spin,
 //                                   size, plane distances) as bf16;
 //   k_mlp                           both layers of one MLP of the forward pass, with
@@ -19,6 +21,8 @@
 //   k_split_reduce, k_colsum*       deterministic reductions (split-K weight
 //                                   gradients, bias gradients);
 //   k_segsum, k_gather_add          message aggregation and its adjoints;
+//   k_sphere_grad, k_gather_add_sum
+//                                   the same fused for rows of 128;
 //   k_mse, k_adam, k_to_bf16,
 //   k_advance                       loss, optimiser, casts, one stride.
 //
