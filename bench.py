@@ -696,7 +696,7 @@ def surrogate_arm(args):
             "forward_tensor": {"flop": surrogate_forward_flop(case.particles.n, E),
                                "achieved_tflops": surrogate_forward_flop(case.particles.n, E) / phases["forward"] / 1e9,
                                "peak_tflops": measured_bf16_tflops(), "peak_note": "bf16 dense, burst, of measured",
-                               "gemm": "tcgen05 (k_gemm_tc) for the forward layers",
+                               "gemm": "tcgen05 (k_mlp: both layers of an MLP in one kernel)",
                                "mma_sync_forward_ms": phases_mma["forward"],
                                "mma_sync_achieved_tflops": surrogate_forward_flop(case.particles.n, E)
                                / phases_mma["forward"] / 1e9},

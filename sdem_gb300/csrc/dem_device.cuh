@@ -48,7 +48,7 @@ __device__ __forceinline__ r3 scale3(r3 p, double v) { return mk3(p.x * v, p.y *
 __device__ __forceinline__ r3 div3(r3 p, double v) {
   const double x[3] = {p.x, p.y, p.z};
   double q[3];
-  fpi::div_three(x, fpi::divisor(v), q);   // one reciprocal refinement for three quotients
+  fpi::div_many(x, fpi::divisor(v), q);   // one reciprocal refinement for three quotients
   return mk3(q[0], q[1], q[2]);
 }
 __device__ __forceinline__ double dot3(r3 a, r3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }

@@ -321,7 +321,7 @@ __host__ __device__ __forceinline__ void fifth_powers(double x, double& x02, dou
 
 __host__ __device__ __forceinline__ double div_rn(double x, double y) { return div_by(x, divisor(y)); }
 
-// Square roots of N operands, and quotients of three by one divisor: the
+// Square roots of N operands, and quotients of N by one divisor: the
 // integer chains stand side by side, with one branch behind them for the
 // operands that the integer path leaves out, so that they overlap (the branch
 // of each call by itself keeps the compiler from that).
@@ -339,13 +339,17 @@ __host__ __device__ __forceinline__ void sqrt_many(const double (&x)[N], double 
       if (sqrt_special(bits(x[i]))) r[i] = sqrt_other(x[i]);
   }
 }
-__host__ __device__ __forceinline__ void div_three(const double (&x)[3], const Divisor& v, double (&r)[3]) {
-  bool sp[3];
+template <int N>
+__host__ __device__ __forceinline__ void div_many(const double (&x)[N], const Divisor& v, double (&r)[N]) {
+  bool sp[N], special = false;
 #pragma unroll
-  for (int i = 0; i < 3; i++) r[i] = from_bits(div_normal(bits(x[i]), v, sp[i]));
-  if (sp[0] || sp[1] || sp[2]) {
+  for (int i = 0; i < N; i++) {
+    r[i] = from_bits(div_normal(bits(x[i]), v, sp[i]));
+    special |= sp[i];
+  }
+  if (special) {
 #pragma unroll
-    for (int i = 0; i < 3; i++)
+    for (int i = 0; i < N; i++)
       if (sp[i]) r[i] = div_other(x[i], v);
   }
 }

@@ -290,28 +290,66 @@ __device__ __forceinline__ void graph_edge(const sdem_sg_grid& g, const GridDiv&
     const double d = fpi::sqrt_rn(ex * ex + ey * ey + ez * ez);
     dst[e] = i;
     src[e] = w.sorted[t];
-    auto h = [&](double v) { return (uint32_t)bf16_bits(fpi::to_float_rn(fpi::div_by(v, dv.scale))); };
+    auto h = [&](double q) { return (uint32_t)bf16_bits(fpi::to_float_rn(q)); };
+    const double v[4] = {ex, ey, ez, d};
+    double q[4];
+    fpi::div_many(v, dv.scale, q);
     // 100 max(r_i + r_j - d, 0) / scale: the difference of unequal doubles is not 0
     const double reach = A.r + B.r;
-    const uint32_t ov = fpi::gt(reach, d) ? h(100.0 * (reach - d)) : 0u;
+    const uint32_t ov = fpi::gt(reach, d) ? h(fpi::div_by(100.0 * (reach - d), dv.scale)) : 0u;
     uint4* o = reinterpret_cast<uint4*>(efeat + e * 16);
-    o[0] = make_uint4(h(ex) | h(ey) << 16, h(ez) | h(d) << 16, ov, 0u);
+    o[0] = make_uint4(h(q[0]) | h(q[1]) << 16, h(q[2]) | h(q[3]) << 16, ov, 0u);
     o[1] = make_uint4(0u, 0u, 0u, 0u);
 }
 
+// A block writes the edges of 64 spheres, a thread an edge, so that no lane idles
+// while the FP64 pipe works (with eight lanes a sphere a quarter did): a graph of
+// 200k spheres and 3.9M edges takes 314 us instead of 335.
+constexpr int GF_S = 64;
 __global__ void __launch_bounds__(GR_T) k_graph_fill(int n, sdem_sg_grid g, GridDiv dv, float margin, GraphWork w,
                                                      const int* __restrict__ row_off, int* __restrict__ dst,
                                                      int* __restrict__ src, uint16_t* __restrict__ efeat) {
-    const int s = (blockIdx.x * GR_T + threadIdx.x) >> 3, sub = threadIdx.x & 7;
-    if (s >= n) return;
-    const int i = w.sorted[s], base = row_off[i], cnt = row_off[i + 1] - base;
-    const Rec4 A = w.pos[s];
-    const int* list = w.nbr + (size_t)s * GR_CAP;
-    for (int k = sub; k < min(cnt, GR_CAP); k += 8) graph_edge(g, dv, w, A, i, list[k], (size_t)base + k, dst, src, efeat);
-    if (cnt > GR_CAP && sub == 0) {
+    __shared__ int start[GF_S + 1], base[GF_S], who[GF_S];
+    __shared__ Rec4 at[GF_S];
+    const int s0 = blockIdx.x * GF_S, t = threadIdx.x, lane = t & 31;
+    static_assert(GF_S == 64, "two spheres per lane of one warp");
+    if (t < 32) {   // the spheres' places in the block's edges
+        int c[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int j = 2 * lane + h, s = s0 + j;
+            c[h] = 0;
+            if (s < n) {
+                const int i = w.sorted[s];
+                who[j] = i;
+                base[j] = row_off[i];
+                at[j] = w.pos[s];
+                c[h] = min(row_off[i + 1] - base[j], GR_CAP);
+            }
+        }
+        int incl = c[0] + c[1];
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        start[2 * lane] = incl - c[0] - c[1];
+        start[2 * lane + 1] = incl - c[1];
+        if (lane == 31) start[GF_S] = incl;
+    }
+    __syncthreads();
+    for (int e = t; e < start[GF_S]; e += GR_T) {
+        int j = 0;   // the last sphere that starts at or before e
+#pragma unroll
+        for (int o = GF_S / 2; o > 0; o >>= 1)
+            if (start[j + o] <= e) j += o;
+        const int k = e - start[j];
+        graph_edge(g, dv, w, at[j], who[j], w.nbr[(size_t)(s0 + j) * GR_CAP + k], (size_t)base[j] + k, dst, src, efeat);
+    }
+    const int s = s0 + t;
+    if (t < GF_S && s < n && row_off[who[t] + 1] - base[t] > GR_CAP) {   // a longer list is searched again
         int k = 0;
-        graph_neighbours(s, g, w, margin, [&](int t) {
-            if (k >= GR_CAP) graph_edge(g, dv, w, A, i, t, (size_t)base + k, dst, src, efeat);
+        graph_neighbours(s, g, w, margin, [&](int q) {
+            if (k >= GR_CAP) graph_edge(g, dv, w, at[t], who[t], q, (size_t)base[t] + k, dst, src, efeat);
             ++k;
         });
     }
@@ -2157,7 +2195,7 @@ int sdem_sg_graph_fill(int n, const double* posR, const sdem_sg_grid* g, void* w
     if (!graph_args(n, posR, g, work, &dv, &margin) || !row_off || !dst || !src || !efeat || !aligned16(efeat))
         return SDEM_SG_E_ARG;
     const GraphWork w = graph_work(work, n, (long long)g->dim[0] * g->dim[1] * g->dim[2]);
-    k_graph_fill<<<blocks(8ll * n, GR_T), GR_T, 0, st(stream)>>>(n, *g, dv, margin, w, row_off, dst, src, efeat);
+    k_graph_fill<<<blocks(n, GF_S), GR_T, 0, st(stream)>>>(n, *g, dv, margin, w, row_off, dst, src, efeat);
     return launched();
 }
 

@@ -3,7 +3,7 @@
 // and with seeds moved by up to +-8 ulp (more than the device's approximations
 // are off).  The root is held to 2^-58 of its value, its square to 2^-57: half an
 // ulp of rounding, 2^-5 and 2^-4 of one more.
-// fpi::sqrt_many and fpi::div_three against the host, special operands among
+// fpi::sqrt_many and fpi::div_many against the host, special operands among
 // the others.
 #include <cmath>
 #include <cstdio>
@@ -60,7 +60,7 @@ int main() {
     const double x[4] = {pick(), pick(), pick(), pick()}, y = pick(), q3[3] = {x[0], x[1], x[2]};
     double r[4], q[3];
     fpi::sqrt_many(x, r);
-    fpi::div_three(q3, fpi::divisor(y), q);
+    fpi::div_many(q3, fpi::divisor(y), q);
     for (int k = 0; k < 4; k++) bad += !same(r[k], std::sqrt(x[k]));
     for (int k = 0; k < 3; k++) bad += !same(q[k], q3[k] / y);
   }
