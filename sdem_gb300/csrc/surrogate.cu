@@ -1727,7 +1727,7 @@ __global__ void __launch_bounds__(ML_T, 1) k_mlp(Operand A, MlpArgs g) {
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(512) : "memory");
 }
 
-// Partial products of a split reduction, added in split order.  A block stages
+// Partial products of a split reduction (or column sums by chunk), added in order.  A block stages
 // SR_SPLITS splits of 32 outputs in shared memory, all loads in flight, and one
 // warp adds them.  One thread per output left 64 blocks with a thread's 152 loads
 // in rounds of latency (11 us a weight gradient of the network's edges, 7 here).
@@ -1869,24 +1869,26 @@ __global__ void k_colsum_part(int M, int J, const float* __restrict__ x, int ldx
     }
 }
 
-// The same chunks and order of additions for rows of 128 floats: the rows of a
-// chunk come through shared memory, three tiles of 32 rows in flight (cp.async),
-// where one thread per column left one load in flight at a time (148 us for
-// 337k rows, 41 here).
-constexpr int CS_ROWS = 32, CS_STAGES = 4;
+// The same chunks and order of additions for rows of 128 floats: a block takes
+// half the columns of a chunk, whose rows come through shared memory, three tiles
+// of 64 in flight (cp.async), where one thread per column left one load in flight
+// at a time (330k rows: 148 us; 36 with whole rows a block, 29 here).
+constexpr int CS_ROWS = 64, CS_COLS = 64, CS_STAGES = 4;
 __global__ void __launch_bounds__(256) k_colsum_part128(int M, const float* __restrict__ x, int ldx,
                                                         float* __restrict__ partial) {
-    extern __shared__ __align__(16) float cs_tile[];   // CS_STAGES x CS_ROWS x 128
+    extern __shared__ __align__(16) float cs_tile[];   // CS_STAGES x CS_ROWS x CS_COLS
     const int chunk = (M + kColsumBlocks - 1) / kColsumBlocks;
     const int r0 = blockIdx.x * chunk, r1 = min(M, r0 + chunk);
     const int tiles = r1 > r0 ? (r1 - r0 + CS_ROWS - 1) / CS_ROWS : 0;
+    constexpr int kLanes = CS_COLS / 4;
+    x += blockIdx.y * CS_COLS;
     auto copy = [&](int t) {
         if (t < tiles) {
-            const uint32_t dst = smem_u32(cs_tile + (t % CS_STAGES) * CS_ROWS * 128);
+            const uint32_t dst = smem_u32(cs_tile + (t % CS_STAGES) * CS_ROWS * CS_COLS);
 #pragma unroll
-            for (int q = 0; q < CS_ROWS * 32 / 256; ++q) {
-                const int c = threadIdx.x + q * 256, r = r0 + t * CS_ROWS + (c >> 5);
-                cp16(dst + c * 16, r < r1 ? x + (size_t)r * ldx + (c & 31) * 4 : x, r < r1 ? 16u : 0u);
+            for (int q = 0; q < CS_ROWS * kLanes / 256; ++q) {
+                const int c = threadIdx.x + q * 256, r = r0 + t * CS_ROWS + c / kLanes;
+                cp16(dst + c * 16, r < r1 ? x + (size_t)r * ldx + (c & (kLanes - 1)) * 4 : x, r < r1 ? 16u : 0u);
             }
         }
         asm volatile("cp.async.commit_group;\n" ::: "memory");
@@ -1897,53 +1899,53 @@ __global__ void __launch_bounds__(256) k_colsum_part128(int M, const float* __re
         asm volatile("cp.async.wait_group %0;\n" ::"n"(CS_STAGES - 2) : "memory");
         __syncthreads();
         copy(t + CS_STAGES - 1);   // into the tile read in the last round
-        if (threadIdx.x < 128) {
-            const float* v = cs_tile + (t % CS_STAGES) * CS_ROWS * 128 + threadIdx.x;
+        if (threadIdx.x < CS_COLS) {
+            const float* v = cs_tile + (t % CS_STAGES) * CS_ROWS * CS_COLS + threadIdx.x;
             const int rows = min(CS_ROWS, r1 - r0 - t * CS_ROWS);
             if (rows == CS_ROWS) {
 #pragma unroll
-                for (int r = 0; r < CS_ROWS; ++r) s += v[r * 128];
+                for (int r = 0; r < CS_ROWS; ++r) s += v[r * CS_COLS];
             } else {
-                for (int r = 0; r < rows; ++r) s += v[r * 128];
+                for (int r = 0; r < rows; ++r) s += v[r * CS_COLS];
             }
         }
     }
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    if (threadIdx.x < 128) partial[(size_t)blockIdx.x * 128 + threadIdx.x] = s;
+    if (threadIdx.x < CS_COLS) partial[(size_t)blockIdx.x * 128 + blockIdx.y * CS_COLS + threadIdx.x] = s;
 }
 
 // out_bf[e] = bf16(v), v = y[e] + x[idx[e]] (rows of 128), and the column sums of v
 // in k_colsum_part128's chunks and order, so that v is neither written nor read
-// back for the bias gradient.  A block takes tiles of 64 rows of its chunk: the
+// back for the bias gradient.  A block takes tiles of 64 half rows of its chunk: the
 // next tile's rows are on their way while this one's go to shared memory, where
-// 128 threads add them.  Bound by HBM (768 B a row).  330k rows: 55 us (4.6 TB/s)
-// instead of 67 and 36 in two kernels; with the gather's indices loaded beside the
-// rows they point to, 83.
-constexpr int GS_ROWS = 64, GS_T = 512;
-constexpr int GS_SMEM = 2 * GS_ROWS * 128 * 4;
+// 64 threads add them.  Bound by HBM (768 B a row).  330k rows: 45 us (5.6 TB/s; 55
+// with all columns in one block) instead of 67 and 36 in two kernels; with the
+// gather's indices loaded beside the rows they point to, 83.
+constexpr int GS_ROWS = 64, GS_COLS = 64, GS_T = 512;
+constexpr int GS_SMEM = 2 * GS_ROWS * GS_COLS * 4;
 __global__ void __launch_bounds__(GS_T) k_gather_add_sum(int M, const int* __restrict__ idx, const float* __restrict__ x,
                                                          int ldx, const float* __restrict__ y, uint16_t* __restrict__ out_bf,
                                                          float* __restrict__ partial) {
-    extern __shared__ __align__(16) float gs_tile[];   // two of GS_ROWS x 128
+    extern __shared__ __align__(16) float gs_tile[];   // two of GS_ROWS x GS_COLS
     const int chunk = (M + kColsumBlocks - 1) / kColsumBlocks;
     const int r0 = blockIdx.x * chunk, r1 = min(M, r0 + chunk);
     const int tiles = r1 > r0 ? (r1 - r0 + GS_ROWS - 1) / GS_ROWS : 0;
-    // 32 consecutive threads take a row, four columns each; four rows a thread, 16 apart
-    const int j = (threadIdx.x & 31) * 4, g = threadIdx.x >> 5;
-    constexpr int kPer = GS_ROWS / (GS_T / 32);
+    // 16 consecutive threads take half a row, four columns each; two rows a thread
+    constexpr int kLanes = GS_COLS / 4, kRows = GS_T / kLanes, kPer = GS_ROWS / kRows;
+    const int jt = (threadIdx.x & (kLanes - 1)) * 4, j = blockIdx.y * GS_COLS + jt, g = threadIdx.x / kLanes;
     float4 a[kPer], u[kPer];
     int ids[kPer];   // of the tile after the one in a and u
     auto load_ids = [&](int t) {
 #pragma unroll
         for (int q = 0; q < kPer; ++q) {
-            const int e = r0 + t * GS_ROWS + q * (GS_T / 32) + g;
+            const int e = r0 + t * GS_ROWS + q * kRows + g;
             ids[q] = e < r1 ? __ldg(idx + e) : 0;
         }
     };
     auto load = [&](int t) {
 #pragma unroll
         for (int q = 0; q < kPer; ++q) {
-            const int e = r0 + t * GS_ROWS + q * (GS_T / 32) + g;
+            const int e = r0 + t * GS_ROWS + q * kRows + g;
             if (e < r1) {
                 u[q] = __ldcs(reinterpret_cast<const float4*>(y + (size_t)e * 128 + j));
                 a[q] = *reinterpret_cast<const float4*>(x + (size_t)ids[q] * ldx + j);
@@ -1955,39 +1957,30 @@ __global__ void __launch_bounds__(GS_T) k_gather_add_sum(int M, const int* __res
     load(0);
     float s = 0.f;
     for (int t = 0; t < tiles; ++t) {
-        float* tile = gs_tile + (t & 1) * GS_ROWS * 128;
+        float* tile = gs_tile + (t & 1) * GS_ROWS * GS_COLS;
 #pragma unroll
         for (int q = 0; q < kPer; ++q) {
-            const int r = q * (GS_T / 32) + g, e = r0 + t * GS_ROWS + r;
+            const int r = q * kRows + g, e = r0 + t * GS_ROWS + r;
             if (e < r1) {
                 const float4 v = make_float4(u[q].x + a[q].x, u[q].y + a[q].y, u[q].z + a[q].z, u[q].w + a[q].w);
-                *reinterpret_cast<float4*>(tile + r * 128 + j) = v;
+                *reinterpret_cast<float4*>(tile + r * GS_COLS + jt) = v;
                 *reinterpret_cast<uint2*>(out_bf + (size_t)e * 128 + j) = make_uint2(bf16_pair(v.x, v.y), bf16_pair(v.z, v.w));
             }
         }
         load(t + 1);
         __syncthreads();   // the tile is whole; the other one is read no more
-        if (threadIdx.x < 128) {
+        if (threadIdx.x < GS_COLS) {
             const float* v = tile + threadIdx.x;
             const int rows = min(GS_ROWS, r1 - r0 - t * GS_ROWS);
             if (rows == GS_ROWS) {
 #pragma unroll
-                for (int r = 0; r < GS_ROWS; ++r) s += v[r * 128];
+                for (int r = 0; r < GS_ROWS; ++r) s += v[r * GS_COLS];
             } else {
-                for (int r = 0; r < rows; ++r) s += v[r * 128];
+                for (int r = 0; r < rows; ++r) s += v[r * GS_COLS];
             }
         }
     }
-    if (threadIdx.x < 128) partial[(size_t)blockIdx.x * 128 + threadIdx.x] = s;
-}
-
-__global__ void k_colsum_final(int J, const float* __restrict__ partial, float* __restrict__ out, int accumulate) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= J) return;
-    float s = 0.f;
-#pragma unroll 32
-    for (int b = 0; b < kColsumBlocks; ++b) s += partial[(size_t)b * J + j];
-    out[j] = accumulate ? out[j] + s : s;
+    if (threadIdx.x < GS_COLS) partial[(size_t)blockIdx.x * 128 + blockIdx.y * GS_COLS + threadIdx.x] = s;
 }
 
 __global__ void k_mse(int n, int K, const float* __restrict__ pred, int ldp, const float* __restrict__ target,
@@ -2373,9 +2366,9 @@ int sdem_sg_gather_add_sum(int rows, const int* idx, const float* x, int ldx, co
     if (!sum || !partial || (rows > 0 && (!idx || !x || !y || !out_bf || !aligned16(x) || !aligned16(y) || !aligned16(out_bf))))
         return SDEM_SG_E_ARG;
     if (!set_smem((const void*)k_gather_add_sum, GS_SMEM)) return SDEM_SG_E_CUDA;
-    k_gather_add_sum<<<kColsumBlocks, GS_T, GS_SMEM, st(stream)>>>(rows, idx, x, ldx, y, out_bf, partial);
+    k_gather_add_sum<<<dim3(kColsumBlocks, 128 / GS_COLS), GS_T, GS_SMEM, st(stream)>>>(rows, idx, x, ldx, y, out_bf, partial);
     if (cudaGetLastError() != cudaSuccess) return SDEM_SG_E_CUDA;
-    k_colsum_final<<<1, 128, 0, st(stream)>>>(128, partial, sum, 1);
+    k_split_reduce<<<blocks(128, 32), 256, 0, st(stream)>>>(1, 128, kColsumBlocks, partial, sum, 128, 1);
     return launched();
 }
 
@@ -2386,14 +2379,14 @@ int sdem_sg_colsum(int M, int J, const float* x, int ldx, float* out, int accumu
     if (J == 0) return SDEM_SG_OK;
     if (!out || !partial || (M > 0 && !x)) return SDEM_SG_E_ARG;
     if (J == 128 && ldx % 4 == 0 && aligned16(x)) {
-        const int smem = CS_STAGES * CS_ROWS * 128 * 4;
+        const int smem = CS_STAGES * CS_ROWS * CS_COLS * 4;
         if (!set_smem((const void*)k_colsum_part128, smem)) return SDEM_SG_E_CUDA;
-        k_colsum_part128<<<kColsumBlocks, 256, smem, st(stream)>>>(M, x, ldx, partial);
+        k_colsum_part128<<<dim3(kColsumBlocks, 128 / CS_COLS), 256, smem, st(stream)>>>(M, x, ldx, partial);
     } else {
         k_colsum_part<<<kColsumBlocks, 128, 0, st(stream)>>>(M, J, x, ldx, partial);
     }
     if (cudaGetLastError() != cudaSuccess) return SDEM_SG_E_CUDA;
-    k_colsum_final<<<blocks(J, 128), 128, 0, st(stream)>>>(J, partial, out, accumulate);
+    k_split_reduce<<<blocks(J, 32), 256, 0, st(stream)>>>(1, J, kColsumBlocks, partial, out, J, accumulate);
     return launched();
 }
 
