@@ -1783,7 +1783,8 @@ __global__ void k_segsum(int nrows, int J, const int* __restrict__ row_off, cons
 // 128..255) added in list order, and its bf16 copy: the additions of
 // sdem_sg_gather_add and two sdem_sg_segsum calls, in their order.
 // Bound by HBM (d, 1 KB an edge, once).  k_segsum keeps one row in flight a warp;
-// here eight: 330k edges of 16k spheres 73 us (4.6 TB/s) instead of 108 in three kernels.
+// here four (with eight, and with 16, too few warps fit: 78 and 93 us against 68):
+// 330k edges of 16k spheres 65 us in a training step (5.1 TB/s), 108 in three kernels.
 __global__ void __launch_bounds__(256) k_sphere_grad(int n, const int* __restrict__ off0, const int* __restrict__ off1,
                                                      const int* __restrict__ perm1, const float* __restrict__ x, int ldx,
                                                      const float* __restrict__ y, const float* __restrict__ d,
@@ -1800,15 +1801,15 @@ __global__ void __launch_bounds__(256) k_sphere_grad(int n, const int* __restric
         const float* __restrict__ dc = d + side * 128 + lane * 4;
         for (int b = e0; b < e1; b += 32) {
             const int mine = b + lane < e1 ? (side ? perm1[b + lane] : b + lane) : 0, m = min(32, e1 - b);
-            for (int k = 0; k < m; k += 8) {
-                float4 v[8];
+            for (int k = 0; k < m; k += 4) {
+                float4 v[4];
 #pragma unroll
-                for (int q = 0; q < 8; ++q) {
+                for (int q = 0; q < 4; ++q) {
                     const int row = __shfl_sync(0xffffffffu, mine, (k + q) & 31);
                     if (k + q < m) v[q] = __ldcs(reinterpret_cast<const float4*>(dc + (size_t)row * 256));
                 }
 #pragma unroll
-                for (int q = 0; q < 8; ++q)
+                for (int q = 0; q < 4; ++q)
                     if (k + q < m) s = make_float4(s.x + v[q].x, s.y + v[q].y, s.z + v[q].z, s.w + v[q].w);
             }
         }
