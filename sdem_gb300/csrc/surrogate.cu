@@ -738,14 +738,14 @@ __global__ void __launch_bounds__(TC_T, 1) k_gemm_tc(int I, int J, int R, Operan
 // swizzle: element (row, k) of a 64-wide slice at row * 128 bytes + ((k / 8) xor
 // (row mod 8)) * 16.  The reduction runs in the same order and steps of 16 as
 // in k_gemm_tc and k_gemm, and the results are the same bits.
-// Bound by L2 on the gathered forward form (600k rows, R = 384: 117 us, 5.9 TB/s
+// Bound by L2 on the gathered forward form (600k rows, R = 384: 108 us, 6.4 TB/s
 // of L2; k_gemm_tc 328 us) and by HBM on the input gradient (J = 384, fp32 out:
-// 206 us, 5.0 TB/s; k_gemm 1150 us).
+// 183 us, 5.8 TB/s; k_gemm 1150 us).
 // An epilogue that reads a mask or a residual (kReads) has eight warps, two to a
 // row quarter, and requests what it reads before it waits for the products: with
 // four warps that read behind the wait, a residual update of 330k rows took 140 us
 // (85 here; 62 for its bytes), a masked gradient 104 (92).  Without reads the four
-// warps are better (fp32 out, J = 384: 206 against 245 us; the copying warps lose
+// warps were better (fp32 out, J = 384: 206 against 245 us; the copying warps lose
 // registers to the others).
 constexpr int RW_M = 128, RW_K = 64, RW_STAGES = 6, RW_LAG = 5, RW_ACC = 4, RW_T = 288, RW_T_READS = 416;
 constexpr int RW_SLICE = RW_M * RW_K * 2;              // 16 KB
