@@ -744,9 +744,9 @@ __global__ void __launch_bounds__(TC_T, 1) k_gemm_tc(int I, int J, int R, Operan
 // An epilogue that reads a mask or a residual (kReads) has eight warps, two to a
 // row quarter, and requests what it reads before it waits for the products: with
 // four warps that read behind the wait, a residual update of 330k rows took 140 us
-// (85 here; 62 for its bytes), a masked gradient 104 (92).  Without reads the four
-// warps were better (fp32 out, J = 384: 206 against 245 us; the copying warps lose
-// registers to the others).
+// (85 here; 62 for its bytes), a masked gradient 104 (92).  Without reads four warps
+// are better (600k rows, both forms above together: 317 against 405 us with eight;
+// the copying warps lose registers to the others).
 constexpr int RW_M = 128, RW_K = 64, RW_STAGES = 6, RW_LAG = 5, RW_ACC = 4, RW_T = 288, RW_T_READS = 416;
 constexpr int RW_SLICE = RW_M * RW_K * 2;              // 16 KB
 constexpr int RW_B_MAX = 98304;                        // bytes of B kept
