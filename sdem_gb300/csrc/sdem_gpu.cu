@@ -157,6 +157,7 @@ struct Dev {
   unsigned long long* near_mask;
   // binning
   int *cell_of, *cell_cnt, *cell_start, *tmp_rank, *tmp_sorted, *sorted, *sortpos;
+  int* unplaced;   // particles without a cell in this step
   float4* spos;      // cell-sorted single-precision copy (offsets in the cell, r) for the prefilter
   float4* pf;        // the same per particle index, written by the binning
   int4* pcell;   // per index: the cell (ix, iy, iz, key in its level's grid), written by the binning
@@ -487,6 +488,10 @@ __global__ void k_fixed_append(Dev d) {
 // Binning: NBSM_clcBoxIndex (Prtcl_NBS_Munjiza.f90:193-198) + counting sort.
 // Linear cell key orders cells as the reference's sweep visits them:
 // row iy (outer), column ix, cell iz (inner).
+// A particle outside the grid (SDEM_E_GRID) is in no cell: it takes a sort
+// position after the last cell's, so that the positions hold every particle once
+// whatever happens -- the sums and the update walk them -- and is neither a
+// target nor a candidate of the search.
 __global__ void k_bin(Dev d) {
   int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= *d.nt) return;
@@ -515,6 +520,7 @@ __global__ void k_bin(Dev d) {
   if (fx < 0 || fy < 0 || fz < 0) {
     raise(d, SDEM_E_GRID, p);
     d.cell_of[p] = -1;
+    if (d.unplaced) d.tmp_rank[p] = atomicAdd(d.unplaced, 1);
     return;
   }
   // offset in [0, 1) as a float from its top 23 bits (1.f - 1 is exact; an
@@ -545,7 +551,10 @@ __global__ void k_cellorder(Dev d) {
   int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= *d.nt) return;
   int key = d.cell_of[p];
-  if (key < 0) return;
+  if (key < 0) {
+    if (d.unplaced) d.sorted[d.cell_start[d.ncell] + d.tmp_rank[p]] = p;
+    return;
+  }
   int a = d.cell_start[key], b = d.cell_start[key + 1];
   // reference search index order: fixed spheres (appended after the moving
   // spheres and images here) come first there, so they rank lowest
@@ -571,12 +580,12 @@ __global__ void k_cellorder(Dev d) {
 template <bool kHier>
 __global__ void __launch_bounds__(kThreads, kSearchBlocksPerSM) k_search(Dev d, int s_begin, int s_end, int chunk) {
   int s = s_begin + blockIdx.x * blockDim.x + threadIdx.x;
-  const int nt = *d.nt;
+  const int placed = d.cell_start[d.ncell];   // targets: the positions of the cells
   const int nloc = *d.n;
   unsigned long long cand = 0, cand_x = 0;
   int rows = 0, m = 0;   // contacts of this thread's row, and its target
   if (s < s_end) {
-    if (s < nt) {
+    if (s < placed) {
       m = d.sorted[s];
       // a periodic image as target pairs with local particles only
       // (LoopNBSMask, Prtcl_NBS_Munjiza.f90:358-405 -> FineSearch3(n, m))
@@ -1478,6 +1487,7 @@ __device__ void step_end_serial(const Dev& d, int* counters_out) {
   d.counters[9] = 0;
   *d.out_cnt = 0;
   *d.wl_cnt = 0;
+  *d.unplaced = 0;
 }
 
 // What the last block of a step's last kernel writes: the counters and a copy
@@ -1726,9 +1736,9 @@ __global__ void k_na_begin(NoAllocScratch* S, int n) {
 // The search of k_search without its rows: the same half shell, the same
 // single-precision decision with the FP64 test in the ambiguous band; it only
 // counts numCntcts(1) and num_Cnsv_cntct.  Only the sort positions this call
-// wrote are searched: a particle outside the grid (SDEM_E_GRID) is not placed,
-// so sorted[cell_start[ncell] .. n) still holds an earlier call's indices,
-// which may lie beyond this call's d_posR.  After a binning error nothing is
+// wrote are searched: a particle outside the grid (SDEM_E_GRID) gets none here
+// (no d.unplaced), so sorted[cell_start[ncell] .. n) still holds an earlier
+// call's indices, which may lie beyond this call's d_posR.  After a binning error nothing is
 // searched at all.
 __global__ void __launch_bounds__(kThreads) k_na_count(Dev d, unsigned long long* counts) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1984,7 +1994,7 @@ int ensure_stage(sdem_h* h, size_t count) {
 
 enum { S_N = 0, S_STATUS = 1, S_ITER = 3, S_NEXT = 4, S_OUTCNT = 5, S_NEARCNT = 6, S_NG = 7, S_COUNTERS = 8,  // counters: 8..16
        S_NT = 20, S_TICKET = 21,  // two tickets
-       S_STALE = 23, S_WLCNT = 24, S_SIZE = 28 };
+       S_STALE = 23, S_WLCNT = 24, S_UNPLACED = 25, S_SIZE = 28 };
 
 Dev make_dev(sdem_h* h) {
   Dev d{};
@@ -2091,6 +2101,7 @@ Dev make_dev(sdem_h* h) {
   d.w_geo = h->w_geo;
   d.wl = h->wl;
   d.wl_cnt = h->scal + S_WLCNT;
+  d.unplaced = h->scal + S_UNPLACED;
   d.near_list = h->near_list;
   d.near_cnt = h->scal + S_NEARCNT;
   d.near_stale = h->scal + S_STALE;
