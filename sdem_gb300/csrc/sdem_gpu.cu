@@ -807,6 +807,20 @@ __global__ void __launch_bounds__(kWallThreads) k_wall_detect(Dev d) {
   if ((threadIdx.x & 31) == 0 && total) atomicAdd(&d.counters[1], (unsigned long long)total);
 }
 
+// Contacts whose records k_force writes in this step: those of the chunks before
+// the first that passes the capacity (all, in a step without SDEM_E_CL_FULL).
+__device__ __forceinline__ int contacts_computed(const Dev& d) {
+  int done = 0;
+  bool fits = true;
+#pragma unroll
+  for (int k = 0; k < kMaxChunks; k++) {
+    const int c = d.c_cnt[k];
+    fits = fits && c <= d.ccap - done;
+    if (fits) done += c;
+  }
+  return done;
+}
+
 // ---------------------------------------------------------------------------
 // One thread per contact: Find_insert's history lookup + ContactForce_PP.
 // Contacts of one chunk of the search.  kOneSided: the search holds periodic
@@ -816,10 +830,10 @@ __global__ void __launch_bounds__(kThreads, SDEM_FORCE_MIN_BLOCKS) k_force(Dev d
   const int nloc = *d.n;
   int c0 = 0;
   for (int k = 0; k < chunk; k++) c0 += d.c_cnt[k];
-  const int npp = d.c_cnt[chunk];
-  if (c0 + npp > d.ccap) {
+  int npp = d.c_cnt[chunk];
+  if (c0 + npp > d.ccap) {   // none of this chunk's pairs (see contacts_computed); the walls all the same
     if (blockIdx.x == 0 && threadIdx.x == 0) raise(d, SDEM_E_CL_FULL, c0 + npp);
-    return;
+    npp = 0;
   }
   // the first chunk's launch also takes the wall contacts, after the pairs
   const int items = npp + (chunk == 0 ? *d.wl_cnt : 0);
@@ -1457,12 +1471,12 @@ __device__ void step_end_serial(const Dev& d, int* counters_out) {
   }
 
   // every value first (the loads issue together), then the stores
+  d.row_off[d.nall_launch] = contacts_computed(d);   // the contact snapshot's count
   int C = 0;
   for (int k = 0; k < kMaxChunks; k++) {
     C += d.c_cnt[k];
     d.c_cnt[k] = 0;
   }
-  d.row_off[d.nall_launch] = C;   // the contact snapshot's count
   const unsigned long long cnsv = d.counters[0], pw = d.counters[1], ppg = d.counters[5], fx = d.counters[8],
                            cross = d.counters[9];
   const int n = *d.n, it = *d.iter + 1, next = *d.next_update;
@@ -1545,7 +1559,7 @@ __global__ void __launch_bounds__(kUpdateThreads) k_integrate(Dev d, StepEnd end
 
 // The sums of the particle at sort position s, and with kUpdate its update.
 template <bool kUpdate>
-__device__ __forceinline__ void gather_one(const Dev& d, const int s) {
+__device__ __forceinline__ void gather_one(const Dev& d, const int s, const int computed) {
   const int p = d.sorted[s];
   const int ncap = d.ncap;
   const double rp = d.posr[p].w;
@@ -1612,7 +1626,7 @@ __device__ __forceinline__ void gather_one(const Dev& d, const int s) {
     const bool tgt = e < 0 || (e & 1);   // a wall record or p's own row: as stored
     dbl4 S, Ms, Mr;
     if (c >= 0) {
-      if (c >= d.ccap) continue;   // past the capacity: reported by k_force, nothing was computed
+      if (c >= computed) continue;   // past the capacity: reported by k_force
       const ContactRec& rec = d.c_rec[c];
       S = rec.S;
       Ms = rec.M;
@@ -1656,12 +1670,13 @@ __global__ void __launch_bounds__(kUpdateThreads) k_gather(Dev d, StepEnd end) {
   static_assert(kDegBuckets == 64, "two buckets per lane of one warp");
   __shared__ int bucket[kDegBuckets];
   __shared__ int order[kUpdateThreads];
-  __shared__ int members;
+  __shared__ int members, computed;
   const int s0 = blockIdx.x * kUpdateThreads;
   const int nloc = *d.n;
   {
     const int s = s0 + threadIdx.x;
     if (threadIdx.x < kDegBuckets) bucket[threadIdx.x] = 0;
+    else if (threadIdx.x == kDegBuckets) computed = contacts_computed(d);
     __syncthreads();
     int deg = -1, rank = 0;
     if (s < *d.nt) {
@@ -1689,7 +1704,7 @@ __global__ void __launch_bounds__(kUpdateThreads) k_gather(Dev d, StepEnd end) {
     if (deg >= 0) order[bucket[deg] + rank] = s;
     __syncthreads();
   }
-  if ((int)threadIdx.x < members) gather_one<kUpdate>(d, order[threadIdx.x]);
+  if ((int)threadIdx.x < members) gather_one<kUpdate>(d, order[threadIdx.x], computed);
   if (kUpdate) end_step(d, end);
 }
 // ---------------------------------------------------------------------------
