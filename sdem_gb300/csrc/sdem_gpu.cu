@@ -2938,6 +2938,11 @@ int sdem_upload_contacts(sdem_h* h, int nc, const int* owner_idx, const int* par
   CK(cudaMemcpyAsync(h->wh_cnt[pv], whc.data(), sizeof(int) * G, cudaMemcpyHostToDevice, h->stream));
   CK(cudaMemcpyAsync(h->wh_wall[pv], whw.data(), sizeof(int) * G * kKw, cudaMemcpyHostToDevice, h->stream));
   CK(cudaMemcpyAsync(h->wh_hist[pv], whh.data(), sizeof(dbl4) * G * kKw, cudaMemcpyHostToDevice, h->stream));
+  // wall histories of particles that are off the near-wall list are cleared
+  // only where the list is made: make it anew at the next step
+  const int zero = 0, one = 1;
+  CK(cudaMemcpyAsync(h->scal + S_NEARCNT, &zero, sizeof zero, cudaMemcpyHostToDevice, h->stream));
+  CK(cudaMemcpyAsync(h->scal + S_STALE, &one, sizeof one, cudaMemcpyHostToDevice, h->stream));
   CK(cudaStreamSynchronize(h->stream));   // the host tables above go out of scope
   return 0;
 }
