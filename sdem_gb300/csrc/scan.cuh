@@ -1,6 +1,6 @@
 // scan.cuh -- exclusive prefix sums of int32 on the device, in one launch up to
-// a million elements and in two beyond, shared by the cell sorts of the particle
-// step and of the surrogate's graph.
+// a million elements and in two or three beyond, shared by the cell sorts of the
+// particle step and of the surrogate's graph.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -101,7 +101,12 @@ __device__ __forceinline__ int sum_before(const int* __restrict__ sums, int tile
 // per-thread runs of 16 are both free of bank conflicts).
 // One launch where the three of a reduce-then-scan took 14.5 us of dependent
 // latency: 6 us at 7,000 cells, 9 us at 60,000.
-template <bool kOnePass>
+// What a tile adds to its own sums: kOnePass, the look-back's prefix; kTileSums,
+// the sums of the tiles before it, added up by each block; kTileOffsets, its entry
+// of a scan of those sums.  kScanOfSums is that scan: kOnePass, in[] left as it is.
+enum ScanForm { kOnePass, kTileSums, kTileOffsets, kScanOfSums };
+inline __host__ __device__ int offsets_at(int tiles) { return (tiles + 3) / 4 * 4; }   // behind the sums
+template <ScanForm kForm>
 static __global__ void __launch_bounds__(kScanThreads) k_scan(int* __restrict__ in, long long n, int* __restrict__ out,
                                                        ScanCtl* ctl, unsigned long long* words, int* status) {
   __shared__ int sh[kScanTile + kScanTile / kScanItems];
@@ -109,7 +114,8 @@ static __global__ void __launch_bounds__(kScanThreads) k_scan(int* __restrict__ 
   __shared__ int s_tile, s_total;
   __shared__ unsigned s_epoch;
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-  if (kOnePass) {
+  constexpr bool kLookBack = kForm == kOnePass || kForm == kScanOfSums;
+  if (kLookBack) {
     if (t == 0) {
       s_epoch = ctl->epoch + 1u;
       s_tile = atomicAdd(&ctl->ticket, 1);
@@ -117,15 +123,15 @@ static __global__ void __launch_bounds__(kScanThreads) k_scan(int* __restrict__ 
     __syncthreads();
     if (s_tile >= (int)gridDim.x) return;   // (only a caller that shares ctl between overlapping launches gets here)
   }
-  const int tile = kOnePass ? s_tile : (int)blockIdx.x;
+  const int tile = kLookBack ? s_tile : (int)blockIdx.x;
   const long long base = (long long)tile * kScanTile;
   const bool whole = base + kScanTile <= n;
   auto pad = [](int e) { return e + e / kScanItems; };
-  if (!kOnePass) {
+  const int* sums = reinterpret_cast<const int*>(words);   // kTileSums, kTileOffsets (see scan_cells)
+  if (!kLookBack) {
     // the tiles' sums are known: a tile without counts is neither read nor cleared
-    const int* sums = reinterpret_cast<const int*>(words);
     if (sums[tile] == 0) {
-      const int excl = sum_before(sums, tile);
+      const int excl = kForm == kTileSums ? sum_before(sums, tile) : sums[offsets_at(gridDim.x) + tile];
       if (whole) {
         int4* v = reinterpret_cast<int4*>(out + base);
 #pragma unroll
@@ -143,7 +149,7 @@ static __global__ void __launch_bounds__(kScanThreads) k_scan(int* __restrict__ 
 #pragma unroll
     for (int j = 0; j < kScanItems / 4; j++) {
       const int4 q = v[j * kScanThreads + t];
-      if (q.x | q.y | q.z | q.w) v[j * kScanThreads + t] = make_int4(0, 0, 0, 0);
+      if (kForm != kScanOfSums && (q.x | q.y | q.z | q.w)) v[j * kScanThreads + t] = make_int4(0, 0, 0, 0);
       const int e = pad((j * kScanThreads + t) * 4);
       sh[e] = q.x;
       sh[e + 1] = q.y;
@@ -153,7 +159,7 @@ static __global__ void __launch_bounds__(kScanThreads) k_scan(int* __restrict__ 
   } else {
     for (int e = t; e < kScanTile; e += kScanThreads) {
       sh[pad(e)] = base + e < n ? in[base + e] : 0;
-      if (base + e < n) in[base + e] = 0;
+      if (kForm != kScanOfSums && base + e < n) in[base + e] = 0;
     }
   }
   __syncthreads();
@@ -184,11 +190,9 @@ static __global__ void __launch_bounds__(kScanThreads) k_scan(int* __restrict__ 
   }
   __syncthreads();
   int excl = 0;
-  if (kOnePass) {
-    excl = scan_lookback(words, s_epoch, tile, s_total, status);
-  } else {
-    excl = sum_before(reinterpret_cast<const int*>(words), tile);
-  }
+  if (kLookBack) excl = scan_lookback(words, s_epoch, tile, s_total, status);
+  else if (kForm == kTileSums) excl = sum_before(sums, tile);
+  else excl = sums[offsets_at(gridDim.x) + tile];
   const int first = excl + wsum[w] + x - sum;
 #pragma unroll
   for (int i = 0; i < kScanItems; i++) sh[t * (kScanItems + 1) + i] = first + loc[i];
@@ -206,7 +210,7 @@ static __global__ void __launch_bounds__(kScanThreads) k_scan(int* __restrict__ 
   }
   if (t == 0) {
     if (tile == (int)gridDim.x - 1) out[n] = excl + s_total;
-    if (kOnePass && atomicAdd(&ctl->done, 1) == (int)gridDim.x - 1) {   // every block has its ticket and epoch
+    if (kLookBack && atomicAdd(&ctl->done, 1) == (int)gridDim.x - 1) {   // every block has its ticket and epoch
       ctl->ticket = 0;
       ctl->done = 0;
       ctl->epoch = s_epoch;
@@ -214,7 +218,7 @@ static __global__ void __launch_bounds__(kScanThreads) k_scan(int* __restrict__ 
   }
 }
 
-// The tiles' sums for the two-launch form.
+// The tiles' sums, for the forms with more than one launch.
 static __global__ void __launch_bounds__(kScanThreads) k_scan_sums(const int* __restrict__ in, long long n, int* __restrict__ sums) {
   __shared__ int part[kScanThreads / 32];
   const long long base = (long long)blockIdx.x * kScanTile;
@@ -249,18 +253,37 @@ static __global__ void __launch_bounds__(kScanThreads) k_scan_sums(const int* __
 // hold a count are cleared.  With that the hopper's step takes 184 us instead of
 // 203.  Sums or flags per tile set by the binning instead of k_scan_sums were
 // slower (215 and 190 us: all spheres of a tile meet at one address).
+// Beyond 12,288 tiles (50M cells) the sums are scanned once, by a third launch:
+// each block adding up all sums before its own is quadratic in the tiles.  400k
+// counts spread over the grid, two launches against three: 4,096 tiles 53 / 57
+// us, 8,192 92 / 92, 16,384 175 / 160, 98,304 1,486 / 757.
 constexpr int kOnePassTiles = 256;
+constexpr int kSumsTiles = 12288;
 inline int scan_tiles(long long n) { return (int)std::max<long long>(1, (n + kScanTile - 1) / kScanTile); }
+// 8-byte words of scratch, zero before the first scan: one a tile; with three
+// launches the sums, their scan (each from a 16-byte boundary) and its own words.
+// A grid has fewer than 2^31 cells, so the scan of the sums takes one launch.
+inline size_t scan_words(long long n) {
+  const size_t tiles = (size_t)scan_tiles(n);
+  return tiles <= (size_t)kSumsTiles ? tiles : (size_t)offsets_at((int)tiles) + 2 + (size_t)scan_tiles((long long)tiles);
+}
 
 inline int scan_cells(int* cnt, long long n, int* out, ScanCtl* ctl, unsigned long long* words, int* status, cudaStream_t st) {
   const int tiles = scan_tiles(n);
   if (tiles <= kOnePassTiles) {
-    k_scan<true><<<tiles, kScanThreads, 0, st>>>(cnt, n, out, ctl, words, status);
+    k_scan<kOnePass><<<tiles, kScanThreads, 0, st>>>(cnt, n, out, ctl, words, status);
     return 1;
   }
-  k_scan_sums<<<tiles, kScanThreads, 0, st>>>(cnt, n, reinterpret_cast<int*>(words));
-  k_scan<false><<<tiles, kScanThreads, 0, st>>>(cnt, n, out, ctl, words, status);
-  return 2;
+  int* sums = reinterpret_cast<int*>(words);
+  k_scan_sums<<<tiles, kScanThreads, 0, st>>>(cnt, n, sums);
+  if (tiles <= kSumsTiles) {
+    k_scan<kTileSums><<<tiles, kScanThreads, 0, st>>>(cnt, n, out, ctl, words, status);
+    return 2;
+  }
+  const int at = offsets_at(tiles);   // tiles + 1 offsets, then the look-back's words
+  k_scan<kScanOfSums><<<scan_tiles(tiles), kScanThreads, 0, st>>>(sums, tiles, sums + at, ctl, words + at + 2, status);
+  k_scan<kTileOffsets><<<tiles, kScanThreads, 0, st>>>(cnt, n, out, ctl, words, status);
+  return 3;
 }
 
 }  // namespace scan

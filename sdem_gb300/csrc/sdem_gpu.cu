@@ -2655,7 +2655,7 @@ int sdem_set_types(sdem_h* h, int nT, const double* radius, const double* mass, 
   rc |= dalloc(h, &h->cell_cnt, (size_t)h->ncell);
   rc |= dalloc(h, &h->cell_start, (size_t)h->ncell + 1);
   rc |= dalloc(h, &h->cctl, 1);
-  rc |= dalloc(h, &h->cwords, (size_t)scan_tiles(h->ncell));
+  rc |= dalloc(h, &h->cwords, scan_words(h->ncell));
   if (rc) return SDEM_E_NOMEM;
   CK(cudaStreamSynchronize(h->stream));
   h->have_types = true;

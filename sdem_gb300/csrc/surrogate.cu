@@ -166,8 +166,8 @@ GraphWork graph_work(void* base, int n, long long ncell) {
     w.status = reinterpret_cast<int*>(head + 8);
     w.cctl = reinterpret_cast<scan::ScanCtl*>(head + 32);
     w.rctl = reinterpret_cast<scan::ScanCtl*>(head + 64);
-    w.cwords = reinterpret_cast<unsigned long long*>(take(8 * (size_t)scan::scan_tiles(ncell)));
-    w.rwords = reinterpret_cast<unsigned long long*>(take(8 * (size_t)scan::scan_tiles(n)));
+    w.cwords = reinterpret_cast<unsigned long long*>(take(8 * scan::scan_words(ncell)));
+    w.rwords = reinterpret_cast<unsigned long long*>(take(8 * scan::scan_words(n)));
     w.cell_cnt = reinterpret_cast<int*>(take(4 * (size_t)ncell));
     w.clear = off;
     w.cell_start = reinterpret_cast<int*>(take(4 * ((size_t)ncell + 1)));
