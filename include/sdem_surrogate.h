@@ -149,8 +149,10 @@ int sdem_sg_mlp(int M, int R, const sdem_sg_operand* a, const uint16_t* w1, cons
  * both transposed), 0 the warp-level mma.sync kernel for every form.  The
  * results are the same bits.  sdem_sg_mlp is always tcgen05. */
 int sdem_sg_set_tensor_path(int use_tcgen05);
-/* Number of tcgen05 GEMM blocks whose bounded mbarrier wait expired (0
- * expected; such a block writes zeros instead of its products). */
+/* Number of blocks of the tcgen05 kernels (sdem_sg_gemm, sdem_sg_mlp) whose
+ * bounded mbarrier wait expired, since the library was loaded (0 expected; such
+ * a block takes zeros for the products it has not read by then: bias, residual
+ * and the rest apply to them, z of sdem_sg_mlp is zero).  Waits for the device. */
 int sdem_sg_tensor_timeouts(unsigned int* count);
 
 /* out[i] (J floats) = (accumulate ? out[i] : 0) + sum over e in row_off[i] ..
