@@ -418,9 +418,25 @@ class Network:
         self.wide_rows = latent == LATENT and torch.device(device).type == "cuda"
         self.refresh_bf16()
         self.saved = None
+        self.lost_before = self._lost_waits()
 
     def refresh_bf16(self) -> None:
         _check(self.lib.sdem_sg_to_bf16(self.p.numel(), _ptr(self.p), _ptr(self.pb), _stream()), "sdem_sg_to_bf16")
+
+    def _lost_waits(self) -> int:
+        if torch.device(self.device).type != "cuda":
+            return 0
+        n = C.c_uint(0)
+        _check(self.lib.sdem_sg_tensor_timeouts(C.byref(n)), "sdem_sg_tensor_timeouts")
+        return n.value
+
+    def check_waits(self) -> None:
+        """Raises where a bounded wait of a tensor-core kernel has run out since
+        this network was made: such a block's products are zeros.  Waits for
+        the device."""
+        lost = self._lost_waits() - self.lost_before
+        if lost:
+            raise RuntimeError(f"a bounded wait ran out in {lost} blocks of the tensor-core kernels")
 
     def host_params(self) -> np.ndarray:
         return self.p.cpu().numpy()
@@ -797,6 +813,7 @@ def evaluate(net: Network, samples: List[DeviceSample]) -> Tuple[float, float]:
         num += float(loss) * n
         base += float((s.target.double() ** 2).mean()) * n
         den += n
+    net.check_waits()
     return num / den, base / den
 
 
@@ -978,6 +995,7 @@ class SurrogateRunner:
             st = self.sys.state()
         except Exception:       # the plain DEM rejected the surrogate's state
             st = None
+        self.net.check_waits()
         self.stats["judged"] += 1
         self.stats["surrogate_strides"] += 1
         if st is None:

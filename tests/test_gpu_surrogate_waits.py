@@ -2,10 +2,11 @@
 more with a limit of no polls, so that every bounded wait but the draining of
 issued products ends at once: each kernel returns, counts its blocks, and leaves
 zeros for its products (bias, ReLU and residual applied to them).  Blocks that
-need no wait are not affected."""
+need no wait are not affected.  A network on that library raises where it looks."""
 import ctypes
 import subprocess
 
+import numpy as np
 import pytest
 import torch
 
@@ -107,3 +108,19 @@ def test_two_layers(lib, agg):
     assert torch.equal(out, resid) and torch.equal(outb, resid.to(torch.bfloat16))
     if agg:
         assert not sums.any()
+
+
+def test_network_raises(lib, monkeypatch):
+    monkeypatch.setattr(sg, "_lib", lib)
+    rng = np.random.default_rng(3)
+    n, d = 500, 1.2e-3
+    p = np.c_[rng.uniform(0, 9e-3, (n, 3)), np.full(n, 0.5 * d)]
+    g = sg.build_graph(torch.from_numpy(p).to(DEV), sg.make_grid((0, 0, 0), (9e-3,) * 3, d))
+    net = sg.Network(seed=1)
+    net.check_waits()                       # what ran out before the network was made is not its own
+    net.forward(g, bf16(n, sg.NODE_IN), keep=False)
+    with pytest.raises(RuntimeError, match="wait ran out"):
+        net.check_waits()
+    sample = sg.DeviceSample(g, bf16(n, sg.NODE_IN), torch.zeros((n, 6), device=DEV))
+    with pytest.raises(RuntimeError, match="wait ran out"):
+        sg.evaluate(sg.Network(seed=1), [sample])
