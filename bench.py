@@ -659,11 +659,9 @@ def surrogate_arm(args):
     runner._surrogate_stride(runner.posR, runner.vel, runner.omega)     # warm-up
     phases, E = surrogate_phases(runner, net, sg, torch, reset)
     # the same forward layer by layer on the warp-level mma.sync kernel, for comparison
-    fused, net.fused = net.fused, False
     assert net.lib.sdem_sg_set_tensor_path(0) == 0
     phases_mma, _ = surrogate_phases(runner, net, sg, torch, reset)
     assert net.lib.sdem_sg_set_tensor_path(1) == 0
-    net.fused = fused
     t_sur = 0.0
     for _ in range(K):
         reset()

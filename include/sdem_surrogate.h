@@ -147,8 +147,10 @@ int sdem_sg_mlp(int M, int R, const sdem_sg_operand* a, const uint16_t* w1, cons
 /* Which tensor-core kernels sdem_sg_gemm uses: 1 (default) the tcgen05 ones
  * where one takes the form (second operand within 96 KB; no transposed operand;
  * both transposed), 0 the warp-level mma.sync kernel for every form.  The
- * results are the same bits.  sdem_sg_mlp is always tcgen05. */
+ * results are the same bits.  sdem_sg_mlp is always tcgen05: a caller that wants
+ * the other path takes the separate calls where sdem_sg_get_tensor_path says 0. */
 int sdem_sg_set_tensor_path(int use_tcgen05);
+int sdem_sg_get_tensor_path(void);
 /* Number of blocks of the tcgen05 kernels (sdem_sg_gemm, sdem_sg_mlp) whose
  * bounded mbarrier wait expired, since the library was loaded (0 expected; such
  * a block takes zeros for the products it has not read by then: bias, residual

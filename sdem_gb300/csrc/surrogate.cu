@@ -2389,6 +2389,8 @@ int sdem_sg_set_tensor_path(int use_tcgen05) {
     return SDEM_SG_OK;
 }
 
+int sdem_sg_get_tensor_path(void) { return g_tc_enabled; }
+
 int sdem_sg_tensor_timeouts(unsigned int* count) {
     if (!count) return SDEM_SG_E_ARG;
     return cudaMemcpyFromSymbol(count, g_tc_timeouts, sizeof(unsigned int)) == cudaSuccess ? SDEM_SG_OK

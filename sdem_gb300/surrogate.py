@@ -56,7 +56,7 @@ EXPORTED = ("sdem_sg_cells", "sdem_sg_edge_count", "sdem_sg_edge_fill", "sdem_sg
             "sdem_sg_segsum", "sdem_sg_gather_add", "sdem_sg_colsum_blocks", "sdem_sg_colsum", "sdem_sg_mse",
             "sdem_sg_adam", "sdem_sg_to_bf16", "sdem_sg_advance", "sdem_sg_set_tensor_path",
             "sdem_sg_tensor_timeouts", "sdem_sg_mlp", "sdem_sg_graph_work", "sdem_sg_graph_count", "sdem_sg_graph_fill",
-            "sdem_sg_sphere_grad", "sdem_sg_gather_add_sum")
+            "sdem_sg_sphere_grad", "sdem_sg_gather_add_sum", "sdem_sg_get_tensor_path")
 
 
 class SgGrid(C.Structure):
@@ -112,6 +112,7 @@ def load(path: str = LIB_PATH):
         "sdem_sg_to_bf16": [LL, P, P, P],
         "sdem_sg_advance": [I, P, I, D, D, D, D, D, C.POINTER(SgBox), P, P, P, P],
         "sdem_sg_set_tensor_path": [I],
+        "sdem_sg_get_tensor_path": [],
         "sdem_sg_tensor_timeouts": [C.POINTER(C.c_uint)],
         "sdem_sg_graph_work": [I, C.POINTER(SgGrid)],
         "sdem_sg_graph_count": [I, P, C.POINTER(SgGrid), P, P, P],
@@ -531,7 +532,7 @@ class Network:
 
     def forward(self, g: Graph, xn: torch.Tensor, keep: bool = True) -> torch.Tensor:
         """(n, 16) fp32 predictions; keep=True saves what backward needs."""
-        if self.fused:
+        if self.fused and self.lib.sdem_sg_get_tensor_path():
             return self._forward_fused(g, xn, keep)
         L, n, E, dev = self.latent, g.n, g.E, self.device
         bf, f32 = torch.bfloat16, torch.float32
