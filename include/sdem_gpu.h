@@ -265,6 +265,8 @@ int sdem_launch_count(sdem_h* h, long long* n);
 int sdem_profile_begin(sdem_h* h, int max_steps);
 /* Stops timing; ms[p] receives the summed milliseconds of phase p over the
  * timed steps (cap entries at most), *nsteps the number of timed steps.
+ * A phase whose work is part of another phase's kernel reports 0 (rows and
+ * contact lists: search; wall forces: force; deletes and counters: gather_integrate).
  * Returns the number of phases (>0) or an error code (<0 never; see status). */
 int sdem_profile_end(sdem_h* h, int cap, double* ms, int* nsteps);
 /* Name of phase i ("" outside the range). */

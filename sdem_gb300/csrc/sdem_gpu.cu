@@ -100,6 +100,12 @@ enum Phase { PH_WALL, PH_BIN, PH_SCAN_CELLS, PH_SCATTER, PH_CELLORDER, PH_SEARCH
 const char* const kPhaseNames[kPhases] = {"wall_refresh", "bin", "scan_cells", "scatter", "cellorder", "search",
                                           "scan_rows", "row_fill", "force", "wall_force", "gather_integrate",
                                           "delete", "step_end"};
+// Phases whose work is part of another kernel: rows and their contacts are laid out
+// by the search, wall forces belong to the force kernel, the end of the step to the
+// update.  They have no events and report no time.
+constexpr bool phase_has_kernels(int p) {
+  return p != PH_SCAN_ROWS && p != PH_ROW_FILL && p != PH_WALL_FORCE && p != PH_DELETE && p != PH_END;
+}
 
 // ---------------------------------------------------------------------------
 // The force kernel's record of one contact for the gather, 96 bytes in one
@@ -2250,8 +2256,6 @@ int enqueue_step(sdem_h* h) {
     else k_search<false><<<grid_for(std::max(b - a, 1)), kThreads, 0, sr>>>(d, a, b, k);
     if (piped) cudaEventRecord(h->ev_chunk[k], s2);
   }
-  mark(PH_SCAN_ROWS);   // rows and their contacts are laid out by the search: these two phases are empty
-  mark(PH_ROW_FILL);
   mark(PH_FORCE);
   if (s2 != st && !piped) cudaStreamWaitEvent(st, h->ev_wall, 0);
   for (int k = 0; k < nchunk; k++) {
@@ -2260,7 +2264,6 @@ int enqueue_step(sdem_h* h) {
     if (h->gcap > 0 || h->nfix > 0) k_force<true><<<blocks, kThreads, 0, st>>>(d, k);
     else k_force<false><<<blocks, kThreads, 0, st>>>(d, k);
   }
-  mark(PH_WALL_FORCE);   // wall forces are part of the force kernel: this phase is empty
   mark(PH_GATHER);
   const StepEnd end{h->scal + S_COUNTERS, h->scal, h->d_mirror, S_SIZE};
   // Sums and update in one kernel while the state (~640 B a sphere) sits in
@@ -2275,8 +2278,6 @@ int enqueue_step(sdem_h* h) {
     k_gather<false><<<grid_for(na, kUpdateThreads), kUpdateThreads, 0, st>>>(d, end);
     k_integrate<<<grid_for(n, kUpdateThreads), kUpdateThreads, 0, st>>>(d, end);
   }
-  mark(PH_DELETE);   // the end of the step is part of the update kernel: these two phases are empty
-  mark(PH_END);
   h->mirror_ok = true;
   mark(kPhases);
   // bin, scatter, cellorder, gather, integrate; per chunk search, force
@@ -3511,8 +3512,11 @@ int sdem_profile_end(sdem_h* h, int cap, double* ms, int* nsteps) {
   for (int s = 0; s < h->prof_steps; s++) {
     cudaEvent_t* ev = &h->prof_ev[(size_t)s * (kPhases + 1)];
     for (int p = 0; p < kPhases && p < cap; p++) {
+      if (!phase_has_kernels(p)) continue;
+      int next = p + 1;
+      while (next < kPhases && !phase_has_kernels(next)) next++;
       float t = 0.f;
-      CK(cudaEventElapsedTime(&t, ev[p], ev[p + 1]));
+      CK(cudaEventElapsedTime(&t, ev[p], ev[next]));
       ms[p] += t;
     }
   }
