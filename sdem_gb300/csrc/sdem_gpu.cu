@@ -815,17 +815,19 @@ __global__ void __launch_bounds__(kWallThreads) k_wall_detect(Dev d) {
 
 // Contacts whose records k_force writes in this step: those of the chunks before
 // the first that passes the capacity (all, in a step without SDEM_E_CL_FULL).
-__device__ __forceinline__ int contacts_computed(const Dev& d) {
+__device__ __forceinline__ int contacts_computed(int ccap, const int4& found) {
+  static_assert(kMaxChunks == 4, "the chunks' counts in one load");
+  const int c[kMaxChunks] = {found.x, found.y, found.z, found.w};
   int done = 0;
   bool fits = true;
 #pragma unroll
   for (int k = 0; k < kMaxChunks; k++) {
-    const int c = d.c_cnt[k];
-    fits = fits && c <= d.ccap - done;
-    if (fits) done += c;
+    fits = fits && c[k] <= ccap - done;
+    if (fits) done += c[k];
   }
   return done;
 }
+__device__ __forceinline__ int4 contacts_found(const Dev& d) { return *reinterpret_cast<const int4*>(d.c_cnt); }
 
 // ---------------------------------------------------------------------------
 // One thread per contact: Find_insert's history lookup + ContactForce_PP.
@@ -1477,15 +1479,13 @@ __device__ void step_end_serial(const Dev& d, int* counters_out) {
   }
 
   // every value first (the loads issue together), then the stores
-  d.row_off[d.nall_launch] = contacts_computed(d);   // the contact snapshot's count
-  int C = 0;
-  for (int k = 0; k < kMaxChunks; k++) {
-    C += d.c_cnt[k];
-    d.c_cnt[k] = 0;
-  }
+  const int4 found = contacts_found(d);
+  const int C = found.x + found.y + found.z + found.w;
   const unsigned long long cnsv = d.counters[0], pw = d.counters[1], ppg = d.counters[5], fx = d.counters[8],
                            cross = d.counters[9];
   const int n = *d.n, it = *d.iter + 1, next = *d.next_update;
+  *reinterpret_cast<int4*>(d.c_cnt) = make_int4(0, 0, 0, 0);
+  d.row_off[d.nall_launch] = contacts_computed(d.ccap, found);   // the contact snapshot's count
   const int pp = C - (int)ppg - (int)fx;
   counters_out[SDEM_CNT_PP] = pp;
   counters_out[SDEM_CNT_PPG] = (int)ppg;
@@ -1565,7 +1565,7 @@ __global__ void __launch_bounds__(kUpdateThreads) k_integrate(Dev d, StepEnd end
 
 // The sums of the particle at sort position s, and with kUpdate its update.
 template <bool kUpdate>
-__device__ __forceinline__ void gather_one(const Dev& d, const int s, const int computed) {
+__device__ __forceinline__ void gather_one(const Dev& d, const int s) {
   const int p = d.sorted[s];
   const int ncap = d.ncap;
   const double rp = d.posr[p].w;
@@ -1579,6 +1579,7 @@ __device__ __forceinline__ void gather_one(const Dev& d, const int s, const int 
   const int own_a = d.row_off[s], own_n = d.row_cnt[s];
   const int nin = min(d.in_cnt[s], d.Kin);
   const int nwc = d.w_cnt[p];
+  const int computed = contacts_computed(d.ccap, contacts_found(d));
   const unsigned* __restrict__ inl = d.in_list + (size_t)s * d.Kin;
   // entry: (contact index << 1) | (p is the row's target), or -(wall slot + 1)
   int list[2 * kMaxK + kKw];
@@ -1676,13 +1677,12 @@ __global__ void __launch_bounds__(kUpdateThreads) k_gather(Dev d, StepEnd end) {
   static_assert(kDegBuckets == 64, "two buckets per lane of one warp");
   __shared__ int bucket[kDegBuckets];
   __shared__ int order[kUpdateThreads];
-  __shared__ int members, computed;
+  __shared__ int members;
   const int s0 = blockIdx.x * kUpdateThreads;
   const int nloc = *d.n;
   {
     const int s = s0 + threadIdx.x;
     if (threadIdx.x < kDegBuckets) bucket[threadIdx.x] = 0;
-    else if (threadIdx.x == kDegBuckets) computed = contacts_computed(d);
     __syncthreads();
     int deg = -1, rank = 0;
     if (s < *d.nt) {
@@ -1710,7 +1710,7 @@ __global__ void __launch_bounds__(kUpdateThreads) k_gather(Dev d, StepEnd end) {
     if (deg >= 0) order[bucket[deg] + rank] = s;
     __syncthreads();
   }
-  if ((int)threadIdx.x < members) gather_one<kUpdate>(d, order[threadIdx.x], computed);
+  if ((int)threadIdx.x < members) gather_one<kUpdate>(d, order[threadIdx.x]);
   if (kUpdate) end_step(d, end);
 }
 // ---------------------------------------------------------------------------
