@@ -855,7 +855,7 @@ def surrogate_gemm_arm(args):
             "dtype": "bf16", "data": "synthetic",
             "config": {"workload": "surrogate_gemm", "rows": E, "node_rows": nodes, "J": L,
                        "R": [3 * L, L], "gather": "rows of two 128-wide segments gathered by edge index"},
-            "roofline": {"bound": "tensor", "kernel": "k_gemm_tc", "achieved": tc["edge_w1_tflops"], "peak": peak,
+            "roofline": {"bound": "tensor", "kernel": "k_gemm_rows", "achieved": tc["edge_w1_tflops"], "peak": peak,
                          "unit": "TFLOP/s", "frac": tc["edge_w1_tflops"] / peak,
                          "peak_note": "bf16 dense, burst, of measured (MEASURED_PEAKS.json)"},
             "paths": res, "tcgen05_wait_timeouts": cnt.value}

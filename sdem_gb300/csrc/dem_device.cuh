@@ -179,16 +179,16 @@ struct LawCfg {
 // Hertz powers: ovrlp**1.5 is evaluated as ovrlp*sqrt(ovrlp) and ovrlp**0.25
 // as sqrt(sqrt(ovrlp)); both agree with libm pow to ~1 ulp (the reference's
 // gfortran calls pow), and cost a tenth of a double-precision pow on GB300.
-// The FP64 pipe issues two operations per SM per clock and is what the force
-// kernel waits for (70% busy).  From the tangential velocity on, products and
-// sums are fused: 98 pipe operations a Hertz contact instead of 120, k_force
-// 300 -> 261 us at 1M spheres with 1.0 contact each (with the update's and the
-// gather's, below, 813 -> 723 us a step).  Against 80-bit arithmetic over 2M
+// The FP64 pipe does at most 1.68 operations per SM per clock and is what the
+// force kernel waits for (95% of that on the settled 1M bed).  From the tangential
+// velocity on, products and sums are fused: 95 pipe operations a Hertz contact
+// instead of 120, k_force 300 -> 261 us at 1M spheres with 1.0 contact each (with
+// the update's and the gather's, below, 813 -> 723 us a step).  Against 80-bit arithmetic over 2M
 // random contacts the fused forces' rms error is 6.8e-17 of the force, the
 // unfused ones' 8.3e-17.  The chain up to vrn keeps the reference's roundings:
 // where a new pair meets almost tangentially |vrn| is the small difference of
 // large terms, and it is kept for the contact's life as VelRel_Init.
-// In a small bed the kernel takes as long as one warp of it: 98 FP64
+// In a small bed the kernel takes as long as one warp of it: 95 FP64
 // instructions of 64 cycles each, and the chains of the roots and quotients,
 // which therefore run in 32-bit products and side by side (fp64_int.cuh).  Per
 // step, before and after: linear spring 54.7 -> 43.7 us at 2k spheres and

@@ -2223,8 +2223,9 @@ int enqueue_step(sdem_h* h) {
   // one chunk, the default, the search stays on the main stream and waits for
   // nothing but the sort.  k_force holds every SM's registers, so a search
   // gains little from running beside it, and every chunk adds a partial last
-  // round of forces: 1 / 2 / 3 chunks take 60 / 80 / 98 us per step at 20k
-  // spheres, 198 / 237 / 228 at 200k, 695 / 761 / 693 at 1M.
+  // round of forces: 1 / 2 / 3 chunks take 49 / 60 / 70 us per step at 20k
+  // spheres (linear spring; Hertz 81 / 98 / 118), 191 / 209 / 220 at 200k,
+  // 659 / 673 / 674 at 1M.
   // Chunk boundaries lie on whole search blocks.  The first chunk's search
   // runs alone, before any force: by default it takes as many whole waves of
   // resident search blocks as fit in an even share, when that trims the share
@@ -2269,8 +2270,8 @@ int enqueue_step(sdem_h* h) {
   // Sums and update in one kernel while the state (~640 B a sphere) sits in
   // L2; beyond, the update in index order reads and writes whole lines where
   // the sums' order would scatter 32-byte records.  One kernel against two,
-  // per step: 100k spheres 126 / 132 us, 20k 60.4 / 62.4, 200k 200.8 / 198.2,
-  // 400k 357 / 322, 1M 896 / 695.
+  // per step: 20k spheres 48.5 / 49.9 us, 100k 120 / 124, 130k 136 / 140, 160k
+  // 167 / 163, 200k 199 / 191, 400k 346 / 308, 1M 844 / 660.
   const bool together = na <= kUpdateTogether;
   if (together) {
     k_gather<true><<<grid_for(na, kUpdateThreads), kUpdateThreads, 0, st>>>(d, end);

@@ -26,12 +26,9 @@
 //   k_mse, k_adam, k_to_bf16,
 //   k_advance                       loss, optimiser, casts, one stride.
 //
-// GEMM tiling: 128 threads (4 warps) per 64x64 output tile, 32-deep slices of
-// the reduction staged in padded shared memory (row stride 40 bf16 = 20
-// words, so the 8x4 fragment reads of a warp hit 32 distinct banks), each
-// warp a 32x32 sub-tile of 2x4 mma.m16n8k16 (bf16 in, fp32 accumulate).
-// Every accumulator element is owned by one thread and summed in a fixed
-// reduction order, so results are bit-reproducible run to run.
+// Every element of a product is summed in steps of 16 in the order of the
+// reduction, whichever kernel takes it, so results are the same bits between the
+// kernels and from run to run.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <math.h>
@@ -124,15 +121,15 @@ __global__ void k_edges(int n, const double* __restrict__ posR, sdem_sg_grid g, 
 
 // ---- the whole graph build on the device (sdem_sg_graph_count / _fill)
 // Counting sort of the spheres by cell, then by index; one thread per sorted
-// sphere lists its neighbours; eight lanes per receiver write its edges.  The
+// sphere lists its neighbours; a block writes the edges of 64 of them.  The
 // candidates are tested in single precision on coordinates relative to their
 // cell's corner; only those within a margin of the cutoff take the exact FP64
 // test (which k_edges runs for every candidate, twice, on GB300's two FP64
 // operations per SM per clock).  Square roots and divisions of the features run
 // on the integer pipes (fp64_int.cuh), bit-identical to the hardware's.
 // 200k spheres, 3.9M edges: 7.0 ms as k_edges twice with torch's sorts and
-// prefix sums in between, 0.36 ms here, of which the edges' features 192 us
-// (FP64 pipe 70% busy).
+// prefix sums in between, 0.31 ms here (111 us until the edges are counted, 146 to
+// write them, bound by the FP64 pipe; the rest is the count on its way to the host).
 constexpr int GR_CAP = 96;    // neighbours kept per sphere between the two calls; longer lists are searched again
 constexpr int GR_T = 256;
 
@@ -442,6 +439,10 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], 
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
+// mma.sync, for every form: 128 threads (4 warps) per 64x64 output tile, 32-deep
+// slices of the reduction staged in padded shared memory (row stride 40 bf16 = 20
+// words, so the 8x4 fragment reads of a warp hit 32 distinct banks), each
+// warp a 32x32 sub-tile of 2x4 mma.m16n8k16 (bf16 in, fp32 accumulate).
 __global__ void __launch_bounds__(GT) k_gemm(int I, int J, int R, Operand A, Operand B, sdem_sg_epilogue ep,
                                              int rchunk, float* __restrict__ partial) {
     __shared__ __align__(16) uint16_t As[BM][LDS];

@@ -16,9 +16,10 @@ acceleration over a stride of S DEM steps:
 Every layer runs on the tensor cores of the library's GEMM (bf16 operands,
 fp32 accumulation, fused bias/ReLU/residual epilogues), forward and
 backward; the aggregation and its adjoints, the loss, Adam and the stride
-update are the library's kernels too.  PyTorch holds the device memory and
-provides the sorts and prefix sums of the graph build.  The product path has
-no CPU fallback: loading fails loudly when the library is missing.
+update are the library's kernels too, and so is the graph but for the sender
+order, which the backward pass needs: PyTorch holds the device memory and sorts
+the edges by sender.  The product path has no CPU fallback: loading fails
+loudly when the library is missing.
 
 SurrogateRunner advances a bed by surrogate strides and, every `judge_every`
 strides, re-advances one stride with the plain FP64 DEM (include/sdem_gpu.h)
