@@ -1376,9 +1376,9 @@ __global__ void __launch_bounds__(WG_T, 1) k_gemm_wgrad(int I, int J, int R, Ope
 // the next tile.  All results are the bits of the separate kernels.
 // Tensor memory (512 columns): one accumulator of the first layer, two of the
 // second, whose readers are the slower ones, and two of z.
-// Two things bound it, measured on an edge block of 974k edges (326 us, 364 with z
-// kept; its HBM bytes would take 230): the sums (252 us alone) and the copies (242
-// for a bf16 result alone; 158 at R = 128).  A thread per row storing 32 bytes of
+// Two things bound it, measured on an edge block of 974k edges (331 us, 367 with z
+// kept; its HBM bytes would take 230): the sums (250 us alone) and the copies (255
+// for a bf16 result alone; 164 at R = 128).  A thread per row storing 32 bytes of
 // 32 rows at a time instead of strips, which make whole lines: 473.  z in shared
 // memory, which leaves room for a ring of three slices instead of five: 373.
 // Slices are handed over two behind the copies (3 behind: 346, 1: 355).
